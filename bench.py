@@ -59,6 +59,10 @@ MMA_K_PAD = 64  # int8 K of every tcgen05 tile (operand bit planes padded to 64)
 UNIT = "pairs/s"
 
 
+# residue-pair kernels (k=24 runs 4 staged and 4 folded levels, as the capture does)
+NCU_WARP_INST_PER_RESIDUE_PAIR = (137859072 + 328428147) / (5409 * 5410 // 2)
+
+
 def issue_roofline(pairs_per_s: float, epilogue: str, sm_mhz, num_sms: int) -> dict:
     """Instruction issue of the tcgen05 path (the bound of its epilogue): warp
     instructions per pair from the ncu capture against 4 warp instructions per
@@ -81,7 +85,7 @@ def parse():
     p.add_argument("--warmup", type=int, default=3)
     p.add_argument("--impl", default="b200", choices=["b200", "reference"])
     p.add_argument("--workload", default="an_k24", choices=["an_k24", "an_k20", "an_k22"])
-    p.add_argument("--kernel", default="auto", choices=["auto", "popc", "mma"])
+    p.add_argument("--kernel", default="auto", choices=["auto", "popc", "mma", "carry"])
     p.add_argument("--epilogue", default="auto", choices=["auto", "paired", "single"],
                    help="tcgen05 epilogue (auto: the autotuner's choice); pin it where a profiler's overhead "
                         "could change the autotuner's choice")
@@ -238,15 +242,15 @@ def counts_digest(counts: list[int]) -> str:
 
 
 def cross_kernel_check(ctx, dd, A: int, k: int, timed) -> dict:
-    """Recomputes the timed histogram on the other kernel (popc <-> tcgen05)
-    and requires the identical raw bins and counts: two independent
+    """Recomputes the timed histogram on another kernel (popc for tcgen05, tcgen05
+    for popc and for the residue-pair kernels) and requires the identical raw bins and counts: two independent
     implementations of the same exact histogram."""
     other = dd.KERNEL_POPC if timed.kernel_used == dd.KERNEL_MMA else dd.KERNEL_MMA
     o = ctx.histogram(dd.Request(dd.CODE_AN, dd.MODE_EXHAUSTIVE, A, k, kernel=other))
     assert o.kernel_used == other
     same = o.raw == timed.raw and o.counts == timed.counts
     assert same, "the two kernels disagree on the headline histogram"
-    name = {dd.KERNEL_POPC: "popc", dd.KERNEL_MMA: "mma"}
+    name = {dd.KERNEL_POPC: "popc", dd.KERNEL_MMA: "mma", dd.KERNEL_CARRY: "carry"}
     return {"cross_kernel": same, "timed_kernel": name[timed.kernel_used], "other_kernel": name[other],
             "other_kernel_pairs_per_s": pairs_of(k) / (o.kernel_ms * 1e-3),
             "sha256_counts": counts_digest(timed.counts)}
@@ -274,7 +278,8 @@ def main() -> None:
     stream = torch.cuda.current_stream()
     ctx = dd.Context(local, stream.cuda_stream)
     A, k = WORKLOADS[args.workload]
-    kernel = {"auto": dd.KERNEL_AUTO, "popc": dd.KERNEL_POPC, "mma": dd.KERNEL_MMA}[args.kernel]
+    kernel = {"auto": dd.KERNEL_AUTO, "popc": dd.KERNEL_POPC, "mma": dd.KERNEL_MMA,
+              "carry": dd.KERNEL_CARRY}[args.kernel]
     tuning = ctx.autotune() if kernel == dd.KERNEL_AUTO else None
     if args.epilogue != "auto":
         ctx.set_mma_epilogue(dd.MMA_EPILOGUE_PAIRED if args.epilogue == "paired" else dd.MMA_EPILOGUE_SINGLE)
@@ -295,6 +300,8 @@ def main() -> None:
         torch.cuda.synchronize()
 
     def kname(r):
+        if r.kernel_used == dd.KERNEL_CARRY:
+            return "carry"
         return ("mma_" + dd.EPILOGUE_NAMES.get(r.mma_epilogue, "?")) if r.kernel_used == dd.KERNEL_MMA else "popc"
 
     for _ in range(args.warmup):
@@ -337,7 +344,21 @@ def main() -> None:
     e2e = replica_throughput(P * args.steps, world, t_total)
     per_gpu = P * args.steps / (kernel_ms * 1e-3)
     mma = results[0].kernel_used == dd.KERNEL_MMA
-    if mma:
+    if results[0].kernel_used == dd.KERNEL_CARRY:
+        # residue-pair kernels: A^2 / 2 pairs of residues stand for the 4^k / 2 pairs of
+        # codewords; the bound is instruction issue
+        rpairs = A * (A + 1) // 2 * args.steps / (kernel_ms * 1e-3)
+        peak = ISSUE_PER_CLOCK_PER_SM * torch.cuda.get_device_properties(local).multi_processor_count * \
+            (clk.get("sm_mhz") or 0) * 1e6
+        roofline = {"bound": "issue", "achieved": rpairs * NCU_WARP_INST_PER_RESIDUE_PAIR / 1e9,
+                    "peak": peak / 1e9 if peak else None, "unit": "Ginst/s",
+                    "frac": rpairs * NCU_WARP_INST_PER_RESIDUE_PAIR / peak if peak else None,
+                    "traffic": None, "residue_pairs_per_s": rpairs, "codeword_pairs_per_residue_pair": P / (A * (A + 1) // 2),
+                    "warp_inst_per_residue_pair": NCU_WARP_INST_PER_RESIDUE_PAIR,
+                    "peak_source": "4 warp instructions per clock per SM at the median SM clock sampled in the timed "
+                                   "region; instructions per residue pair from sm__inst_executed.sum of the staging and "
+                                   "folding kernels of one block (A=5409, k=21), ncu capture"}
+    elif mma:
         # tcgen05 path: the tensor core computes the distances; the bound is the
         # histogram epilogue's shared-memory atomics: one per pair (single
         # epilogue) or one per two pairs (paired epilogue, packed distance pairs)
@@ -389,7 +410,7 @@ def main() -> None:
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": 256, "d2h_bytes_per_step": 64 * 8 * 8},
         "gpu_launches": args.steps,
         "clocks": clk,
-        "kernel_used": ("mma_" + dd.EPILOGUE_NAMES.get(results[0].mma_epilogue, "?")) if mma else "popc",
+        "kernel_used": kname(results[0]),
         "autotune": tuning,
     }
     if parity is not None:
@@ -488,7 +509,8 @@ def serving_extra(dd, rate_per_s=16.0) -> dict:
             "p99_ms": percentile(lat, 0.99), "per_class": per_class,
             "pairs": pairs, "pairs_per_s_wall": pairs / wall, "pairs_per_s_device": st["pairs_per_s"],
             "rounds": st["rounds"], "wall_s": wall,
-            "kernels_used": sorted({dd.KERNEL_POPC: "popc", dd.KERNEL_MMA: "mma"}.get(x, str(x)) for x in kernels),
+            "kernels_used": sorted({dd.KERNEL_POPC: "popc", dd.KERNEL_MMA: "mma", dd.KERNEL_CARRY: "carry"}.get(x, str(x))
+                                   for x in kernels),
             "mix": "A odd 8-16 bit, k in {8,12,16,20,24,32}; exhaustive k<=20; k>=24 grid stride 2^(k-16) "
                    "(m=2^16) or Monte Carlo 2^32..2^36 samples"}
 

@@ -21,7 +21,7 @@ from pathlib import Path
 
 __all__ = [
     "CODE_AN", "CODE_EXT_HAMMING", "MODE_EXHAUSTIVE", "MODE_GRID_1D", "MODE_GRID_2D", "MODE_MONTE_CARLO",
-    "KERNEL_AUTO", "KERNEL_POPC", "KERNEL_MMA", "HAMMING_WEIGHTS", "HAMMING_ALL_PAIRS", "HAMMING_ALL_PAIRS_DISTINCT",
+    "KERNEL_AUTO", "KERNEL_POPC", "KERNEL_MMA", "KERNEL_CARRY", "HAMMING_WEIGHTS", "HAMMING_ALL_PAIRS", "HAMMING_ALL_PAIRS_DISTINCT",
     "CONV_GPU", "CONV_CPU", "CONV_SUPER_A", "MMA_EPILOGUE_AUTO", "MMA_EPILOGUE_PAIRED",
     "MMA_EPILOGUE_SINGLE", "MAX_BINS", "DDError", "Request", "Result", "Context", "Server",
     "load", "lib_path", "postprocess", "request_plan", "format_result", "request_shape", "philox4x32_10", "device_count",
@@ -31,7 +31,7 @@ __all__ = [
 
 CODE_AN, CODE_EXT_HAMMING = 0, 1
 MODE_EXHAUSTIVE, MODE_GRID_1D, MODE_GRID_2D, MODE_MONTE_CARLO = 0, 1, 2, 3
-KERNEL_AUTO, KERNEL_POPC, KERNEL_MMA = 0, 1, 2
+KERNEL_AUTO, KERNEL_POPC, KERNEL_MMA, KERNEL_CARRY = 0, 1, 2, 3
 HAMMING_WEIGHTS, HAMMING_ALL_PAIRS, HAMMING_ALL_PAIRS_DISTINCT = 0, 1, 2
 CONV_GPU, CONV_CPU, CONV_SUPER_A = 0, 1, 2
 MMA_EPILOGUE_AUTO, MMA_EPILOGUE_PAIRED, MMA_EPILOGUE_SINGLE = 0, 1, 2

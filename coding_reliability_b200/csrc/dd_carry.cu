@@ -1,0 +1,683 @@
+// dd_carry.cu — exact AN exhaustive histograms without visiting the pairs one by one.
+//
+// A codeword A*x with A odd and x in [0, 2^k) is fixed by its low k bits t (A is
+// invertible mod 2^k, so t takes every value once): its high word is the c with
+// t + 2^k c = 0 mod A, c in [0, A), that is
+//     c(t) = psi(t mod A),   psi(v) = g v mod A,   g = -2^-k mod A.
+// So the distance of two codewords is popc(t ^ t') + popc(psi(v) ^ psi(v')) with
+// v = t mod A: 4^k pairs see only A^2 different high-word distances.  Written as
+// a polynomial in z (coefficient of z^d = pairs at distance d) the histogram is
+//     T = sum over t, t' of z^popc(t ^ t') Q(v, v'),  Q(v, v') = z^popc(psi(v) ^ psi(v')).
+// Split t = 2^b q + r.  The sum over the low parts r, r' in [0, 2^b) is a window
+//     G(v, v') = sum over r, r' of z^popc(r ^ r') Q(v + r, v' + r'),
+// which b two-by-two steps build for all residue pairs at once, one per bit j:
+//     H'(v, v') = H(v, v') + H(v+s, v'+s) + z (H(v, v'+s) + H(v+s, v')),  s = 2^j
+// (the steps commute; they run from the largest s to s = 1).  Then
+//     T = sum over q, q' in [0, 2^(k-b)) of z^popc(q ^ q') G(2^b q mod A, 2^b q' mod A),
+// where residue v is hit by q = qinv v mod A, plus multiples of A below 2^(k-b).
+// With b = k - bits(A) that is about b A^2 / 2 small steps instead of 4^k / 2 pairs
+// (A = 58659, k = 22: 1.0e10 against 8.8e12), all in integers.
+//
+// Measured on B200 against the tcgen05 kernel: A = 62307, k = 22: 67.5 ms against
+// 965 ms, k = 20: 26.8 against 63.5 ms; A = 867, k = 21: 0.66 against 231 ms, k = 16:
+// 0.065 against 0.37 ms.  Bound by instruction issue: ncu (A = 30011, k = 19) counts
+// 367 warp instructions per 32 residue pairs at 67 % issue, the ALU pipe 67 % and the
+// shared-memory pipe 63 % busy; DRAM carries nothing below 5 window bits and the
+// staged histograms (24 bytes a residue pair, once each way) above.
+//
+// A histogram lives in registers, packed: four 8-bit counts per word while the
+// counts stay within 4^4, two 16-bit counts per word up to 4^8.  Words hold
+// every second (every fourth) bin, so that multiplying by z renames words and
+// shifts only one word in two (in four).  The count 4^4 (4^8) itself does not
+// fit its field: it needs all pairs of a window at one distance; the field would
+// wrap, and the histogram's total with it, which the caller compares with the
+// number of pairs (and computes the job on the direct kernels if they differ).
+//
+// Thread = residue column v', time = residue rows v, descending.  A step needs
+// the neighbour column v'+s of the same row (through shared memory) and both of
+// row v+s (kept as Y = H(v, v'+s) + z H(v, v') in a register ring of s rows).
+// Windows of up to 4 bits run in one kernel from the popcounts to the bins;
+// longer ones run their largest steps first, in a kernel whose rows and columns
+// are 16 residues apart, and stage the 8-bit histograms in memory.
+#include <algorithm>
+#include <type_traits>
+
+#include "dd_carry.h"
+
+namespace dd {
+namespace {
+
+constexpr int kStageThreads = 512;  // staging kernel: 4 column residues mod 16 x 128 columns 16 apart
+constexpr int kStageCols = kStageThreads / 4;
+constexpr int kUnit = 16;           // residues between the staging kernel's rows and columns
+constexpr int kTabRows = 48;        // distances a table holds: q part <= 16, window part <= 28
+constexpr int kLeafThreads = 256;   // folding kernel reading popcounts
+constexpr int kFoldThreads = 192;   // folding kernel reading staged histograms
+constexpr int kLead = 8;            // rows above a step's own that its first level reads
+constexpr int kAhead = 3;           // rows loaded ahead
+constexpr int kSlots = kLead + 1 + kAhead;
+
+struct CarryArgs {
+  uint32_t A, psi, qinv, b, nq, many, slices;
+  uint32_t row0, rows, col0, cols;  // residues of this launch: [row0, row0+rows) x [col0, col0+cols)
+  uint32_t seg;                     // rows per CTA
+  uint32_t srows, scols;            // staged rows and columns (from row0, col0)
+  uint4* st16;                      // staged histograms: words e0 e1 e2 o0 ...
+  uint2* st8;                       // ... and o1 o2
+  unsigned long long* acc;          // [0, kMaxBins): residue pairs v < v'; then v = v'
+};
+
+// Counts of bins 8j + 2i (e[j], byte i) and 8j + 2i + 1 (o[j], byte i).
+struct H8 {
+  uint32_t e[3], o[3];
+};
+// Counts of bins 8j + m (low half of pm[j]) and 8j + 4 + m (high half).
+struct H16 {
+  uint32_t p0[4], p1[3], p2[3], p3[3];
+};
+template <int kLevel>
+using Hist = std::conditional_t<(kLevel <= 4), H8, H16>;
+
+__device__ __forceinline__ void zero(H8& h) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) h.e[j] = h.o[j] = 0;
+}
+__device__ __forceinline__ void zero(H16& h) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) h.p0[j] = h.p1[j] = h.p2[j] = h.p3[j] = 0;
+  h.p0[3] = 0;
+}
+
+// x + z y
+__device__ __forceinline__ H8 add_z(const H8& x, const H8& y) {
+  H8 r;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    r.e[j] = x.e[j] + (j ? __funnelshift_l(y.o[j - 1], y.o[j], 8) : y.o[0] << 8);
+    r.o[j] = x.o[j] + y.e[j];
+  }
+  return r;
+}
+__device__ __forceinline__ H16 add_z(const H16& x, const H16& y) {
+  H16 r;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    r.p0[j] = x.p0[j] + (j ? __funnelshift_l(y.p3[j - 1], y.p3[j], 16) : y.p3[0] << 16);
+    r.p1[j] = x.p1[j] + y.p0[j];
+    r.p2[j] = x.p2[j] + y.p1[j];
+    r.p3[j] = x.p3[j] + y.p2[j];
+  }
+  r.p0[3] = x.p0[3] + (y.p3[2] >> 16);
+  return r;
+}
+__device__ __forceinline__ H8 add(const H8& x, const H8& y) {
+  H8 r;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    r.e[j] = x.e[j] + y.e[j];
+    r.o[j] = x.o[j] + y.o[j];
+  }
+  return r;
+}
+__device__ __forceinline__ H16 add(const H16& x, const H16& y) {
+  H16 r;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    r.p0[j] = x.p0[j] + y.p0[j];
+    r.p1[j] = x.p1[j] + y.p1[j];
+    r.p2[j] = x.p2[j] + y.p2[j];
+    r.p3[j] = x.p3[j] + y.p3[j];
+  }
+  r.p0[3] = x.p0[3] + y.p0[3];
+  return r;
+}
+__device__ __forceinline__ H16 widen(const H8& h) {
+  H16 r;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    r.p0[j] = h.e[j] & 0x00FF00FFu;
+    r.p1[j] = h.o[j] & 0x00FF00FFu;
+    r.p2[j] = (h.e[j] >> 8) & 0x00FF00FFu;
+    r.p3[j] = (h.o[j] >> 8) & 0x00FF00FFu;
+  }
+  r.p0[3] = 0;
+  return r;
+}
+template <int kLevel>
+__device__ __forceinline__ Hist<kLevel> as_level(const Hist<kLevel - 1>& h) {
+  if constexpr (kLevel == 5) return widen(h);
+  else return h;
+}
+
+// One column's histogram in a shared exchange row: 24 bytes (8-bit counts) or 48
+// (16-bit counts below the last level, whose bins stop at 23), at strides that
+// make the vector accesses conflict-free.
+template <typename H>
+__host__ __device__ constexpr int slot_bytes() { return std::is_same_v<H, H8> ? 24 : 48; }
+__device__ __forceinline__ void put(uint8_t* row, int c, const H8& h) {
+  uint2* p = reinterpret_cast<uint2*>(row + c * 24);
+  p[0] = make_uint2(h.e[0], h.e[1]);
+  p[1] = make_uint2(h.e[2], h.o[0]);
+  p[2] = make_uint2(h.o[1], h.o[2]);
+}
+__device__ __forceinline__ void get(const uint8_t* row, int c, H8& h) {
+  const uint2* p = reinterpret_cast<const uint2*>(row + c * 24);
+  const uint2 x = p[0], y = p[1], w = p[2];
+  h.e[0] = x.x; h.e[1] = x.y; h.e[2] = y.x; h.o[0] = y.y; h.o[1] = w.x; h.o[2] = w.y;
+}
+__device__ __forceinline__ void put(uint8_t* row, int c, const H16& h) {
+  uint4* p = reinterpret_cast<uint4*>(row + c * 48);
+  p[0] = make_uint4(h.p0[0], h.p0[1], h.p0[2], h.p1[0]);
+  p[1] = make_uint4(h.p1[1], h.p1[2], h.p2[0], h.p2[1]);
+  p[2] = make_uint4(h.p2[2], h.p3[0], h.p3[1], h.p3[2]);
+}
+__device__ __forceinline__ void get(const uint8_t* row, int c, H16& h) {
+  const uint4* p = reinterpret_cast<const uint4*>(row + c * 48);
+  const uint4 x = p[0], y = p[1], w = p[2];
+  h.p0[0] = x.x; h.p0[1] = x.y; h.p0[2] = x.z; h.p1[0] = x.w;
+  h.p1[1] = y.x; h.p1[2] = y.y; h.p2[0] = y.z; h.p2[1] = y.w;
+  h.p2[2] = w.x; h.p3[0] = w.y; h.p3[1] = w.z; h.p3[2] = w.w;
+  h.p0[3] = 0;
+}
+
+// The first level from the four high-word distances: z^ha + z^hd + z (z^hb + z^hc).
+// Each distance adds 1 to a nibble (two nibbles per byte: bins 8 apart), a
+// distance of 16 to the count x.
+struct Nibbles {
+  uint32_t e = 0, o = 0, x = 0;
+  __device__ __forceinline__ void count(uint32_t h) {
+    const uint32_t one = 1u << (((h << 2) & 24u) | ((h >> 1) & 4u));
+    if (h & 1u) o += one;
+    else e += one;
+    x += h >> 4;
+  }
+  __device__ __forceinline__ H8 bytes() const {
+    const uint32_t ev = e - x;  // a distance of 16 was counted in bin 0, too
+    return H8{{ev & 0x0F0F0F0Fu, (ev >> 4) & 0x0F0F0F0Fu, x}, {o & 0x0F0F0F0Fu, (o >> 4) & 0x0F0F0F0Fu, 0u}};
+  }
+};
+__device__ __forceinline__ H8 first_level(uint32_t ra, uint32_t rb, uint32_t ca, uint32_t cb) {
+  Nibbles same, cross;
+  same.count(__popc(ra ^ ca));
+  same.count(__popc(rb ^ cb));
+  cross.count(__popc(ra ^ cb));
+  cross.count(__popc(rb ^ ca));
+  return add_z(same.bytes(), cross.bytes());
+}
+
+// One step in a running column: exchange with column c + s, combine, rotate the ring entry y.
+template <int kLevel>
+__device__ __forceinline__ Hist<kLevel> level(const Hist<kLevel - 1>& own, uint8_t* row, int c, int s,
+                                              Hist<kLevel>& y) {
+  put(row, c, own);
+  __syncthreads();
+  Hist<kLevel - 1> nb;
+  get(row, c + s, nb);
+  const Hist<kLevel> a = as_level<kLevel>(own), n = as_level<kLevel>(nb);
+  const Hist<kLevel> r = add(add_z(a, n), y);
+  y = add_z(n, a);
+  return r;
+}
+
+__device__ __forceinline__ uint32_t mul_mod(uint32_t a, uint32_t v, uint32_t A) {
+  return (uint32_t)((uint64_t)a * v % A);
+}
+__device__ __forceinline__ uint32_t sub_mod(uint32_t x, uint32_t d, uint32_t A) { return x >= d ? x - d : x + A - d; }
+
+// Shared bytes of the exchange rows: one per level after the first; with a single
+// one, two that take turns (a row's only barrier then separates them).
+template <int kBefore, int kLevels>
+__host__ __device__ constexpr int exchange_bytes(int cols) {
+  int n = 0;
+  for (int i = 1; i < kLevels; ++i) n += (kBefore + i <= 4 ? 24 : 48) * cols;
+  return kLevels == 2 ? 2 * n : n;
+}
+
+// ---------------------------------------------------------------- staging kernel
+// The kLevels largest steps (s = 16 * 2^(kLevels-1) .. 16) for a block of residue
+// pairs.  CTA: rows v = row0 + rho + 16 w for one rho and a run of w; columns v' =
+// col0 + sigma + 16 w' for four neighbouring sigma (so that the stores of a warp
+// fill sectors) and kStageCols consecutive w', of which the last 2^kLevels - 1
+// only feed their neighbours.
+template <int kLevels>
+__global__ void __launch_bounds__(kStageThreads) carry_stage_kernel(CarryArgs a) {
+  constexpr int kFirst = 1 << (kLevels - 1);
+  constexpr int kWarm = kFirst - 1;
+  constexpr int kUseful = kStageCols - ((1 << kLevels) - 1);
+  constexpr int kUnroll = kLevels >= 3 ? kFirst / 2 : 1;
+  constexpr int kCols = kStageThreads + 4 * kFirst;
+  __shared__ __align__(16) uint8_t ex[exchange_bytes<0, kLevels>(kCols) + 16];
+
+  const int tid = threadIdx.x, sub = tid & 3, wi = tid >> 2;
+  const uint32_t rho = blockIdx.y % kUnit, seg = blockIdx.y / kUnit;
+  const uint32_t sigma = (blockIdx.x & 3) * 4 + sub, w0 = (blockIdx.x >> 2) * kUseful;
+  const uint32_t wrows = (a.srows - rho + kUnit - 1) / kUnit;  // rows of this rho in the block
+  const uint32_t wr0 = seg * a.seg;
+  if (wr0 >= wrows) return;
+  const uint32_t wr1 = min(wrows, wr0 + a.seg);
+  // residue pairs v' < v are their mirror images; a final row reads staged rows up to 15 above it
+  {
+    const uint32_t vtop = a.col0 + (blockIdx.x & 3) * 4 + 3 + kUnit * (w0 + kUseful - 1);
+    if (vtop + 15 < a.row0 + rho + kUnit * wr0) return;
+  }
+  const uint32_t col = sigma + kUnit * (w0 + wi), vc = a.col0 + col;
+  const bool store = wi < kUseful && col < a.scols;
+  const uint32_t ca = mul_mod(a.psi, vc, a.A), cb = mul_mod(a.psi, vc + kUnit * kFirst, a.A);
+  const int total = ((int)(wr1 - wr0) + kWarm + kUnroll - 1) / kUnroll * kUnroll;
+  uint32_t w = wr0 + total - 1;  // descending
+  const uint32_t step = mul_mod(a.psi, kUnit, a.A);
+  uint32_t ra = mul_mod(a.psi, a.row0 + rho + kUnit * w, a.A);
+  uint32_t rb = mul_mod(a.psi, a.row0 + rho + kUnit * (w + kFirst), a.A);
+
+  H8 y4[4], y2[2], y1;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) zero(y4[i]);
+  zero(y2[0]); zero(y2[1]); zero(y1);
+  for (int it = 0; it < total; it += kUnroll) {
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u, --w) {
+      H8 h = first_level(ra, rb, ca, cb);
+      ra = sub_mod(ra, step, a.A);
+      rb = sub_mod(rb, step, a.A);
+      uint8_t* row = ex;
+      if constexpr (kLevels >= 4) { h = level<2>(h, row, tid, 4 * 4, y4[u & 3]); row += 24 * kCols; }
+      if constexpr (kLevels >= 3) { h = level<2>(h, row, tid, 4 * 2, y2[u & 1]); row += 24 * kCols; }
+      if constexpr (kLevels == 2) row += ((it + u) & 1) * 24 * kCols;
+      if constexpr (kLevels >= 2) h = level<2>(h, row, tid, 4, y1);
+      if (store && w < wr1) {
+        const size_t at = (size_t)(rho + kUnit * w) * a.scols + col;
+        a.st16[at] = make_uint4(h.e[0], h.e[1], h.e[2], h.o[0]);
+        a.st8[at] = make_uint2(h.o[1], h.o[2]);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------- folding kernel
+template <int kOffset>
+__device__ __forceinline__ void red_add(uint32_t addr, uint32_t x) {
+  asm volatile("red.shared.add.u32 [%0+%1], %2;" ::"r"(addr), "n"(kOffset), "r"(x) : "memory");
+}
+
+// Adds f x (the counts of h) to a lane's table column, bin d at at + 128 d.  kWide:
+// products of 64 bits, low 16 bits to the first table, the rest to the one hi bytes on.
+constexpr int kTabBytes = kTabRows * 128;
+template <bool kWide, int kBin>
+__device__ __forceinline__ void add_bin(uint32_t at, uint32_t f, uint32_t x) {
+  if constexpr (kWide) {
+    const unsigned long long p = (unsigned long long)f * x;
+    red_add<kBin * 128>(at, (uint32_t)p & 0xFFFFu);
+    red_add<kBin * 128 + 2 * kTabBytes>(at, (uint32_t)(p >> 16));
+  } else {
+    red_add<kBin * 128>(at, x);
+  }
+}
+template <bool kWide, int kBin>
+__device__ __forceinline__ void add_bytes(uint32_t at, uint32_t f, uint32_t w) {
+  if (w) {
+    add_bin<kWide, kBin>(at, f, w & 0xFFu);
+    add_bin<kWide, kBin + 2>(at, f, (w >> 8) & 0xFFu);
+    add_bin<kWide, kBin + 4>(at, f, (w >> 16) & 0xFFu);
+    add_bin<kWide, kBin + 6>(at, f, w >> 24);
+  }
+}
+template <bool kWide, int kBin>
+__device__ __forceinline__ void add_halves(uint32_t at, uint32_t f, uint32_t w) {
+  if (w) {
+    add_bin<kWide, kBin>(at, f, w & 0xFFFFu);
+    add_bin<kWide, kBin + 4>(at, f, w >> 16);
+  }
+}
+template <bool kWide>
+__device__ __forceinline__ void add_hist(uint32_t at, uint32_t f, const H8& h) {
+  add_bytes<kWide, 0>(at, f, h.e[0]); add_bytes<kWide, 1>(at, f, h.o[0]);
+  add_bytes<kWide, 8>(at, f, h.e[1]); add_bytes<kWide, 9>(at, f, h.o[1]);
+  add_bytes<kWide, 16>(at, f, h.e[2]); add_bytes<kWide, 17>(at, f, h.o[2]);
+}
+template <bool kWide>
+__device__ __forceinline__ void add_hist(uint32_t at, uint32_t f, const H16& h) {
+  add_halves<kWide, 0>(at, f, h.p0[0]); add_halves<kWide, 1>(at, f, h.p1[0]);
+  add_halves<kWide, 2>(at, f, h.p2[0]); add_halves<kWide, 3>(at, f, h.p3[0]);
+  add_halves<kWide, 8>(at, f, h.p0[1]); add_halves<kWide, 9>(at, f, h.p1[1]);
+  add_halves<kWide, 10>(at, f, h.p2[1]); add_halves<kWide, 11>(at, f, h.p3[1]);
+  add_halves<kWide, 16>(at, f, h.p0[2]); add_halves<kWide, 17>(at, f, h.p1[2]);
+  add_halves<kWide, 18>(at, f, h.p2[2]); add_halves<kWide, 19>(at, f, h.p3[2]);
+  add_halves<kWide, 24>(at, f, h.p0[3]);
+}
+
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
+
+template <int kBefore>
+__host__ __device__ constexpr int fold_threads() { return kBefore ? kFoldThreads : kLeafThreads; }
+
+// Shared memory of the folding kernel: tables (U and D, twice for wide products),
+// exchange rows, the ring of staged rows, and the q-distance counts of each thread (many).
+template <int kBefore, int kLevels>
+constexpr size_t fold_smem(bool many) {
+  constexpr int nt = fold_threads<kBefore>(), cols = nt + (1 << (kLevels - 1));
+  size_t n = (size_t)kTabBytes * (many ? 4 : 2) + exchange_bytes<kBefore, kLevels>(cols);
+  if (kBefore) n += (size_t)kSlots * cols * 24;
+  if (many) n += (size_t)(16 + 1) * nt * 4;
+  return n + 32;
+}
+
+// The last kLevels steps (s = 2^(kLevels-1) .. 1) and the sum over q, q'.  kBefore:
+// levels already in the staged input (0: the input is the popcounts).  CTA: a
+// strip of columns (one per thread, the last 2^kLevels - 1 only feed their
+// neighbours) x a segment of rows.
+template <int kBefore, int kLevels, bool kMany>
+__global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carry_fold_kernel(CarryArgs a) {
+  constexpr int kThreads = fold_threads<kBefore>();
+  constexpr int kFirst = 1 << (kLevels - 1);
+  constexpr int kWarm = kFirst - 1;
+  constexpr int kUseful = kThreads - ((1 << kLevels) - 1);
+  constexpr int kUnroll = kLevels >= 3 ? kFirst / 2 : 1;
+  constexpr int kCols = kThreads + kFirst;
+  constexpr int kL1 = kBefore + 1;
+  constexpr int kLast = kBefore + kLevels;
+  extern __shared__ __align__(16) uint8_t smem[];
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t r0 = blockIdx.y * a.seg;
+  if (r0 >= a.rows) return;
+  const uint32_t r1 = min(a.rows, r0 + a.seg);
+  const uint32_t c0 = blockIdx.x * kUseful;
+  if (c0 >= a.cols) return;
+  if (a.col0 + min(a.cols, c0 + kUseful) <= a.row0 + r0) return;  // no v' >= v here
+
+  // shared memory
+  uint32_t* tab = reinterpret_cast<uint32_t*>(smem);  // U, D (and their high parts)
+  uint8_t* ex = smem + kTabBytes * (kMany ? 4 : 2);
+  uint4* in16 = reinterpret_cast<uint4*>(ex + exchange_bytes<kBefore, kLevels>(kCols));
+  uint2* in8 = reinterpret_cast<uint2*>(in16 + (kBefore ? kSlots * kCols : 0));
+  uint32_t* qd = reinterpret_cast<uint32_t*>(in8 + (kBefore ? kSlots * kCols : 0));
+  for (int i = tid; i < kTabBytes * (kMany ? 4 : 2) / 4; i += kThreads) tab[i] = 0;
+  if constexpr (kMany)
+    for (int i = tid; i < 17 * kThreads; i += kThreads) qd[i] = 0;
+
+  const uint32_t col = c0 + tid, vc = a.col0 + col;
+  const bool mine = tid < kUseful && col < a.cols;
+  const uint32_t qc = mul_mod(a.qinv, vc, a.A);
+  const int total = ((int)(r1 - r0) + kWarm + kUnroll - 1) / kUnroll * kUnroll;
+  uint32_t r = r0 + total - 1;  // descending, from row0
+  uint32_t qr = mul_mod(a.qinv, a.row0 + r, a.A);
+  const uint32_t tab_u = (uint32_t)__cvta_generic_to_shared(tab) + lane * 4u;
+
+  // input: popcounts, or staged rows through a ring of kSlots rows
+  uint32_t ca = 0, cb = 0, ra = 0, rb = 0;
+  int slot = 0;  // ring slot of load number it (row r + kLead of that step)
+  uint32_t scol = 0;
+  auto load = [&](int sl, uint32_t row) {
+    const size_t at = (size_t)min(row, a.srows - 1) * a.scols;
+    copy_async16(in16 + sl * kCols + tid, a.st16 + at + scol);
+    copy_async8(in8 + sl * kCols + tid, a.st8 + at + scol);
+    copy_commit();
+  };
+  if constexpr (kBefore == 0) {
+    ca = mul_mod(a.psi, vc, a.A);
+    cb = mul_mod(a.psi, vc + kFirst, a.A);
+    ra = mul_mod(a.psi, a.row0 + r, a.A);
+    rb = mul_mod(a.psi, a.row0 + r + kFirst, a.A);
+  } else {
+    scol = min(col, a.scols - 1);
+    for (int l = 0; l < kLead + kAhead; ++l) load(l, r + kLead - l);
+    copy_wait<kAhead - 1>();
+  }
+  __syncthreads();
+
+  Hist<kBefore ? (kLevels == 4 ? kLast - 2 : 1) : 1> y4[4];
+  Hist<kBefore ? kLast - 1 : 1> y2[2];
+  Hist<kLast> y1;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) zero(y4[i]);
+  zero(y2[0]); zero(y2[1]); zero(y1);
+
+  for (int it = 0; it < total; it += kUnroll) {
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u, --r) {
+      // first level
+      Hist<kL1> h1;
+      if constexpr (kBefore == 0) {
+        h1 = first_level(ra, rb, ca, cb);
+        ra = sub_mod(ra, a.psi, a.A);
+        rb = sub_mod(rb, a.psi, a.A);
+      } else {
+        auto fetch = [&](int sl, int c) {
+          const uint4 x = in16[sl * kCols + c];
+          const uint2 w = in8[sl * kCols + c];
+          return as_level<kL1>(H8{{x.x, x.y, x.z}, {x.w, w.x, w.y}});
+        };
+        const int lo = slot, hi = slot + kLead < kSlots ? slot + kLead : slot + kLead - kSlots;
+        h1 = add_z(add(fetch(hi, tid), fetch(lo, tid + kFirst)), add(fetch(hi, tid + kFirst), fetch(lo, tid)));
+        int nx = slot + kLead + kAhead;
+        if (nx >= kSlots) nx -= kSlots;
+        // r + kLead - (kLead + kAhead): rows below the block's first are never used
+        load(nx, r >= kAhead ? r - kAhead : 0u);
+        slot = slot + 1 == kSlots ? 0 : slot + 1;
+        copy_wait<kAhead - 1>();
+      }
+      // remaining levels
+      uint8_t* row = ex;
+      Hist<kLast> g;
+      if constexpr (kLevels == 1) {
+        g = h1;
+      } else if constexpr (kLevels == 2) {
+        g = level<kLast>(h1, row + ((it + u) & 1) * slot_bytes<Hist<kL1>>() * kCols, tid, 1, y1);
+      } else if constexpr (kLevels == 3) {
+        const Hist<kLast - 1> h2 = level<kLast - 1>(h1, row, tid, 2, y2[u & 1]);
+        row += slot_bytes<Hist<kL1>>() * kCols;
+        g = level<kLast>(h2, row, tid, 1, y1);
+      } else {
+        const Hist<kLast - 2> h2 = level<kLast - 2>(h1, row, tid, 4, y4[u & 3]);
+        row += slot_bytes<Hist<kL1>>() * kCols;
+        const Hist<kLast - 1> h3 = level<kLast - 1>(h2, row, tid, 2, y2[u & 1]);
+        row += slot_bytes<Hist<kLast - 2>>() * kCols;
+        g = level<kLast>(h3, row, tid, 1, y1);
+      }
+      // fold: every q of row residue v with every q' of column residue v'
+      const uint32_t v = a.row0 + r;
+      if (mine && r < r1 && vc >= v) {
+        const uint32_t at = tab_u + (vc == v ? kTabBytes : 0);
+        if constexpr (!kMany) {
+          const bool c2 = qc + a.A < a.nq;
+          add_hist<false>(at + (__popc(qr ^ qc) << 7), 1, g);
+          if (c2) add_hist<false>(at + (__popc(qr ^ (qc + a.A)) << 7), 1, g);
+          if (qr + a.A < a.nq) {
+            add_hist<false>(at + (__popc((qr + a.A) ^ qc) << 7), 1, g);
+            if (c2) add_hist<false>(at + (__popc((qr + a.A) ^ (qc + a.A)) << 7), 1, g);
+          }
+        } else {
+          uint32_t* f = qd + tid;
+          for (uint32_t q = qr + blockIdx.z * a.A; q < a.nq; q += a.slices * a.A)
+            for (uint32_t p = qc; p < a.nq; p += a.A) f[__popc(q ^ p) * kThreads] += 1;
+          for (uint32_t d = 0; d <= 16; ++d) {
+            const uint32_t x = f[d * kThreads];
+            if (x) {
+              f[d * kThreads] = 0;
+              add_hist<true>(at + (d << 7), x, g);
+            }
+          }
+        }
+      }
+      qr = sub_mod(qr, a.qinv, a.A);
+    }
+  }
+  if constexpr (kBefore != 0) copy_wait<0>();
+  __syncthreads();
+  // tables -> global sums
+  for (int d = warp; d < 2 * kTabRows; d += kThreads / 32) {
+    const uint32_t x = tab[d * 32 + lane];
+    unsigned long long t = (unsigned long long)__reduce_add_sync(0xffffffffu, x & 0xFFFFu) +
+                           ((unsigned long long)__reduce_add_sync(0xffffffffu, x >> 16) << 16);
+    if constexpr (kMany) {
+      const uint32_t y = tab[(2 * kTabRows + d) * 32 + lane];
+      t += ((unsigned long long)__reduce_add_sync(0xffffffffu, y & 0xFFFFu) << 16) +
+           ((unsigned long long)__reduce_add_sync(0xffffffffu, y >> 16) << 32);
+    }
+    if (lane == 0 && t) atomicAdd(a.acc + (d < kTabRows ? d : kMaxBins + d - kTabRows), t);
+  }
+}
+
+// Residue pairs v < v' stand for one unordered pair of codewords each; pairs of
+// one residue were counted in both orders, and each codeword with itself.
+__global__ void carry_finish_kernel(const Job* jobs, const unsigned long long* acc) {
+  const Job& j = jobs[blockIdx.x];
+  const unsigned long long* t = acc + (size_t)blockIdx.x * 2 * kMaxBins;
+  const uint32_t d = threadIdx.x;
+  j.bins[d] = t[d] + (t[kMaxBins + d] - (d == 0 ? 1ull << j.n : 0ull)) / 2;
+}
+
+template <int kBefore, int kLevels, bool kMany>
+cudaError_t run_fold(const CarryArgs& a, uint32_t slices, cudaStream_t stream) {
+  constexpr int nt = fold_threads<kBefore>(), useful = nt - ((1 << kLevels) - 1);
+  constexpr size_t smem = fold_smem<kBefore, kLevels>(kMany);
+  auto fn = carry_fold_kernel<kBefore, kLevels, kMany>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((a.cols + useful - 1) / useful, (a.rows + a.seg - 1) / a.seg, slices);
+  fn<<<grid, nt, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
+template <int kBefore, int kLevels>
+cudaError_t run_fold(const CarryPlan& p, const CarryArgs& a, cudaStream_t stream) {
+  return p.many ? run_fold<kBefore, kLevels, true>(a, p.slices, stream)
+                : run_fold<kBefore, kLevels, false>(a, 1, stream);
+}
+
+template <int kLevels>
+cudaError_t run_stage(CarryArgs a, cudaStream_t stream) {
+  constexpr uint32_t useful = kStageCols - ((1 << kLevels) - 1);
+  const uint32_t w = (a.scols + kUnit - 1) / kUnit, wr = (a.srows + kUnit - 1) / kUnit;
+  a.seg = (wr + (wr + 63) / 64 - 1) / ((wr + 63) / 64);
+  const dim3 grid(4 * ((w + useful - 1) / useful), kUnit * ((wr + a.seg - 1) / a.seg));
+  carry_stage_kernel<kLevels><<<grid, kStageThreads, 0, stream>>>(a);
+  return cudaGetLastError();
+}
+
+uint32_t inverse_pow2(uint32_t e, uint32_t A) {  // 2^-e mod A, A odd
+  uint64_t x = 1 % A;
+  const uint64_t half = (A + 1) / 2 % A;
+  for (uint32_t i = 0; i < e; ++i) x = x * half % A;
+  return (uint32_t)x;
+}
+
+uint32_t odd_part(uint64_t A) {
+  while (A && !(A & 1)) A >>= 1;
+  return (uint32_t)A;
+}
+uint32_t bits_of(uint32_t x) {
+  uint32_t n = 0;
+  for (; x; x >>= 1) ++n;
+  return n;
+}
+
+}  // namespace
+
+bool carry_eligible(const Job& j) {
+  if (j.kind != JOB_PAIRS || j.shape != SHAPE_TRIANGLE || j.row_kind != ROW_PROGRESSION ||
+      j.col_kind != COL_PROGRESSION || j.tile_offset != 0 || j.A == 0 || (j.A >> 32) || j.n > 24)
+    return false;
+  const uint32_t a = bits_of(odd_part(j.A));
+  return a <= 16 && j.n > a;
+}
+
+// Residue pairs cost about as much as the tcgen05 kernel's 16^2 codeword pairs
+// (16-bit A: k = 19, 17.9 ms here and 15.3 ms there; k = 20, 26.8 and 63.5 ms); below
+// k = 14 a launch of the popc kernel takes no longer than this path's three.
+bool carry_wins(const Job& j) {
+  const uint32_t a = bits_of(odd_part(j.A));
+  return j.n >= a + 4 && j.n >= 14;
+}
+
+void carry_plan(const Job& j, int num_sms, CarryPlan& p) {
+  p = CarryPlan();
+  p.A = odd_part(j.A);
+  p.k = j.n;
+  p.b = std::min<uint32_t>(8, p.k - bits_of(p.A));
+  p.s = p.k - p.b;
+  p.staged = p.b > 4 ? p.b - 4 : 0;
+  p.psi = (p.A - inverse_pow2(p.k, p.A)) % p.A;
+  p.qinv = inverse_pow2(p.b, p.A);
+  const uint64_t nq = 1ull << p.s;
+  p.many = nq > 2ull * p.A;
+  if (p.staged) {
+    const uint32_t useful = kStageCols - ((1u << p.staged) - 1);
+    p.side = std::min(p.A, kUnit * useful * 3 - 15);
+    p.pitch = p.side + 15;
+    p.cells = (size_t)p.pitch * p.pitch;
+  } else {
+    p.side = p.A;
+  }
+  // rows per CTA: long runs amortise the rows a segment computes twice; short ones
+  // where the residue square would leave SMs without a CTA
+  const uint32_t useful = p.staged ? kFoldThreads - 15 : kLeafThreads - ((1u << p.b) - 1);
+  const uint64_t strips = (p.side + useful - 1) / useful;
+  p.seg = 256;
+  while (p.seg > 16 && strips * ((p.side + p.seg - 1) / p.seg) < 8ull * num_sms) p.seg /= 2;
+  if (p.many) {
+    const uint64_t ctas = strips * ((p.side + p.seg - 1) / p.seg), per = (nq + p.A - 1) / p.A;
+    p.slices = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(per, 4096), std::max<uint64_t>(1, 8ull * num_sms / ctas));
+  }
+}
+
+size_t carry_stage_bytes(const CarryPlan& p) { return p.staged ? p.cells * 24 + 256 : 0; }
+
+cudaError_t launch_carry(const CarryPlan& p, unsigned long long* acc, void* stage, cudaStream_t stream) {
+  cudaError_t e = cudaSuccess;
+  CarryArgs a{};
+  a.A = p.A;
+  a.psi = p.psi;
+  a.qinv = p.qinv;
+  a.b = p.b;
+  a.nq = 1u << p.s;
+  a.many = p.many;
+  a.slices = p.slices;
+  a.acc = acc;
+  a.seg = p.seg;
+  if (!p.staged) {
+    a.rows = a.cols = p.A;
+    switch (p.b) {
+      case 1: e = run_fold<0, 1>(p, a, stream); break;
+      case 2: e = run_fold<0, 2>(p, a, stream); break;
+      case 3: e = run_fold<0, 3>(p, a, stream); break;
+      default: e = run_fold<0, 4>(p, a, stream); break;
+    }
+  } else {
+    a.st16 = static_cast<uint4*>(stage);
+    a.st8 = reinterpret_cast<uint2*>(a.st16 + p.cells);
+    for (uint32_t r0 = 0; r0 < p.A && e == cudaSuccess; r0 += p.side)
+      for (uint32_t c0 = r0; c0 < p.A && e == cudaSuccess; c0 += p.side) {
+        a.row0 = r0;
+        a.col0 = c0;
+        a.rows = std::min(p.side, p.A - r0);
+        a.cols = std::min(p.side, p.A - c0);
+        a.srows = a.rows + 15;
+        a.scols = a.cols + 15;
+        switch (p.staged) {
+          case 1: e = run_stage<1>(a, stream); if (e == cudaSuccess) e = run_fold<1, 4>(p, a, stream); break;
+          case 2: e = run_stage<2>(a, stream); if (e == cudaSuccess) e = run_fold<2, 4>(p, a, stream); break;
+          case 3: e = run_stage<3>(a, stream); if (e == cudaSuccess) e = run_fold<3, 4>(p, a, stream); break;
+          default: e = run_stage<4>(a, stream); if (e == cudaSuccess) e = run_fold<4, 4>(p, a, stream); break;
+        }
+      }
+  }
+  return e;
+}
+
+cudaError_t launch_carry_finish(const Job* jobs, const unsigned long long* acc, uint32_t n, cudaStream_t stream) {
+  carry_finish_kernel<<<n, kMaxBins, 0, stream>>>(jobs, acc);
+  return cudaGetLastError();
+}
+
+}  // namespace dd

@@ -1,0 +1,42 @@
+// dd_carry.h — exhaustive AN histograms by residue-pair counting (see dd_carry.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <cstddef>
+#include <cstdint>
+
+#include "dd_jobs.h"
+
+namespace dd {
+
+// One job as the carry kernels run it.
+struct CarryPlan {
+  uint32_t A = 0;       // odd part of the multiplier
+  uint32_t k = 0;       // data bits
+  uint32_t b = 0;       // window bits: levels of the pair recursion
+  uint32_t s = 0;       // k - b: bits enumerated at the end
+  uint32_t staged = 0;  // levels the staging kernel computes (b - 4 when b > 4, else 0)
+  uint32_t psi = 0;     // high word of t: psi * t mod A
+  uint32_t qinv = 0;    // first q of residue v: qinv * v mod A
+  uint32_t many = 0;    // a residue has more than two q
+  uint32_t slices = 1;  // many: CTAs that share a tile's q rows
+  uint32_t side = 0;    // residues per side of a staged block (staged > 0)
+  uint32_t pitch = 0;   // staged columns
+  uint32_t seg = 0;     // residue rows per CTA of the folding kernel
+  size_t cells = 0;     // staged histograms of one block
+};
+
+// AN exhaustive jobs over the whole instance, A's odd part of at most 16 bits, k <= 24.
+bool carry_eligible(const Job& j);
+// The rule that picks this path for an eligible job under AUTO.
+bool carry_wins(const Job& j);
+void carry_plan(const Job& j, int num_sms, CarryPlan& p);
+// Bytes of staging memory a plan needs (0: none).
+size_t carry_stage_bytes(const CarryPlan& p);
+// Enqueues one job's kernels: its sums are added to acc (2 x kMaxBins uint64, zeroed
+// by the caller); stage is carry_stage_bytes(p) bytes, free for the next job in the
+// stream afterwards.
+cudaError_t launch_carry(const CarryPlan& p, unsigned long long* acc, void* stage, cudaStream_t stream);
+// acc of n jobs (2 x kMaxBins each) -> their bins; jobs: the device's table entries.
+cudaError_t launch_carry_finish(const Job* jobs, const unsigned long long* acc, uint32_t n, cudaStream_t stream);
+
+}  // namespace dd

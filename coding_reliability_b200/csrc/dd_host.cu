@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/codrel_b200.h"
+#include "dd_carry.h"
 #include "dd_device.cuh"
 #include "dd_host.h"
 #include "dd_kernels.h"
@@ -28,11 +29,13 @@ struct dd_context {
   bool own_stream = false;
   int num_sms = 0;
   // device state
-  unsigned long long* d_bins = nullptr;  // bin_slots x kMaxBins
+  unsigned long long* d_bins = nullptr;  // bin_slots x kMaxBins, then the carry path's sums (2 x kMaxBins a slot)
   uint32_t bin_slots = 0;
   unsigned long long* d_ctl = nullptr;   // [0] popc work counter, [1] MMA work counter, [2] status, [3..15] diagnostics
   dd::Job* d_jobs = nullptr;
   uint32_t job_cap = 0;
+  void* d_stage = nullptr;               // carry path: staged histograms of one block
+  size_t stage_cap = 0;
   // pinned host mirrors
   unsigned long long* h_bins = nullptr;
   unsigned long long* h_ctl = nullptr;
@@ -89,7 +92,7 @@ static int ensure_capacity(dd_context* ctx, uint32_t slots, uint32_t njobs) {
     ctx->h_bins = nullptr;
     ctx->bin_slots = 0;
     const uint32_t cap = std::max<uint32_t>(slots, 64);
-    cudaError_t e = cudaMalloc(&ctx->d_bins, (size_t)cap * kMaxBins * sizeof(unsigned long long));
+    cudaError_t e = cudaMalloc(&ctx->d_bins, (size_t)cap * 3 * kMaxBins * sizeof(unsigned long long));
     if (e != cudaSuccess) { set_error("bins: cudaMalloc failed"); return DD_ERR_OUT_OF_MEMORY; }
     DD_CUDA(cudaMallocHost(&ctx->h_bins, (size_t)cap * kMaxBins * sizeof(unsigned long long)));
     ctx->bin_slots = cap;
@@ -109,6 +112,24 @@ static int ensure_capacity(dd_context* ctx, uint32_t slots, uint32_t njobs) {
   return DD_OK;
 }
 
+// Staging memory of the carry path, kept by the context and grown on demand; false
+// when the device has no room for it (its jobs then take the pair kernels).
+static bool ensure_stage(dd_context* ctx, size_t bytes) {
+  if (bytes <= ctx->stage_cap) return true;
+  drop_graph(ctx);
+  if (ctx->d_stage) cudaFree(ctx->d_stage);
+  ctx->d_stage = nullptr;
+  ctx->stage_cap = 0;
+  if (cudaMalloc(&ctx->d_stage, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  ctx->stage_cap = bytes;
+  return true;
+}
+
+enum Route : uint32_t { ROUTE_POPC = 0, ROUTE_MMA = 1, ROUTE_CARRY = 2 };
+
 struct LaunchPlan {
   LaunchArgs pargs;          // popc kernel: table entries [0, npopc)
   int pgrid = 0;
@@ -118,6 +139,7 @@ struct LaunchPlan {
   int mgrid = 0;
   size_t msmem = 0;
   uint32_t nmma = 0;
+  std::vector<CarryPlan> carry;  // carry path: the table entries after those
   uint32_t nslots = 0;       // bin slots (one per request, in request order)
 };
 
@@ -145,27 +167,41 @@ static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel) {
   return ctx->tuned == 2 && pairs >= kMmaMinPairs;  // autotuner's verdict for AN exhaustive shapes
 }
 
-// Orders the job table (popc jobs first, then MMA jobs), assigns tile ranges
-// and bin slots (slot = request index), and sizes both persistent grids.
-static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vector<uint32_t>& kernels,
+// The route of a whole instance: the carry path where it is asked for or wins
+// (carry_wins) and its staging memory is to be had, else a pair kernel.
+static Route route_of(dd_context* ctx, const Job& j, uint32_t kernel) {
+  if (carry_eligible(j) && (kernel == DD_KERNEL_CARRY || (kernel == DD_KERNEL_AUTO && carry_wins(j)))) {
+    CarryPlan p;
+    carry_plan(j, ctx->num_sms, p);
+    if (ensure_stage(ctx, carry_stage_bytes(p))) return ROUTE_CARRY;
+  }
+  return want_mma(ctx, j, kernel) ? ROUTE_MMA : ROUTE_POPC;
+}
+
+// Orders the job table (popc jobs first, then MMA jobs, then carry jobs), assigns
+// tile ranges and bin slots (slot = request index), and sizes both persistent grids.
+static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vector<Route>& routes,
                        LaunchPlan& lp, bool own_bins = true) {
   std::vector<Job> table;
   table.reserve(jobs.size());
-  for (int pass = 0; pass < 2; ++pass)
+  uint32_t of_route[3] = {0, 0, 0};
+  for (uint32_t route = 0; route < 3; ++route)
     for (size_t i = 0; i < jobs.size(); ++i) {
-      const bool m = want_mma(ctx, jobs[i], kernels[i]);
-      if ((pass == 1) != m) continue;
+      if (routes[i] != route) continue;
       Job j = jobs[i];
       if (own_bins) j.bins = ctx->d_bins + i * kMaxBins;
       table.push_back(j);
+      ++of_route[route];
     }
   lp.nslots = (uint32_t)jobs.size();
   uint64_t tp = 0, tm = 0;
   uint32_t maxb = 1, maxbm = 1;
   bool col_table = false;
-  lp.npopc = 0;
-  for (size_t i = 0; i < jobs.size(); ++i) lp.npopc += want_mma(ctx, jobs[i], kernels[i]) ? 0 : 1;
-  lp.nmma = (uint32_t)table.size() - lp.npopc;
+  lp.npopc = of_route[ROUTE_POPC];
+  lp.nmma = of_route[ROUTE_MMA];
+  lp.carry.resize(of_route[ROUTE_CARRY]);
+  for (size_t c = 0; c < lp.carry.size(); ++c) carry_plan(table[lp.npopc + lp.nmma + c], ctx->num_sms, lp.carry[c]);
+  const uint32_t pair_jobs = lp.npopc + lp.nmma;
   for (uint32_t k = 0; k < lp.npopc; ++k) {
     Job& j = table[k];
     j.tile_begin = tp;
@@ -173,7 +209,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
     maxb = std::max(maxb, j.nbins);
     col_table |= (j.kind == JOB_PAIRS && j.col_kind == COL_HAMMING_EXT && !j.wide);
   }
-  for (uint32_t k = lp.npopc; k < table.size(); ++k) {
+  for (uint32_t k = lp.npopc; k < pair_jobs; ++k) {
     Job& j = table[k];
     j.tile_begin = tm;
     tm += j.tiles;
@@ -200,7 +236,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.margs.njobs = lp.nmma;
   // rows for every distance an operand can produce (<= L), flagged at flush when >= nbins
   uint32_t maxl = 0;
-  for (uint32_t k = lp.npopc; k < table.size(); ++k) maxl = std::max(maxl, (uint32_t)mma_operand_bits(table[k]));
+  for (uint32_t k = lp.npopc; k < pair_jobs; ++k) maxl = std::max(maxl, (uint32_t)mma_operand_bits(table[k]));
   lp.margs.hist_rows = std::max(maxbm, maxl + 1);
   lp.margs.total_tiles = tm;
   lp.margs.counter = ctx->d_ctl + 1;
@@ -214,10 +250,10 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
       // one joint table for the launch, sized for its largest S; each job's
       // window of d2 rows and its packing parameters follow from it
       uint32_t smax = 1;
-      for (uint32_t k = lp.npopc; k < table.size(); ++k)
+      for (uint32_t k = lp.npopc; k < pair_jobs; ++k)
         smax = std::max(smax, (uint32_t)mma_max_distance(table[k]) + 1u);
       mma_pk_layout(smax, &lp.margs.pk_cells, &lp.margs.b_bufs);
-      for (uint32_t k = lp.npopc; k < table.size(); ++k) mma_pack_setup(table[k], lp.margs.pk_cells);
+      for (uint32_t k = lp.npopc; k < pair_jobs; ++k) mma_pack_setup(table[k], lp.margs.pk_cells);
     } else {
       lp.margs.b_bufs = mma_b_bufs(lp.margs.hist_rows);
     }
@@ -232,8 +268,10 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
 // by events), bins + status D2H.
 static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing) {
   cudaStream_t s = ctx->stream;
-  const uint32_t njobs = lp.npopc + lp.nmma;
+  const uint32_t ncarry = (uint32_t)lp.carry.size(), njobs = lp.npopc + lp.nmma + ncarry;
   DD_CUDA(cudaMemcpyAsync(ctx->d_jobs, ctx->h_jobs, njobs * sizeof(Job), cudaMemcpyHostToDevice, s));
+  unsigned long long* acc = ctx->d_bins + (size_t)ctx->bin_slots * kMaxBins;
+  if (ncarry) DD_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncarry * 2 * kMaxBins * sizeof(unsigned long long), s));
   DD_CUDA(cudaMemsetAsync(ctx->d_bins, 0, (size_t)lp.nslots * kMaxBins * sizeof(unsigned long long), s));
   DD_CUDA(cudaMemsetAsync(ctx->d_ctl, 0, kCtlWords * sizeof(unsigned long long), s));
   // Inside a stream capture the records must be external so that they become
@@ -243,6 +281,9 @@ static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing)
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev0, s, evflags));
   if (lp.pgrid) DD_CUDA(launch_hist(ctx->hist_mode, lp.pargs, lp.pgrid, lp.psmem, s));
   if (lp.mgrid) DD_CUDA(launch_mma(lp.margs, lp.mgrid, lp.msmem, s));
+  for (uint32_t c = 0; c < ncarry; ++c)
+    DD_CUDA(launch_carry(lp.carry[c], acc + (size_t)c * 2 * kMaxBins, ctx->d_stage, s));
+  if (ncarry) DD_CUDA(launch_carry_finish(ctx->d_jobs + lp.npopc + lp.nmma, acc, ncarry, s));
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev1, s, evflags));
   DD_CUDA(cudaMemcpyAsync(ctx->h_bins, ctx->d_bins, (size_t)lp.nslots * kMaxBins * sizeof(unsigned long long),
                           cudaMemcpyDeviceToHost, s));
@@ -272,8 +313,11 @@ static int check_status(dd_context* ctx) {
 int launch_round(dd_context* ctx, std::vector<Job>& jobs, const std::vector<uint32_t>& kernels, float* kernel_ms) {
   int st = ensure_capacity(ctx, 1, (uint32_t)jobs.size());
   if (st != DD_OK) return st;
+  // tile sub-ranges are the pair kernels' work
+  std::vector<Route> routes(jobs.size());
+  for (size_t i = 0; i < jobs.size(); ++i) routes[i] = want_mma(ctx, jobs[i], kernels[i]) ? ROUTE_MMA : ROUTE_POPC;
   LaunchPlan lp;
-  st = plan_launch(ctx, jobs, kernels, lp, false);
+  st = plan_launch(ctx, jobs, routes, lp, false);
   if (st != DD_OK) return st;
   cudaStream_t s = ctx->stream;
   const uint32_t njobs = lp.npopc + lp.nmma;
@@ -396,6 +440,7 @@ int dd_context_destroy(dd_context* ctx) {
   if (ctx->d_ctl) cudaFree(ctx->d_ctl);
   if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
   if (ctx->d_jobs) cudaFree(ctx->d_jobs);
+  if (ctx->d_stage) cudaFree(ctx->d_stage);
   if (ctx->h_bins) cudaFreeHost(ctx->h_bins);
   if (ctx->h_jobs) cudaFreeHost(ctx->h_jobs);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -471,7 +516,6 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
   const double t0 = now_ms();
   std::vector<Shape> shapes(count);
   std::vector<Job> jobs;
-  std::vector<uint32_t> kernels(count);
   jobs.reserve(count);
   for (uint32_t i = 0; i < count; ++i) {
     std::string err;
@@ -481,7 +525,6 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
       return st;
     }
     plan_jobs(shapes[i], reqs[i], jobs);
-    kernels[i] = reqs[i].kernel;
   }
   if (continued) {
     Job& j = jobs[0];
@@ -490,12 +533,14 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
   }
   int st = ensure_capacity(ctx, count, count);
   if (st != DD_OK) return st;
+  std::vector<Route> routes(count);
+  for (uint32_t i = 0; i < count; ++i) routes[i] = route_of(ctx, jobs[i], reqs[i].kernel);
   LaunchPlan lp;
-  st = plan_launch(ctx, jobs, kernels, lp);
+  st = plan_launch(ctx, jobs, routes, lp);
   if (st != DD_OK) return st;
   cudaStream_t s = ctx->stream;
   if (use_graph) {
-    const size_t nj = lp.npopc + lp.nmma;
+    const size_t nj = lp.npopc + lp.nmma + lp.carry.size();
     const bool same = ctx->gexec && ctx->gjobs.size() == nj && ctx->ggrid[0] == lp.pgrid &&
                       ctx->ggrid[1] == lp.mgrid && ctx->gsmem[0] == lp.psmem && ctx->gsmem[1] == lp.msmem &&
                       ctx->ghist_mode == ctx->hist_mode && ctx->gtimeout_ns == lp.margs.timeout_ns &&
@@ -528,6 +573,7 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
   float ms = 0;
   DD_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   const double total = now_ms() - t0;
+  std::vector<uint32_t> redo;
   for (uint32_t i = 0; i < count; ++i) {
     dd_result& r = results[i];
     std::memset(&r, 0, sizeof(r));
@@ -540,12 +586,25 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
     }
     postprocess(reqs[i], shapes[i], raw, r);
     fill_pairs(r, pairs);
-    r.kernel_used = want_mma(ctx, jobs[i], kernels[i]) ? DD_KERNEL_MMA : DD_KERNEL_POPC;
+    r.kernel_used = routes[i] == ROUTE_CARRY ? DD_KERNEL_CARRY : routes[i] == ROUTE_MMA ? DD_KERNEL_MMA : DD_KERNEL_POPC;
     r.mma_epilogue = r.kernel_used == DD_KERNEL_MMA ? mma_epilogue_of(ctx) : 0u;
     r.kernel_ms = ms;  // one launch: the whole batch's device time
     r.total_ms = total;
     r.user_tag = reqs[i].user_tag;
     r.status = DD_OK;
+    // a packed count that left its field makes the total wrong (dd_carry.cu): the
+    // instance is then computed pair by pair
+    if (routes[i] == ROUTE_CARRY) {
+      u128 total_pairs = 0;
+      for (int b = 0; b < kMaxBins; ++b) total_pairs += raw[b];
+      if (total_pairs != pairs) redo.push_back(i);
+    }
+  }
+  for (uint32_t i : redo) {
+    dd_request q = reqs[i];
+    q.kernel = DD_KERNEL_MMA;
+    st = run_requests(ctx, &q, 1, &results[i], false);
+    if (st != DD_OK) return st;
   }
   return DD_OK;
 }

@@ -68,10 +68,14 @@ typedef enum dd_mode {
  * Ext-Hamming all-pairs brute force (Monte Carlo, the Ext-Hamming weight
  * enumerator and anything wider than 60-bit operands use the popc kernel). */
 typedef enum dd_kernel {
-  DD_KERNEL_AUTO = 0,  /* autotuner's choice for the shape; jobs below 2^30 pairs stay on the popc
-                          kernel, whose launch costs less than the tcgen05 kernel's fixed set-up */
+  DD_KERNEL_AUTO = 0,  /* the carry kernels where they win (dd_carry.cu), else the autotuner's choice
+                          for the shape; jobs below 2^30 pairs stay on the popc kernel, whose launch
+                          costs less than the tcgen05 kernel's fixed set-up */
   DD_KERNEL_POPC = 1,  /* XOR + POPC, warp-private shared-memory bins */
-  DD_KERNEL_MMA = 2    /* tcgen05 kind::i8 bit-plane MMA, histogram epilogue from TMEM */
+  DD_KERNEL_MMA = 2,   /* tcgen05 kind::i8 bit-plane MMA, histogram epilogue from TMEM */
+  DD_KERNEL_CARRY = 3  /* AN exhaustive by residue pairs (odd part of A up to 16 bits and shorter
+                          than n, n <= 24, whole instances): about n A^2 steps instead of 4^n / 2
+                          pairs; other jobs follow AUTO's choice of a pair kernel */
 } dd_kernel;
 
 /* Histogram epilogue of the tcgen05 kernel (dd_set_mma_epilogue). */

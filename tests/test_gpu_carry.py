@@ -1,0 +1,53 @@
+"""The residue-pair kernels (dd_carry.cu) against the oracle and the tcgen05
+kernel, bit-exact: every window length (k - bits(A) = 1..8 levels, one kernel up to
+4, staged above), residues hit by one, two and many q, and residue counts at the
+edges of the column strips (241 and 177 useful columns), row segments and staged
+blocks (5409 and 6081 residues a side)."""
+import pytest
+
+import coding_reliability_b200 as dd
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def req(A, k, kernel, **kw):
+    return dd.Request(dd.CODE_AN, dd.MODE_EXHAUSTIVE, A, k, kernel=kernel, **kw)
+
+
+@pytest.mark.parametrize("A,k", [(1, 2), (1, 9), (3, 3), (3, 12), (5, 4), (7, 13), (33, 7), (61, 8), (61, 13), (63, 10),
+                                 (91, 13), (177, 12), (241, 13), (243, 12), (255, 9), (257, 13), (353, 11), (511, 13)])
+def test_carry_vs_oracle(ctx, A, k):
+    q = req(A, k, dd.KERNEL_CARRY)
+    nb, h, Aeff = dd.request_shape(q)
+    res = ctx.histogram(q)
+    assert res.kernel_used == dd.KERNEL_CARRY
+    assert res.raw == oracle.an_exhaustive_raw(Aeff, k, nb)
+    assert res.counts == oracle.an_exhaustive_counts(Aeff, k, nb)
+
+
+@pytest.mark.parametrize("A,k", [(4097, 14), (4819, 15), (4821, 16), (8191, 17), (32769, 17), (65535, 18),  # one kernel
+                                 (33, 14), (867, 20), (129, 16),                       # staged, many q per residue
+                                 (6081, 18), (6083, 18), (4097, 19), (5409, 21), (5411, 20), (12161, 19), (40001, 21)])
+def test_carry_vs_tcgen05(ctx, A, k):
+    res = ctx.histogram(req(A, k, dd.KERNEL_CARRY))
+    mma = ctx.histogram(req(A, k, dd.KERNEL_MMA))
+    assert (res.kernel_used, mma.kernel_used) == (dd.KERNEL_CARRY, dd.KERNEL_MMA)
+    assert res.raw == mma.raw and res.counts == mma.counts and res.minb == mma.minb
+
+
+def test_route(ctx):
+    """AUTO takes the path where its rule says so, for a batch's jobs one by one; an
+    even multiplier (kept by the CPU convention) counts as its odd part; jobs outside
+    the path's range run on a pair kernel although it is asked for."""
+    qs = [req(641, 14, dd.KERNEL_AUTO), req(641, 13, dd.KERNEL_AUTO), req(1283, 14, dd.KERNEL_AUTO),
+          req(976, 15, dd.KERNEL_AUTO, convention=dd.CONV_CPU), req(61, 15, dd.KERNEL_POPC),
+          req(131071, 12, dd.KERNEL_CARRY), req(641, 10, dd.KERNEL_CARRY)]
+    want = [dd.KERNEL_CARRY, dd.KERNEL_POPC, dd.KERNEL_POPC, dd.KERNEL_CARRY, dd.KERNEL_POPC, dd.KERNEL_POPC,
+            dd.KERNEL_POPC]
+    for graph in (False, True, True):
+        out = ctx.batch(qs, use_graph=graph)
+        assert [r.kernel_used for r in out] == want
+        for q, r in zip(qs, out):
+            p = ctx.histogram(req(q.A, q.n, dd.KERNEL_POPC, convention=q.convention))
+            assert r.raw == p.raw and r.counts == p.counts and r.pairs == p.pairs
