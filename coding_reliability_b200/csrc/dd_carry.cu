@@ -40,9 +40,8 @@
 // longer ones run their largest steps first, in a kernel whose rows and columns
 // are 16 residues apart, and stage the 8-bit histograms in memory.
 #include <algorithm>
-#include <type_traits>
 
-#include "dd_carry.h"
+#include "dd_carry.cuh"
 
 namespace dd {
 namespace {
@@ -50,7 +49,6 @@ namespace {
 constexpr int kStageThreads = 512;  // staging kernel: 4 column residues mod 16 x 128 columns 16 apart
 constexpr int kStageCols = kStageThreads / 4;
 constexpr int kUnit = 16;           // residues between the staging kernel's rows and columns
-constexpr int kTabRows = 48;        // distances a table holds: q part <= 16, window part <= 28
 constexpr int kLeafThreads = 256;   // folding kernel reading popcounts
 constexpr int kFoldThreads = 192;   // folding kernel reading staged histograms
 constexpr int kLead = 8;            // rows above a step's own that its first level reads
@@ -67,144 +65,6 @@ struct CarryArgs {
   unsigned long long* acc;          // [0, kMaxBins): residue pairs v < v'; then v = v'
 };
 
-// Counts of bins 8j + 2i (e[j], byte i) and 8j + 2i + 1 (o[j], byte i).
-struct H8 {
-  uint32_t e[3], o[3];
-};
-// Counts of bins 8j + m (low half of pm[j]) and 8j + 4 + m (high half).
-struct H16 {
-  uint32_t p0[4], p1[3], p2[3], p3[3];
-};
-template <int kLevel>
-using Hist = std::conditional_t<(kLevel <= 4), H8, H16>;
-
-__device__ __forceinline__ void zero(H8& h) {
-#pragma unroll
-  for (int j = 0; j < 3; ++j) h.e[j] = h.o[j] = 0;
-}
-__device__ __forceinline__ void zero(H16& h) {
-#pragma unroll
-  for (int j = 0; j < 3; ++j) h.p0[j] = h.p1[j] = h.p2[j] = h.p3[j] = 0;
-  h.p0[3] = 0;
-}
-
-// x + z y
-__device__ __forceinline__ H8 add_z(const H8& x, const H8& y) {
-  H8 r;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    r.e[j] = x.e[j] + (j ? __funnelshift_l(y.o[j - 1], y.o[j], 8) : y.o[0] << 8);
-    r.o[j] = x.o[j] + y.e[j];
-  }
-  return r;
-}
-__device__ __forceinline__ H16 add_z(const H16& x, const H16& y) {
-  H16 r;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    r.p0[j] = x.p0[j] + (j ? __funnelshift_l(y.p3[j - 1], y.p3[j], 16) : y.p3[0] << 16);
-    r.p1[j] = x.p1[j] + y.p0[j];
-    r.p2[j] = x.p2[j] + y.p1[j];
-    r.p3[j] = x.p3[j] + y.p2[j];
-  }
-  r.p0[3] = x.p0[3] + (y.p3[2] >> 16);
-  return r;
-}
-__device__ __forceinline__ H8 add(const H8& x, const H8& y) {
-  H8 r;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    r.e[j] = x.e[j] + y.e[j];
-    r.o[j] = x.o[j] + y.o[j];
-  }
-  return r;
-}
-__device__ __forceinline__ H16 add(const H16& x, const H16& y) {
-  H16 r;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    r.p0[j] = x.p0[j] + y.p0[j];
-    r.p1[j] = x.p1[j] + y.p1[j];
-    r.p2[j] = x.p2[j] + y.p2[j];
-    r.p3[j] = x.p3[j] + y.p3[j];
-  }
-  r.p0[3] = x.p0[3] + y.p0[3];
-  return r;
-}
-__device__ __forceinline__ H16 widen(const H8& h) {
-  H16 r;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    r.p0[j] = h.e[j] & 0x00FF00FFu;
-    r.p1[j] = h.o[j] & 0x00FF00FFu;
-    r.p2[j] = (h.e[j] >> 8) & 0x00FF00FFu;
-    r.p3[j] = (h.o[j] >> 8) & 0x00FF00FFu;
-  }
-  r.p0[3] = 0;
-  return r;
-}
-template <int kLevel>
-__device__ __forceinline__ Hist<kLevel> as_level(const Hist<kLevel - 1>& h) {
-  if constexpr (kLevel == 5) return widen(h);
-  else return h;
-}
-
-// One column's histogram in a shared exchange row: 24 bytes (8-bit counts) or 48
-// (16-bit counts below the last level, whose bins stop at 23), at strides that
-// make the vector accesses conflict-free.
-template <typename H>
-__host__ __device__ constexpr int slot_bytes() { return std::is_same_v<H, H8> ? 24 : 48; }
-__device__ __forceinline__ void put(uint8_t* row, int c, const H8& h) {
-  uint2* p = reinterpret_cast<uint2*>(row + c * 24);
-  p[0] = make_uint2(h.e[0], h.e[1]);
-  p[1] = make_uint2(h.e[2], h.o[0]);
-  p[2] = make_uint2(h.o[1], h.o[2]);
-}
-__device__ __forceinline__ void get(const uint8_t* row, int c, H8& h) {
-  const uint2* p = reinterpret_cast<const uint2*>(row + c * 24);
-  const uint2 x = p[0], y = p[1], w = p[2];
-  h.e[0] = x.x; h.e[1] = x.y; h.e[2] = y.x; h.o[0] = y.y; h.o[1] = w.x; h.o[2] = w.y;
-}
-__device__ __forceinline__ void put(uint8_t* row, int c, const H16& h) {
-  uint4* p = reinterpret_cast<uint4*>(row + c * 48);
-  p[0] = make_uint4(h.p0[0], h.p0[1], h.p0[2], h.p1[0]);
-  p[1] = make_uint4(h.p1[1], h.p1[2], h.p2[0], h.p2[1]);
-  p[2] = make_uint4(h.p2[2], h.p3[0], h.p3[1], h.p3[2]);
-}
-__device__ __forceinline__ void get(const uint8_t* row, int c, H16& h) {
-  const uint4* p = reinterpret_cast<const uint4*>(row + c * 48);
-  const uint4 x = p[0], y = p[1], w = p[2];
-  h.p0[0] = x.x; h.p0[1] = x.y; h.p0[2] = x.z; h.p1[0] = x.w;
-  h.p1[1] = y.x; h.p1[2] = y.y; h.p2[0] = y.z; h.p2[1] = y.w;
-  h.p2[2] = w.x; h.p3[0] = w.y; h.p3[1] = w.z; h.p3[2] = w.w;
-  h.p0[3] = 0;
-}
-
-// The first level from the four high-word distances: z^ha + z^hd + z (z^hb + z^hc).
-// Each distance adds 1 to a nibble (two nibbles per byte: bins 8 apart), a
-// distance of 16 to the count x.
-struct Nibbles {
-  uint32_t e = 0, o = 0, x = 0;
-  __device__ __forceinline__ void count(uint32_t h) {
-    const uint32_t one = 1u << (((h << 2) & 24u) | ((h >> 1) & 4u));
-    if (h & 1u) o += one;
-    else e += one;
-    x += h >> 4;
-  }
-  __device__ __forceinline__ H8 bytes() const {
-    const uint32_t ev = e - x;  // a distance of 16 was counted in bin 0, too
-    return H8{{ev & 0x0F0F0F0Fu, (ev >> 4) & 0x0F0F0F0Fu, x}, {o & 0x0F0F0F0Fu, (o >> 4) & 0x0F0F0F0Fu, 0u}};
-  }
-};
-__device__ __forceinline__ H8 first_level(uint32_t ra, uint32_t rb, uint32_t ca, uint32_t cb) {
-  Nibbles same, cross;
-  same.count(__popc(ra ^ ca));
-  same.count(__popc(rb ^ cb));
-  cross.count(__popc(ra ^ cb));
-  cross.count(__popc(rb ^ ca));
-  return add_z(same.bytes(), cross.bytes());
-}
-
 // One step in a running column: exchange with column c + s, combine, rotate the ring entry y.
 template <int kLevel>
 __device__ __forceinline__ Hist<kLevel> level(const Hist<kLevel - 1>& own, uint8_t* row, int c, int s,
@@ -218,11 +78,6 @@ __device__ __forceinline__ Hist<kLevel> level(const Hist<kLevel - 1>& own, uint8
   y = add_z(n, a);
   return r;
 }
-
-__device__ __forceinline__ uint32_t mul_mod(uint32_t a, uint32_t v, uint32_t A) {
-  return (uint32_t)((uint64_t)a * v % A);
-}
-__device__ __forceinline__ uint32_t sub_mod(uint32_t x, uint32_t d, uint32_t A) { return x >= d ? x - d : x + A - d; }
 
 // Shared bytes of the exchange rows: one per level after the first; with a single
 // one, two that take turns (a row's only barrier then separates them).
@@ -294,57 +149,6 @@ __global__ void __launch_bounds__(kStageThreads) carry_stage_kernel(CarryArgs a)
 }
 
 // ---------------------------------------------------------------- folding kernel
-template <int kOffset>
-__device__ __forceinline__ void red_add(uint32_t addr, uint32_t x) {
-  asm volatile("red.shared.add.u32 [%0+%1], %2;" ::"r"(addr), "n"(kOffset), "r"(x) : "memory");
-}
-
-// Adds f x (the counts of h) to a lane's table column, bin d at at + 128 d.  kWide:
-// products of 64 bits, low 16 bits to the first table, the rest to the one hi bytes on.
-constexpr int kTabBytes = kTabRows * 128;
-template <bool kWide, int kBin>
-__device__ __forceinline__ void add_bin(uint32_t at, uint32_t f, uint32_t x) {
-  if constexpr (kWide) {
-    const unsigned long long p = (unsigned long long)f * x;
-    red_add<kBin * 128>(at, (uint32_t)p & 0xFFFFu);
-    red_add<kBin * 128 + 2 * kTabBytes>(at, (uint32_t)(p >> 16));
-  } else {
-    red_add<kBin * 128>(at, x);
-  }
-}
-template <bool kWide, int kBin>
-__device__ __forceinline__ void add_bytes(uint32_t at, uint32_t f, uint32_t w) {
-  if (w) {
-    add_bin<kWide, kBin>(at, f, w & 0xFFu);
-    add_bin<kWide, kBin + 2>(at, f, (w >> 8) & 0xFFu);
-    add_bin<kWide, kBin + 4>(at, f, (w >> 16) & 0xFFu);
-    add_bin<kWide, kBin + 6>(at, f, w >> 24);
-  }
-}
-template <bool kWide, int kBin>
-__device__ __forceinline__ void add_halves(uint32_t at, uint32_t f, uint32_t w) {
-  if (w) {
-    add_bin<kWide, kBin>(at, f, w & 0xFFFFu);
-    add_bin<kWide, kBin + 4>(at, f, w >> 16);
-  }
-}
-template <bool kWide>
-__device__ __forceinline__ void add_hist(uint32_t at, uint32_t f, const H8& h) {
-  add_bytes<kWide, 0>(at, f, h.e[0]); add_bytes<kWide, 1>(at, f, h.o[0]);
-  add_bytes<kWide, 8>(at, f, h.e[1]); add_bytes<kWide, 9>(at, f, h.o[1]);
-  add_bytes<kWide, 16>(at, f, h.e[2]); add_bytes<kWide, 17>(at, f, h.o[2]);
-}
-template <bool kWide>
-__device__ __forceinline__ void add_hist(uint32_t at, uint32_t f, const H16& h) {
-  add_halves<kWide, 0>(at, f, h.p0[0]); add_halves<kWide, 1>(at, f, h.p1[0]);
-  add_halves<kWide, 2>(at, f, h.p2[0]); add_halves<kWide, 3>(at, f, h.p3[0]);
-  add_halves<kWide, 8>(at, f, h.p0[1]); add_halves<kWide, 9>(at, f, h.p1[1]);
-  add_halves<kWide, 10>(at, f, h.p2[1]); add_halves<kWide, 11>(at, f, h.p3[1]);
-  add_halves<kWide, 16>(at, f, h.p0[2]); add_halves<kWide, 17>(at, f, h.p1[2]);
-  add_halves<kWide, 18>(at, f, h.p2[2]); add_halves<kWide, 19>(at, f, h.p3[2]);
-  add_halves<kWide, 24>(at, f, h.p0[3]);
-}
-
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
@@ -490,11 +294,11 @@ __global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carr
         const uint32_t at = tab_u + (vc == v ? kTabBytes : 0);
         if constexpr (!kMany) {
           const bool c2 = qc + a.A < a.nq;
-          add_hist<false>(at + (__popc(qr ^ qc) << 7), 1, g);
-          if (c2) add_hist<false>(at + (__popc(qr ^ (qc + a.A)) << 7), 1, g);
+          add_hist<kOne>(at + (__popc(qr ^ qc) << 7), 1, g);
+          if (c2) add_hist<kOne>(at + (__popc(qr ^ (qc + a.A)) << 7), 1, g);
           if (qr + a.A < a.nq) {
-            add_hist<false>(at + (__popc((qr + a.A) ^ qc) << 7), 1, g);
-            if (c2) add_hist<false>(at + (__popc((qr + a.A) ^ (qc + a.A)) << 7), 1, g);
+            add_hist<kOne>(at + (__popc((qr + a.A) ^ qc) << 7), 1, g);
+            if (c2) add_hist<kOne>(at + (__popc((qr + a.A) ^ (qc + a.A)) << 7), 1, g);
           }
         } else {
           uint32_t* f = qd + tid;
@@ -504,7 +308,7 @@ __global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carr
             const uint32_t x = f[d * kThreads];
             if (x) {
               f[d * kThreads] = 0;
-              add_hist<true>(at + (d << 7), x, g);
+              add_hist<kWideProduct>(at + (d << 7), x, g);
             }
           }
         }
@@ -563,23 +367,6 @@ cudaError_t run_stage(CarryArgs a, cudaStream_t stream) {
   const dim3 grid(4 * ((w + useful - 1) / useful), kUnit * ((wr + a.seg - 1) / a.seg));
   carry_stage_kernel<kLevels><<<grid, kStageThreads, 0, stream>>>(a);
   return cudaGetLastError();
-}
-
-uint32_t inverse_pow2(uint32_t e, uint32_t A) {  // 2^-e mod A, A odd
-  uint64_t x = 1 % A;
-  const uint64_t half = (A + 1) / 2 % A;
-  for (uint32_t i = 0; i < e; ++i) x = x * half % A;
-  return (uint32_t)x;
-}
-
-uint32_t odd_part(uint64_t A) {
-  while (A && !(A & 1)) A >>= 1;
-  return (uint32_t)A;
-}
-uint32_t bits_of(uint32_t x) {
-  uint32_t n = 0;
-  for (; x; x >>= 1) ++n;
-  return n;
 }
 
 }  // namespace

@@ -1,4 +1,4 @@
-// dd_carry.h — exhaustive AN histograms by residue-pair counting (see dd_carry.cu).
+// dd_carry.h — AN histograms through residues: exhaustive (dd_carry.cu), 1-D grids (dd_carry_rows.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>
@@ -38,5 +38,24 @@ size_t carry_stage_bytes(const CarryPlan& p);
 cudaError_t launch_carry(const CarryPlan& p, unsigned long long* acc, void* stage, cudaStream_t stream);
 // acc of n jobs (2 x kMaxBins each) -> their bins; jobs: the device's table entries.
 cudaError_t launch_carry_finish(const Job* jobs, const unsigned long long* acc, uint32_t n, cudaStream_t stream);
+
+// One 1-D grid job as carry_rows_kernel runs it.
+struct RowsPlan {
+  uint32_t A = 0;           // odd part of the multiplier
+  uint32_t tree = 0;        // rows with a power-of-two stride, in blocks
+  uint32_t stride_log = 0;  // tree: log2 of the stride
+  uint32_t many = 0;        // a residue stands for more columns than are worth visiting one by one
+  uint32_t per = 0;         // columns of a residue per CTA
+  uint32_t slices = 1;      // CTAs that share a residue's columns
+  uint32_t seg = 0;         // rows (blocks) per CTA
+  uint64_t rows = 0;        // rows (list) or blocks of rows (tree)
+};
+// False where the job is no 1-D grid this path runs (whole instances, A's odd part of
+// at most 16 bits, 12 <= n <= 32).
+bool rows_plan(const Job& j, int num_sms, RowsPlan& p);
+// The rule that picks this path under AUTO.
+bool rows_win(const Job& j, const RowsPlan& p);
+// Adds the job's histogram to its (zeroed) bins.
+cudaError_t launch_rows(const Job& j, const RowsPlan& p, cudaStream_t stream);
 
 }  // namespace dd

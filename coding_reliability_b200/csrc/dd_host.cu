@@ -128,7 +128,7 @@ static bool ensure_stage(dd_context* ctx, size_t bytes) {
   return true;
 }
 
-enum Route : uint32_t { ROUTE_POPC = 0, ROUTE_MMA = 1, ROUTE_CARRY = 2 };
+enum Route : uint32_t { ROUTE_POPC = 0, ROUTE_MMA = 1, ROUTE_CARRY = 2, ROUTE_ROWS = 3 };
 
 struct LaunchPlan {
   LaunchArgs pargs;          // popc kernel: table entries [0, npopc)
@@ -139,7 +139,8 @@ struct LaunchPlan {
   int mgrid = 0;
   size_t msmem = 0;
   uint32_t nmma = 0;
-  std::vector<CarryPlan> carry;  // carry path: the table entries after those
+  std::vector<CarryPlan> carry;  // residue pairs, exhaustive: the table entries after those
+  std::vector<RowsPlan> rows;    // residue pairs, 1-D grids: the last table entries
   uint32_t nslots = 0;       // bin slots (one per request, in request order)
 };
 
@@ -175,17 +176,21 @@ static Route route_of(dd_context* ctx, const Job& j, uint32_t kernel) {
     carry_plan(j, ctx->num_sms, p);
     if (ensure_stage(ctx, carry_stage_bytes(p))) return ROUTE_CARRY;
   }
+  RowsPlan rp;
+  if ((kernel == DD_KERNEL_CARRY || kernel == DD_KERNEL_AUTO) && rows_plan(j, ctx->num_sms, rp) &&
+      (kernel == DD_KERNEL_CARRY || rows_win(j, rp)))
+    return ROUTE_ROWS;
   return want_mma(ctx, j, kernel) ? ROUTE_MMA : ROUTE_POPC;
 }
 
-// Orders the job table (popc jobs first, then MMA jobs, then carry jobs), assigns
+// Orders the job table (popc jobs, MMA jobs, then the two kinds of carry jobs), assigns
 // tile ranges and bin slots (slot = request index), and sizes both persistent grids.
 static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vector<Route>& routes,
                        LaunchPlan& lp, bool own_bins = true) {
   std::vector<Job> table;
   table.reserve(jobs.size());
-  uint32_t of_route[3] = {0, 0, 0};
-  for (uint32_t route = 0; route < 3; ++route)
+  uint32_t of_route[4] = {0, 0, 0, 0};
+  for (uint32_t route = 0; route < 4; ++route)
     for (size_t i = 0; i < jobs.size(); ++i) {
       if (routes[i] != route) continue;
       Job j = jobs[i];
@@ -202,6 +207,8 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.carry.resize(of_route[ROUTE_CARRY]);
   for (size_t c = 0; c < lp.carry.size(); ++c) carry_plan(table[lp.npopc + lp.nmma + c], ctx->num_sms, lp.carry[c]);
   const uint32_t pair_jobs = lp.npopc + lp.nmma;
+  lp.rows.resize(of_route[ROUTE_ROWS]);
+  for (size_t c = 0; c < lp.rows.size(); ++c) rows_plan(table[pair_jobs + lp.carry.size() + c], ctx->num_sms, lp.rows[c]);
   for (uint32_t k = 0; k < lp.npopc; ++k) {
     Job& j = table[k];
     j.tile_begin = tp;
@@ -268,7 +275,8 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
 // by events), bins + status D2H.
 static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing) {
   cudaStream_t s = ctx->stream;
-  const uint32_t ncarry = (uint32_t)lp.carry.size(), njobs = lp.npopc + lp.nmma + ncarry;
+  const uint32_t ncarry = (uint32_t)lp.carry.size(), nrows = (uint32_t)lp.rows.size();
+  const uint32_t njobs = lp.npopc + lp.nmma + ncarry + nrows;
   DD_CUDA(cudaMemcpyAsync(ctx->d_jobs, ctx->h_jobs, njobs * sizeof(Job), cudaMemcpyHostToDevice, s));
   unsigned long long* acc = ctx->d_bins + (size_t)ctx->bin_slots * kMaxBins;
   if (ncarry) DD_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncarry * 2 * kMaxBins * sizeof(unsigned long long), s));
@@ -284,6 +292,7 @@ static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing)
   for (uint32_t c = 0; c < ncarry; ++c)
     DD_CUDA(launch_carry(lp.carry[c], acc + (size_t)c * 2 * kMaxBins, ctx->d_stage, s));
   if (ncarry) DD_CUDA(launch_carry_finish(ctx->d_jobs + lp.npopc + lp.nmma, acc, ncarry, s));
+  for (uint32_t c = 0; c < nrows; ++c) DD_CUDA(launch_rows(ctx->h_jobs[njobs - nrows + c], lp.rows[c], s));
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev1, s, evflags));
   DD_CUDA(cudaMemcpyAsync(ctx->h_bins, ctx->d_bins, (size_t)lp.nslots * kMaxBins * sizeof(unsigned long long),
                           cudaMemcpyDeviceToHost, s));
@@ -540,7 +549,7 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
   if (st != DD_OK) return st;
   cudaStream_t s = ctx->stream;
   if (use_graph) {
-    const size_t nj = lp.npopc + lp.nmma + lp.carry.size();
+    const size_t nj = lp.npopc + lp.nmma + lp.carry.size() + lp.rows.size();
     const bool same = ctx->gexec && ctx->gjobs.size() == nj && ctx->ggrid[0] == lp.pgrid &&
                       ctx->ggrid[1] == lp.mgrid && ctx->gsmem[0] == lp.psmem && ctx->gsmem[1] == lp.msmem &&
                       ctx->ghist_mode == ctx->hist_mode && ctx->gtimeout_ns == lp.margs.timeout_ns &&
@@ -586,7 +595,7 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
     }
     postprocess(reqs[i], shapes[i], raw, r);
     fill_pairs(r, pairs);
-    r.kernel_used = routes[i] == ROUTE_CARRY ? DD_KERNEL_CARRY : routes[i] == ROUTE_MMA ? DD_KERNEL_MMA : DD_KERNEL_POPC;
+    r.kernel_used = routes[i] >= ROUTE_CARRY ? DD_KERNEL_CARRY : routes[i] == ROUTE_MMA ? DD_KERNEL_MMA : DD_KERNEL_POPC;
     r.mma_epilogue = r.kernel_used == DD_KERNEL_MMA ? mma_epilogue_of(ctx) : 0u;
     r.kernel_ms = ms;  // one launch: the whole batch's device time
     r.total_ms = total;
@@ -594,7 +603,7 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
     r.status = DD_OK;
     // a packed count that left its field makes the total wrong (dd_carry.cu): the
     // instance is then computed pair by pair
-    if (routes[i] == ROUTE_CARRY) {
+    if (routes[i] >= ROUTE_CARRY) {
       u128 total_pairs = 0;
       for (int b = 0; b < kMaxBins; ++b) total_pairs += raw[b];
       if (total_pairs != pairs) redo.push_back(i);

@@ -73,9 +73,10 @@ typedef enum dd_kernel {
                           costs less than the tcgen05 kernel's fixed set-up */
   DD_KERNEL_POPC = 1,  /* XOR + POPC, warp-private shared-memory bins */
   DD_KERNEL_MMA = 2,   /* tcgen05 kind::i8 bit-plane MMA, histogram epilogue from TMEM */
-  DD_KERNEL_CARRY = 3  /* AN exhaustive by residue pairs (odd part of A up to 16 bits and shorter
-                          than n, n <= 24, whole instances): about n A^2 steps instead of 4^n / 2
-                          pairs; other jobs follow AUTO's choice of a pair kernel */
+  DD_KERNEL_CARRY = 3  /* residues of A (odd part of at most 16 bits) instead of codewords, whole
+                          instances: AN exhaustive (bits of A < n <= 24) in about n A^2 steps for
+                          4^n / 2 pairs, 1-D grids (12 <= n <= 32) in about 8 A steps a row for
+                          2^n; other jobs follow AUTO's choice of a pair kernel */
 } dd_kernel;
 
 /* Histogram epilogue of the tcgen05 kernel (dd_set_mma_epilogue). */

@@ -2,7 +2,9 @@
 kernel, bit-exact: every window length (k - bits(A) = 1..8 levels, one kernel up to
 4, staged above), residues hit by one, two and many q, and residue counts at the
 edges of the column strips (241 and 177 useful columns), row segments and staged
-blocks (5409 and 6081 residues a side)."""
+blocks (5409 and 6081 residues a side).  The 1-D grid form (dd_carry_rows.cu): rows
+in blocks of a power-of-two stride and listed rows, strips of 449 and 769 useful
+columns, few and many columns a residue, several slices of them."""
 import pytest
 
 import coding_reliability_b200 as dd
@@ -36,18 +38,43 @@ def test_carry_vs_tcgen05(ctx, A, k):
     assert res.raw == mma.raw and res.counts == mma.counts and res.minb == mma.minb
 
 
+def grid(A, k, m, kernel, **kw):
+    return dd.Request(dd.CODE_AN, dd.MODE_GRID_1D, A, k, m=m, kernel=kernel, **kw)
+
+
+@pytest.mark.parametrize("A,k,m", [(1, 12, 64), (3, 12, 13), (5, 13, 4096), (61, 12, 4096), (449, 12, 65), (451, 13, 64),
+                                   (641, 14, 1000), (769, 13, 3), (771, 12, 17), (1021, 15, 333), (976, 14, 128)])
+def test_grid_vs_oracle(ctx, A, k, m):
+    q = grid(A, k, m, dd.KERNEL_CARRY)
+    nb, h, Aeff = dd.request_shape(q)
+    res = ctx.histogram(q)
+    assert res.kernel_used == dd.KERNEL_CARRY
+    assert res.raw == oracle.an_grid1d_raw(Aeff, k, h, m, nb)[0]
+
+
+@pytest.mark.parametrize("A,k,m", [(65535, 16, 256), (65535, 20, 100), (32769, 24, 128), (8191, 22, 1 << 12),
+                                   (1283, 24, 99), (61, 24, 1 << 10), (33, 27, 64), (35, 25, 21), (65535, 27, 64)])
+def test_grid_vs_tcgen05(ctx, A, k, m):
+    res = ctx.histogram(grid(A, k, m, dd.KERNEL_CARRY))
+    mma = ctx.histogram(grid(A, k, m, dd.KERNEL_MMA))
+    assert (res.kernel_used, mma.kernel_used) == (dd.KERNEL_CARRY, dd.KERNEL_MMA)
+    assert res.raw == mma.raw and res.counts == mma.counts and res.minb == mma.minb
+
+
 def test_route(ctx):
     """AUTO takes the path where its rule says so, for a batch's jobs one by one; an
     even multiplier (kept by the CPU convention) counts as its odd part; jobs outside
     the path's range run on a pair kernel although it is asked for."""
     qs = [req(641, 14, dd.KERNEL_AUTO), req(641, 13, dd.KERNEL_AUTO), req(1283, 14, dd.KERNEL_AUTO),
           req(976, 15, dd.KERNEL_AUTO, convention=dd.CONV_CPU), req(61, 15, dd.KERNEL_POPC),
-          req(131071, 12, dd.KERNEL_CARRY), req(641, 10, dd.KERNEL_CARRY)]
+          req(131071, 12, dd.KERNEL_CARRY), req(641, 10, dd.KERNEL_CARRY),
+          grid(641, 18, 1024, dd.KERNEL_AUTO), grid(641, 18, 1023, dd.KERNEL_AUTO), grid(641, 18, 1025, dd.KERNEL_AUTO),
+          grid(641, 11, 64, dd.KERNEL_CARRY)]
     want = [dd.KERNEL_CARRY, dd.KERNEL_POPC, dd.KERNEL_POPC, dd.KERNEL_CARRY, dd.KERNEL_POPC, dd.KERNEL_POPC,
-            dd.KERNEL_POPC]
+            dd.KERNEL_POPC, dd.KERNEL_CARRY, dd.KERNEL_POPC, dd.KERNEL_CARRY, dd.KERNEL_POPC]
     for graph in (False, True, True):
         out = ctx.batch(qs, use_graph=graph)
         assert [r.kernel_used for r in out] == want
         for q, r in zip(qs, out):
-            p = ctx.histogram(req(q.A, q.n, dd.KERNEL_POPC, convention=q.convention))
+            p = ctx.histogram(dd.Request(q.code, q.mode, q.A, q.n, m=q.m, convention=q.convention, kernel=dd.KERNEL_POPC))
             assert r.raw == p.raw and r.counts == p.counts and r.pairs == p.pairs
