@@ -33,6 +33,50 @@ __host__ __device__ __forceinline__ Philox4 philox4x32_10(uint32_t c0, uint32_t 
   return Philox4{c0, c1, c2, c3};
 }
 
+#if defined(__CUDACC__)
+// The same generator for a run of blocks that differ in the counter's low word b
+// only: rounds one and two share what depends on the other words (M1 * i and the
+// M0 product that follows from it), and M0 * b moves by additions from block to
+// block, so a block takes 34 of the 40 multiplies that bound the samplers.
+struct PhiloxRun {
+  uint32_t k0, k1, i1;
+  uint32_t lo1;       // M1 * i0, low word: the second round's c1
+  uint32_t lo0, hi0;  // second round's M0 * c0, c0 = hi(M1 * i0) ^ (counter word 1) ^ k0
+  __device__ __forceinline__ PhiloxRun(uint32_t b_high, uint32_t i0_, uint32_t i1_, uint32_t k0_, uint32_t k1_)
+      : k0(k0_), k1(k1_), i1(i1_) {
+    lo1 = 0xCD9E8D57u * i0_;
+    const uint32_t c0 = __umulhi(0xCD9E8D57u, i0_) ^ b_high ^ k0_;
+    lo0 = 0xD2511F53u * c0;
+    hi0 = __umulhi(0xD2511F53u, c0);
+  }
+  static __device__ __forceinline__ uint64_t first(uint32_t b) { return (uint64_t)0xD2511F53u * b; }
+  static __device__ __forceinline__ uint64_t next(uint64_t p, uint32_t blocks) {
+    return p + (uint64_t)0xD2511F53u * blocks;
+  }
+  // Block of M0 * b = p.
+  __device__ __forceinline__ Philox4 block(uint64_t p) const {
+    // after round one: c0 as above, c1 = lo1, c2, c3
+    uint32_t c2 = (uint32_t)(p >> 32) ^ i1 ^ k1;
+    uint32_t c3 = (uint32_t)p;
+    uint32_t a0 = k0 + 0x9E3779B9u, a1 = k1 + 0xBB67AE85u;
+    uint32_t c0 = __umulhi(0xCD9E8D57u, c2) ^ lo1 ^ a0;
+    uint32_t c1 = 0xCD9E8D57u * c2;
+    c2 = hi0 ^ c3 ^ a1;
+    c3 = lo0;
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+      a0 += 0x9E3779B9u;
+      a1 += 0xBB67AE85u;
+      const uint32_t l0 = 0xD2511F53u * c0, h0 = __umulhi(0xD2511F53u, c0);
+      const uint32_t l1 = 0xCD9E8D57u * c2, h1 = __umulhi(0xCD9E8D57u, c2);
+      const uint32_t n0 = h1 ^ c1 ^ a0, n2 = h0 ^ c3 ^ a1;
+      c0 = n0; c1 = l1; c2 = n2; c3 = l0;
+    }
+    return Philox4{c0, c1, c2, c3};
+  }
+};
+#endif
+
 // ---------------------------------------------------------------------------
 // Ext-Hamming codewords.  Two definitions exist in the reference:
 //  - hamming_cw_gpu: parity bits WITHOUT the overall parity bit, placed in the

@@ -132,7 +132,7 @@ enum Route : uint32_t { ROUTE_POPC = 0, ROUTE_MMA = 1, ROUTE_CARRY = 2, ROUTE_RO
 
 struct LaunchPlan {
   LaunchArgs pargs;          // popc kernel: table entries [0, npopc)
-  int pgrid = 0;
+  int pgrid = 0, pkind = kMixedKinds;
   size_t psmem = 0;
   uint32_t npopc = 0;
   MmaArgs margs;             // MMA kernel: table entries [npopc, npopc + nmma)
@@ -214,6 +214,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
     j.tile_begin = tp;
     tp += j.tiles;
     maxb = std::max(maxb, j.nbins);
+    lp.pkind = k == 0 || lp.pkind == (int)j.kind ? (int)j.kind : kMixedKinds;
     col_table |= (j.kind == JOB_PAIRS && j.col_kind == COL_HAMMING_EXT && !j.wide);
   }
   for (uint32_t k = lp.npopc; k < pair_jobs; ++k) {
@@ -230,13 +231,14 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.pargs.counter = ctx->d_ctl;
   lp.pargs.status = status;
   lp.pargs.use_col_table = col_table ? 1u : 0u;
-  lp.pargs.pad = 0;
+  lp.pargs.split_log = 0;
   if (lp.npopc && tp) {
     lp.psmem = hist_smem_bytes(maxb, col_table);
     int occ = 0;
-    DD_CUDA(hist_occupancy(ctx->hist_mode, lp.psmem, &occ));
+    DD_CUDA(hist_occupancy(ctx->hist_mode, lp.pkind, lp.psmem, &occ));
     if (occ < 1) { set_error("kernel does not fit on an SM"); return DD_ERR_UNSUPPORTED; }
-    const uint64_t want = (tp + kWarpsPerCta - 1) / kWarpsPerCta;
+    lp.pargs.split_log = hist_split_log(tp, (uint64_t)ctx->num_sms * occ * kWarpsPerCta);
+    const uint64_t want = ((tp << lp.pargs.split_log) + kWarpsPerCta - 1) / kWarpsPerCta;
     lp.pgrid = (int)std::min<uint64_t>((uint64_t)ctx->num_sms * occ, std::max<uint64_t>(want, 1));
   }
   lp.margs.jobs = ctx->d_jobs + lp.npopc;
@@ -287,7 +289,7 @@ static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing)
   // every replay); outside a capture the flag is not accepted.
   const unsigned evflags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev0, s, evflags));
-  if (lp.pgrid) DD_CUDA(launch_hist(ctx->hist_mode, lp.pargs, lp.pgrid, lp.psmem, s));
+  if (lp.pgrid) DD_CUDA(launch_hist(ctx->hist_mode, lp.pkind, lp.pargs, lp.pgrid, lp.psmem, s));
   if (lp.mgrid) DD_CUDA(launch_mma(lp.margs, lp.mgrid, lp.msmem, s));
   for (uint32_t c = 0; c < ncarry; ++c)
     DD_CUDA(launch_carry(lp.carry[c], acc + (size_t)c * 2 * kMaxBins, ctx->d_stage, s));
@@ -333,7 +335,7 @@ int launch_round(dd_context* ctx, std::vector<Job>& jobs, const std::vector<uint
   DD_CUDA(cudaMemcpyAsync(ctx->d_jobs, ctx->h_jobs, njobs * sizeof(Job), cudaMemcpyHostToDevice, s));
   DD_CUDA(cudaMemsetAsync(ctx->d_ctl, 0, kCtlWords * sizeof(unsigned long long), s));
   DD_CUDA(cudaEventRecord(ctx->ev0, s));
-  if (lp.pgrid) DD_CUDA(launch_hist(ctx->hist_mode, lp.pargs, lp.pgrid, lp.psmem, s));
+  if (lp.pgrid) DD_CUDA(launch_hist(ctx->hist_mode, lp.pkind, lp.pargs, lp.pgrid, lp.psmem, s));
   if (lp.mgrid) DD_CUDA(launch_mma(lp.margs, lp.mgrid, lp.msmem, s));
   DD_CUDA(cudaEventRecord(ctx->ev1, s));
   DD_CUDA(cudaMemcpyAsync(ctx->h_ctl, ctx->d_ctl, kCtlWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));

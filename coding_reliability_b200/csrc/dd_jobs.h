@@ -39,6 +39,7 @@ DD_HOST_DEVICE inline uint64_t mc_rows_per_lane(uint64_t spl) {
 DD_HOST_DEVICE inline uint64_t mc_chunks(uint64_t spl) {
   return spl >= (uint64_t)kMcSamplesPerTile ? (spl + kMcSamplesPerTile - 1) / kMcSamplesPerTile : 1;
 }
+constexpr uint32_t kMaxSplitLog = 5;           // a tile is claimed in at most 32 parts
 constexpr uint32_t kFlushEvery = 1u << 16;     // warp tiles between flushes (uint32 counter bound)
 
 enum JobKind : uint32_t {
@@ -99,7 +100,7 @@ struct LaunchArgs {
   unsigned long long* counter;  // global work counter (zeroed before launch)
   unsigned* status;          // KSTATUS_* bits
   uint32_t use_col_table;    // reserve a per-warp column table
-  uint32_t pad;
+  uint32_t split_log;        // a claim is one of a tile's 2^split_log parts (hist_split_log)
 };
 
 }  // namespace dd

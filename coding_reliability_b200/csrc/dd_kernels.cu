@@ -1,7 +1,8 @@
 // dd_kernels.cu — the popc-path histogram kernels (sm_100a).
 //
 // One persistent kernel serves every job kind.  Each warp is an independent
-// worker: it claims a tile from a global counter, accumulates distances into
+// worker: it claims a tile (or, in a launch of few tiles, a part of one:
+// hist_split_log) from a global counter, accumulates distances into
 // its own shared-memory bins (one uint32 column per lane, so increments never
 // collide), and flushes those bins warp-aggregated into the job's uint64
 // global bins when it moves to another job, every kFlushEvery tiles, and at
@@ -119,10 +120,23 @@ __device__ __forceinline__ uint64_t col_value(const Job& J, uint64_t j) {
 // Fast path: 32 lanes x kRowsPerLane valid rows, columns [c, ce) an arithmetic
 // progression v = A*j with warp-uniform v; `off[q]` is the shared address of
 // lane's bin 0 for row q, already shifted by the high-word distance.
-template <int kMode>
+// kMasked (diagonal columns): a pair counts where its column, `first` for the first
+// one (both relative to the tile's first row), lies above its row.
+template <int kMode, bool kMasked = false>
 __device__ __forceinline__ void run_progression(const uint32_t (&w)[kRowsPerLane], const uint32_t (&off)[kRowsPerLane],
-                                                uint32_t v, uint32_t a, uint32_t count) {
+                                                uint32_t v, uint32_t a, uint32_t count, uint32_t first = 0) {
   uint32_t j = 0;
+  if constexpr (kMasked) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll 4
+    for (; j < count; ++j) {
+#pragma unroll
+      for (int q = 0; q < kRowsPerLane; ++q)
+        if (first + j > q * 32 + lane) bump<kMode>(off[q] + (__popc(w[q] ^ v) << 7));
+      v += a;
+    }
+    return;
+  }
   for (; j + 8 <= count; j += 8) {
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -173,9 +187,12 @@ __device__ __forceinline__ void run_generic(const Job& J, const uint64_t (&w)[kR
   }
 }
 
+// Part `part` of the tile's 2^split_log column slices.
 template <int kMode>
-__device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t* table, int lane, unsigned* status) {
+__device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t part, uint32_t split_log, uint32_t* wbins,
+                           uint32_t* table, int lane, unsigned* status) {
   uint64_t r0, c0, c1;
+  const uint32_t width = kTileCols >> split_log;
   bool diag = false;
   if (J.shape == SHAPE_TRIANGLE) {
     const uint64_t s = lt / kStrips;
@@ -184,14 +201,15 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
     tri_decode(s, J.col_tiles, sr, sc);
     r0 = sr * kSuper + (uint64_t)strip * kWarpRows;
     c0 = sc * kSuper;
-    c1 = c0 + kSuper < J.cols ? c0 + kSuper : J.cols;
     diag = (sr == sc);
   } else {
     static_assert(kWarpRows == 128 && kTileCols == 1024, "rect_decode's tile shape");
     rect_decode(lt, (J.rows + kWarpRows - 1) / kWarpRows, r0, c0);
-    c1 = c0 + kTileCols < J.cols ? c0 + kTileCols : J.cols;
   }
-  if (r0 >= J.rows) return;
+  static_assert(kSuper == kTileCols, "a triangle tile's columns");
+  c0 += (uint64_t)part * width;
+  c1 = c0 + width < J.cols ? c0 + width : J.cols;
+  if (r0 >= J.rows || c0 >= c1 || (diag && c1 <= r0 + 1)) return;
 
   uint64_t w[kRowsPerLane], ri[kRowsPerLane];
   bool rv[kRowsPerLane];
@@ -207,16 +225,13 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
   const uint32_t lane_base = (uint32_t)__cvta_generic_to_shared(wbins) + (uint32_t)lane * 4u;
 
   // Diagonal tile: columns <= r0 pair with no row; (r0, r0+kWarpRows) need the
-  // j > i mask; the rest is a full rectangle.
+  // j > i mask; from cf on the tile is a full rectangle.
   uint64_t cf = c0;
   if (diag) {
-    const uint64_t mlo = r0 + 1 > c0 ? r0 + 1 : c0;
-    const uint64_t mhi = r0 + kWarpRows < c1 ? r0 + kWarpRows : c1;
-    if (mlo < mhi) run_generic<kMode>(J, w, ri, rv, lane_base, mlo, mhi, true, status);
-    cf = mhi > mlo ? mhi : mlo;
+    if (c0 < r0 + 1) c0 = r0 + 1;
+    cf = r0 + kWarpRows < c1 ? r0 + kWarpRows : c1;
     if (cf < c0) cf = c0;
   }
-  if (cf >= c1) return;
 
   // The unchecked fast paths need every distance of the tile below nbins: the
   // widest row or column codeword of the tile must have at most nbins-1 bits.
@@ -229,6 +244,7 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
 
   if (!all_valid || !fits || J.col_kind == COL_LATTICE || (J.wide && J.col_kind != COL_PROGRESSION) ||
       (J.col_kind == COL_PROGRESSION && J.wide && (J.A >> 32))) {
+    run_generic<kMode>(J, w, ri, rv, lane_base, c0, cf, true, status);
     run_generic<kMode>(J, w, ri, rv, lane_base, cf, c1, false, status);
     return;
   }
@@ -238,6 +254,7 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
   for (int q = 0; q < kRowsPerLane; ++q) wl[q] = (uint32_t)w[q];
 
   if (J.col_kind == COL_HAMMING_EXT) {
+    run_generic<kMode>(J, w, ri, rv, lane_base, c0, cf, true, status);
     const uint32_t cnt = (uint32_t)(c1 - cf);
     for (uint32_t jj = lane; jj < cnt; jj += 32) table[jj] = (uint32_t)hamming_cw_ext(cf + jj, J.n);
     __syncwarp();
@@ -252,6 +269,7 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
   if (!J.wide) {
 #pragma unroll
     for (int q = 0; q < kRowsPerLane; ++q) off[q] = lane_base;
+    run_progression<kMode, true>(wl, off, (uint32_t)(J.A * c0), a, (uint32_t)(cf - c0), (uint32_t)(c0 - r0));
     run_progression<kMode>(wl, off, (uint32_t)(J.A * cf), a, (uint32_t)(c1 - cf));
     return;
   }
@@ -261,15 +279,17 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
   uint32_t wh[kRowsPerLane];
 #pragma unroll
   for (int q = 0; q < kRowsPerLane; ++q) wh[q] = (uint32_t)(w[q] >> 32);
-  uint64_t j = cf;
+  uint64_t j = c0;
   uint64_t v = J.A * j;
   while (j < c1) {
     const uint32_t vl = (uint32_t)v, vh = (uint32_t)(v >> 32);
     const uint64_t to_wrap = ((1ull << 32) - vl + a - 1) / a;
-    const uint64_t je = j + to_wrap < c1 ? j + to_wrap : c1;
+    uint64_t je = j + to_wrap < c1 ? j + to_wrap : c1;
+    if (j < cf && je > cf) je = cf;
 #pragma unroll
     for (int q = 0; q < kRowsPerLane; ++q) off[q] = lane_base + (__popc(wh[q] ^ vh) << 7);
-    run_progression<kMode>(wl, off, vl, a, (uint32_t)(je - j));
+    if (j < cf) run_progression<kMode, true>(wl, off, vl, a, (uint32_t)(je - j), (uint32_t)(j - r0));
+    else run_progression<kMode>(wl, off, vl, a, (uint32_t)(je - j));
     v += J.A * (je - j);
     j = je;
   }
@@ -286,33 +306,38 @@ __device__ void pairs_tile(const Job& J, uint64_t lt, uint32_t* wbins, uint32_t*
 constexpr int kMcBlocksPerStep = 4;
 
 // Many samples per codeword: one codeword per lane, up to kMcSamplesPerTile of
-// its samples, drawn kMcBlocksPerStep Philox blocks at a time.
+// its samples, drawn kMcBlocksPerStep Philox blocks at a time.  Both codewords of a
+// sample have at most n + h = nbins - 1 bits (derive_shape), so the distances index
+// the bins unchecked.  Bound by the multiplies of Philox; 2^24 codewords x 257 samples
+// (A = 62307): 4.35 ms, 5.4 ms with the whole generator per block and checked bins; see
+// PhiloxRun for what the blocks of a codeword share.
 template <int kMode>
-__device__ __forceinline__ void mc_many(const Job& J, uint64_t i, uint64_t t, uint64_t t1, uint32_t lane_base,
-                                        unsigned* status) {
+__device__ __forceinline__ void mc_many(const Job& J, uint64_t i, uint64_t t, uint64_t t1, uint32_t lane_base) {
   const uint64_t w = J.A * i;
-  const uint32_t k0 = (uint32_t)J.seed, k1 = (uint32_t)(J.seed >> 32);
-  const uint32_t i0 = (uint32_t)i, i1 = (uint32_t)(i >> 32);
-  if (J.n <= 32) {
+  const uint32_t a = (uint32_t)J.A;  // A < 2^32
+  const uint32_t n = J.n, per_log = n <= 32 ? 2u : 1u;
+  auto one = [&](uint64_t t_) { bump<kMode>(lane_base + (popc64(w ^ (J.A * mc_index(J.seed, i, t_, n))) << 7)); };
+  // up to the next block boundary (a continued run may start inside a block), and
+  // all samples of a run whose block numbers cross 2^32
+  const bool crosses = ((t1 >> per_log) >> 32) != ((t >> per_log) >> 32);
+  for (; t < t1 && (crosses || (t & ((1u << per_log) - 1))); ++t) one(t);
+  const PhiloxRun run((uint32_t)((t >> per_log) >> 32), (uint32_t)i, (uint32_t)(i >> 32), (uint32_t)J.seed,
+                      (uint32_t)(J.seed >> 32));
+  uint64_t p = PhiloxRun::first((uint32_t)(t >> per_log));
+  if (n <= 32) {
     // four 32-bit samples per block (counter (t >> 2, i)); index = top n bits
-    const unsigned sh = 32 - J.n;
+    const unsigned sh = 32 - n;
     const uint32_t wl = (uint32_t)w;
-    const uint32_t a = (uint32_t)J.A;  // A < 2^32
     const bool wide = J.wide != 0;
-    // up to the next block boundary (a continued run may start inside a block)
-    for (; t < t1 && (t & 3); ++t) {
-      const uint64_t v = J.A * mc_index(J.seed, i, t, J.n);
-      bump_checked<kMode>(lane_base, popc64(w ^ v), J.nbins, status);
-    }
     constexpr int kS = 4 * kMcBlocksPerStep;
     for (; t + kS <= t1; t += kS) {
       uint32_t r[kS], d[kS];
 #pragma unroll
       for (int b = 0; b < kMcBlocksPerStep; ++b) {
-        const uint64_t blk = (t >> 2) + b;
-        const Philox4 o = philox4x32_10((uint32_t)blk, (uint32_t)(blk >> 32), i0, i1, k0, k1);
+        const Philox4 o = run.block(PhiloxRun::next(p, b));
         r[4 * b] = o.x; r[4 * b + 1] = o.y; r[4 * b + 2] = o.z; r[4 * b + 3] = o.w;
       }
+      p = PhiloxRun::next(p, kMcBlocksPerStep);
       if (wide) {
 #pragma unroll
         for (int u = 0; u < kS; ++u) d[u] = popc64(w ^ ((uint64_t)a * (r[u] >> sh)));
@@ -321,51 +346,43 @@ __device__ __forceinline__ void mc_many(const Job& J, uint64_t i, uint64_t t, ui
         for (int u = 0; u < kS; ++u) d[u] = __popc(wl ^ (a * (r[u] >> sh)));
       }
 #pragma unroll
-      for (int u = 0; u < kS; ++u) bump_checked<kMode>(lane_base, d[u], J.nbins, status);
+      for (int u = 0; u < kS; ++u) bump<kMode>(lane_base + (d[u] << 7));
     }
   } else {
     // two 64-bit samples per block (counter (t >> 1, i)); index = top n bits
-    const unsigned sh = 64 - J.n;
-    if (t < t1 && (t & 1)) {
-      const uint64_t v = J.A * mc_index(J.seed, i, t, J.n);
-      bump_checked<kMode>(lane_base, popc64(w ^ v), J.nbins, status);
-      ++t;
-    }
+    const unsigned sh = 64 - n;
     constexpr int kS = 2 * kMcBlocksPerStep;
     for (; t + kS <= t1; t += kS) {
       uint64_t r[kS];
       uint32_t d[kS];
 #pragma unroll
       for (int b = 0; b < kMcBlocksPerStep; ++b) {
-        const uint64_t blk = (t >> 1) + b;
-        const Philox4 o = philox4x32_10((uint32_t)blk, (uint32_t)(blk >> 32), i0, i1, k0, k1);
+        const Philox4 o = run.block(PhiloxRun::next(p, b));
         r[2 * b] = ((uint64_t)o.x << 32) | o.y;
         r[2 * b + 1] = ((uint64_t)o.z << 32) | o.w;
       }
+      p = PhiloxRun::next(p, kMcBlocksPerStep);
 #pragma unroll
-      for (int u = 0; u < kS; ++u) d[u] = popc64(w ^ ((uint64_t)(uint32_t)J.A * (r[u] >> sh)));
+      for (int u = 0; u < kS; ++u) d[u] = popc64(w ^ ((uint64_t)a * (r[u] >> sh)));
 #pragma unroll
-      for (int u = 0; u < kS; ++u) bump_checked<kMode>(lane_base, d[u], J.nbins, status);
+      for (int u = 0; u < kS; ++u) bump<kMode>(lane_base + (d[u] << 7));
     }
   }
-  for (; t < t1; ++t) {
-    const uint64_t v = J.A * mc_index(J.seed, i, t, J.n);
-    bump_checked<kMode>(lane_base, popc64(w ^ v), J.nbins, status);
-  }
+  for (; t < t1; ++t) one(t);
 }
 
 // Few samples per codeword (fewer than kMcSamplesPerTile): each lane takes
 // several codewords with all of their samples, one Philox block at a time.
 template <int kMode>
-__device__ __noinline__ void mc_few(uint64_t A, uint64_t seed, uint32_t n, uint32_t nbins, uint64_t i, uint64_t t,
-                                    uint64_t t1, uint32_t lane_base, unsigned* status) {
+__device__ __noinline__ void mc_few(uint64_t A, uint64_t seed, uint32_t n, uint64_t i, uint64_t t, uint64_t t1,
+                                    uint32_t lane_base) {
   const uint64_t w = A * i;
   const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
   const uint32_t i0 = (uint32_t)i, i1 = (uint32_t)(i >> 32);
   const uint64_t a = (uint32_t)A;  // A < 2^32
   const unsigned per_block = n <= 32 ? 4u : 2u;
   for (; t < t1 && (t & (per_block - 1)); ++t)
-    bump_checked<kMode>(lane_base, popc64(w ^ (A * mc_index(seed, i, t, n))), nbins, status);
+    bump<kMode>(lane_base + (popc64(w ^ (A * mc_index(seed, i, t, n))) << 7));
   for (; t + per_block <= t1; t += per_block) {
     const uint64_t blk = t / per_block;
     const Philox4 o = philox4x32_10((uint32_t)blk, (uint32_t)(blk >> 32), i0, i1, k0, k1);
@@ -373,50 +390,112 @@ __device__ __noinline__ void mc_few(uint64_t A, uint64_t seed, uint32_t n, uint3
       const unsigned sh = 32 - n;
       const uint32_t d0 = popc64(w ^ (a * (o.x >> sh))), d1 = popc64(w ^ (a * (o.y >> sh)));
       const uint32_t d2 = popc64(w ^ (a * (o.z >> sh))), d3 = popc64(w ^ (a * (o.w >> sh)));
-      bump_checked<kMode>(lane_base, d0, nbins, status);
-      bump_checked<kMode>(lane_base, d1, nbins, status);
-      bump_checked<kMode>(lane_base, d2, nbins, status);
-      bump_checked<kMode>(lane_base, d3, nbins, status);
+      bump<kMode>(lane_base + (d0 << 7));
+      bump<kMode>(lane_base + (d1 << 7));
+      bump<kMode>(lane_base + (d2 << 7));
+      bump<kMode>(lane_base + (d3 << 7));
     } else {
       const unsigned sh = 64 - n;
       const uint32_t d0 = popc64(w ^ (a * ((((uint64_t)o.x << 32) | o.y) >> sh)));
       const uint32_t d1 = popc64(w ^ (a * ((((uint64_t)o.z << 32) | o.w) >> sh)));
-      bump_checked<kMode>(lane_base, d0, nbins, status);
-      bump_checked<kMode>(lane_base, d1, nbins, status);
+      bump<kMode>(lane_base + (d0 << 7));
+      bump<kMode>(lane_base + (d1 << 7));
     }
   }
-  for (; t < t1; ++t) bump_checked<kMode>(lane_base, popc64(w ^ (A * mc_index(seed, i, t, n))), nbins, status);
+  for (; t < t1; ++t) bump<kMode>(lane_base + (popc64(w ^ (A * mc_index(seed, i, t, n))) << 7));
 }
 
 template <int kMode>
-__device__ void mc_tile(const Job& J, uint64_t lt, uint32_t* wbins, int lane, unsigned* status) {
+__device__ void mc_tile(const Job& J, uint64_t lt, uint32_t part, uint32_t split_log, uint32_t* wbins, int lane) {
   const uint64_t spl = J.iters - J.sample_begin;
   const uint64_t rpl = mc_rows_per_lane(spl), chunks = mc_chunks(spl);
   const uint64_t rt = lt / chunks, ch = lt % chunks;
-  const uint64_t t0 = J.sample_begin + ch * kMcSamplesPerTile;
-  const uint64_t t1 = t0 + kMcSamplesPerTile < J.iters ? t0 + kMcSamplesPerTile : J.iters;
+  uint64_t t0 = J.sample_begin + ch * kMcSamplesPerTile;
+  uint64_t t1 = t0 + kMcSamplesPerTile < J.iters ? t0 + kMcSamplesPerTile : J.iters;
   const uint32_t lane_base = (uint32_t)__cvta_generic_to_shared(wbins) + (uint32_t)lane * 4u;
   if (rpl == 1) {
+    // a part takes its share of the tile's samples
+    const uint32_t width = kMcSamplesPerTile >> split_log;
+    t0 += (uint64_t)part * width;
+    if (t0 + width < t1) t1 = t0 + width;
     const uint64_t i = rt * 32 + lane;
-    if (i < J.rows) mc_many<kMode>(J, i, t0, t1, lane_base, status);
+    if (i < J.rows && t0 < t1) mc_many<kMode>(J, i, t0, t1, lane_base);
     return;
   }
-  for (uint64_t r = 0; r < rpl; ++r) {
+  // ... or of its codewords
+  for (uint64_t r = (rpl * part) >> split_log, re = (rpl * (part + 1)) >> split_log; r < re; ++r) {
     const uint64_t i = (rt * rpl + r) * 32 + lane;
     if (i >= J.rows) return;
-    mc_few<kMode>(J.A, J.seed, J.n, J.nbins, i, t0, t1, lane_base, status);
+    mc_few<kMode>(J.A, J.seed, J.n, i, t0, t1, lane_base);
   }
 }
 
 // ---------------------------------------------------------------------------
 // Ext-Hamming weight tiles: 32 lanes x 256 generated messages.
 // ---------------------------------------------------------------------------
+// Weight of hamming_cw_gpu(v, N, n4): the message's bits and its parity bits.  The
+// masks cover the low 32 message bits, so a parity is one 32-bit popcount.
+__device__ __forceinline__ uint32_t hamming_weight_gpu(uint64_t v, unsigned N, bool n4_branch) {
+  const uint32_t x = (uint32_t)v;
+  uint32_t w = popc64(v) + (__popc(x & 0x56AAAD5Bu) & 1) + (__popc(x & 0x9B33366Du) & 1) + (__popc(x & 0xE3C3C78Eu) & 1);
+  if (n4_branch && N < 8) return w;
+  w += __popc(x & 0x03FC07F0u) & 1;
+  if (N < 16) return w;
+  w += __popc(x & 0x03FFF800u) & 1;
+  if (N < 32) return w;
+  return w + (__popc(x & 0xFC000000u) & 1);
+}
+
 template <int kMode>
-__device__ void weights_tile(const Job& J, uint64_t lt, uint32_t* wbins, int lane, unsigned* status) {
+__device__ void weights_tile(const Job& J, uint64_t lt, uint32_t part, uint32_t split_log, uint32_t* wbins, int lane,
+                             unsigned* status) {
   const uint32_t lane_base = (uint32_t)__cvta_generic_to_shared(wbins) + (uint32_t)lane * 4u;
-  const uint64_t g0 = lt * (32ull * 256ull);
+  const uint32_t width = 256u >> split_log;
+  const uint64_t g0 = lt * (32ull * 256ull) + (uint64_t)part * width * 32;
+  if (J.wgen == WGEN_MC) {
+    // a lane takes every sample of its Philox blocks (four 32-bit or two 64-bit ones,
+    // mc_index), a few blocks at a time: the bins' asm keeps the compiler from
+    // overlapping their multiply chains otherwise.  A weight is at most the message's
+    // and six parity bits, below nbins.  2^26 samples: n = 40 0.39 -> 0.21 ms, n = 32
+    // 0.46 -> 0.16 ms against one sample per block and checked bins.
+    const uint32_t per_log = J.bucket <= 32 ? 2u : 1u;
+    const uint64_t blk0 = g0 >> per_log;  // a multiple of 64: the tile's block numbers share their high word
+    const PhiloxRun run((uint32_t)(blk0 >> 32), 0u, 0u, (uint32_t)J.seed, (uint32_t)(J.seed >> 32));
+    uint64_t p = PhiloxRun::first((uint32_t)blk0 + lane);
+    const bool whole = g0 + (uint64_t)width * 32 <= J.iters;
+    constexpr int kB = 4;
+    for (uint32_t k = 0; k < width >> per_log; k += kB) {
+      uint32_t w[4 * kB];
+#pragma unroll
+      for (int b = 0; b < kB; ++b) {
+        const Philox4 o = run.block(PhiloxRun::next(p, 32 * b));
+        if (per_log == 2) {
+          const unsigned sh = 32 - J.bucket;
+          w[4 * b] = hamming_weight_gpu(o.x >> sh, J.bucket, false);
+          w[4 * b + 1] = hamming_weight_gpu(o.y >> sh, J.bucket, false);
+          w[4 * b + 2] = hamming_weight_gpu(o.z >> sh, J.bucket, false);
+          w[4 * b + 3] = hamming_weight_gpu(o.w >> sh, J.bucket, false);
+        } else {
+          const unsigned sh = 64 - J.bucket;
+          w[4 * b] = hamming_weight_gpu((((uint64_t)o.x << 32) | o.y) >> sh, J.bucket, false);
+          w[4 * b + 1] = hamming_weight_gpu((((uint64_t)o.z << 32) | o.w) >> sh, J.bucket, false);
+        }
+      }
+      p = PhiloxRun::next(p, 32 * kB);
+#pragma unroll
+      for (int b = 0; b < kB; ++b) {
+        const uint64_t g = (blk0 + (uint64_t)(k + b) * 32 + lane) << per_log;
+        if (k + b < width >> per_log) {
+#pragma unroll
+          for (uint32_t u = 0; u < 4; ++u)
+            if (u < 1u << per_log && (whole || g + u < J.iters)) bump<kMode>(lane_base + (w[4 * b + u] << 7));
+        }
+      }
+    }
+    return;
+  }
 #pragma unroll 4
-  for (uint32_t k = 0; k < 256; ++k) {
+  for (uint32_t k = 0; k < width; ++k) {
     const uint64_t g = g0 + (uint64_t)k * 32 + lane;
     if (g >= J.iters) break;
     uint64_t x;
@@ -425,13 +504,11 @@ __device__ void weights_tile(const Job& J, uint64_t lt, uint32_t* wbins, int lan
       const uint64_t sh = g / J.shard, kk = g % J.shard;
       const uint64_t wsh = sh * J.shard * (uint64_t)J.row_step;
       x = (uint64_t)fma((double)kk, J.row_step, (double)wsh);
-    } else if (J.wgen == WGEN_MC) {
-      x = mc_index(J.seed, 0, g, J.bucket);
     } else {
       x = g;
       n4 = true;
     }
-    bump_checked<kMode>(lane_base, popc64(hamming_cw_gpu(x, J.bucket, n4)), J.nbins, status);
+    bump_checked<kMode>(lane_base, hamming_weight_gpu(x, J.bucket, n4), J.nbins, status);
   }
 }
 
@@ -447,7 +524,9 @@ __device__ __forceinline__ uint32_t find_job(const Job* jobs, uint32_t njobs, ui
   return lo;
 }
 
-template <int kMode>
+// kKind: the one kind of all the launch's jobs, or kMixedKinds.  A kernel of one kind
+// holds that kind's registers only.
+template <int kMode, int kKind>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) hist_kernel(LaunchArgs args) {
   extern __shared__ __align__(16) uint32_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -474,6 +553,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) hist_kernel(LaunchArgs args
     unsigned long long t = 0;
     if (lane == 0) t = atomicAdd(args.counter, 1ull);
     t = __shfl_sync(0xffffffffu, t, 0);
+    const uint32_t part = (uint32_t)t & ((1u << args.split_log) - 1);
+    t >>= args.split_log;
     if (t >= args.total_tiles) break;
     const uint32_t jn = find_job(args.jobs, args.njobs, t);
     if (jn >= args.njobs || t < args.jobs[jn].tile_begin ||
@@ -492,9 +573,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) hist_kernel(LaunchArgs args
     if (lane == 0) check_state().tile = t;
     __syncwarp();
 #endif
-    if (J.kind == JOB_PAIRS) pairs_tile<kMode>(J, lt, wbins, table, lane, args.status);
-    else if (J.kind == JOB_MC) mc_tile<kMode>(J, lt, wbins, lane, args.status);
-    else weights_tile<kMode>(J, lt, wbins, lane, args.status);
+    const int kind = kKind == kMixedKinds ? (int)J.kind : kKind;
+    if (kind == JOB_PAIRS) pairs_tile<kMode>(J, lt, part, args.split_log, wbins, table, lane, args.status);
+    else if (kind == JOB_MC) mc_tile<kMode>(J, lt, part, args.split_log, wbins, lane);
+    else weights_tile<kMode>(J, lt, part, args.split_log, wbins, lane, args.status);
     if (++since_flush >= kFlushEvery) { flush_bins(wbins, J.bins, J.nbins, lane); since_flush = 0; }
   }
   if (cur != 0xffffffffu && since_flush) flush_bins(wbins, J.bins, J.nbins, lane);
@@ -609,33 +691,51 @@ size_t hist_smem_bytes(uint32_t smem_bins, bool col_table) {
   return (size_t)kWarpsPerCta * ((size_t)smem_bins * 32 + (col_table ? kTileCols : 0)) * sizeof(uint32_t);
 }
 
-static const void* kernel_ptr(int mode) {
-  return mode == HIST_RED ? (const void*)hist_kernel<HIST_RED> : (const void*)hist_kernel<HIST_LDST>;
+using HistKernel = void (*)(LaunchArgs);
+template <int kMode>
+static HistKernel kernel_of(int kind) {
+  switch (kind) {
+    case JOB_PAIRS: return hist_kernel<kMode, JOB_PAIRS>;
+    case JOB_MC: return hist_kernel<kMode, JOB_MC>;
+    case JOB_WEIGHTS: return hist_kernel<kMode, JOB_WEIGHTS>;
+    default: return hist_kernel<kMode, kMixedKinds>;
+  }
+}
+static HistKernel kernel_ptr(int mode, int kind) {
+  return mode == HIST_RED ? kernel_of<HIST_RED>(kind) : kernel_of<HIST_LDST>(kind);
 }
 
 // The dynamic shared-memory limit of hist_kernel is a per-function attribute
 // shared by every host thread, so every caller sets the same value: the largest
 // any plan asks for (kMaxBins bin rows and the column table).  A per-launch
 // value could be lowered by one thread between another's set and launch.
-static cudaError_t hist_smem_limit(int mode, size_t smem) {
+static cudaError_t hist_smem_limit(int mode, int kind, size_t smem) {
   const size_t limit = hist_smem_bytes(kMaxBins, true);
   if (smem > limit) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(kernel_ptr(mode), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+  return cudaFuncSetAttribute(kernel_ptr(mode, kind), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
 }
 
-cudaError_t hist_occupancy(int mode, size_t smem, int* ctas_per_sm) {
-  cudaError_t e = hist_smem_limit(mode, smem);
+cudaError_t hist_occupancy(int mode, int kind, size_t smem, int* ctas_per_sm) {
+  cudaError_t e = hist_smem_limit(mode, kind, smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, kernel_ptr(mode), kWarpsPerCta * 32, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, kernel_ptr(mode, kind), kWarpsPerCta * 32, smem);
 }
 
-cudaError_t launch_hist(int mode, const LaunchArgs& args, int grid, size_t smem, cudaStream_t stream) {
-  cudaError_t e = hist_smem_limit(mode, smem);
+// Few tiles leave SMs without work and a lane with hundreds of serial steps: the
+// warps then claim 2^split_log-th parts of a tile (32 columns, 8 samples at least),
+// enough of them for two per resident warp.  Whole tiles against parts, kernel time:
+// A = 641, k = 10 70 -> 13 us, k = 12 68 -> 17 us, A = 58659, k = 14 70 -> 49 us,
+// Ext-Hamming n = 16 weights 56 -> 9 us (diagonal tiles on the fast path included).
+uint32_t hist_split_log(uint64_t tiles, uint64_t warps) {
+  uint32_t s = 0;
+  while (s < kMaxSplitLog && (tiles << s) < 2 * warps) ++s;
+  return s;
+}
+
+cudaError_t launch_hist(int mode, int kind, const LaunchArgs& args, int grid, size_t smem, cudaStream_t stream) {
+  cudaError_t e = hist_smem_limit(mode, kind, smem);
   if (e != cudaSuccess) return e;
-  if (mode == HIST_RED)
-    hist_kernel<HIST_RED><<<grid, kWarpsPerCta * 32, smem, stream>>>(args);
-  else
-    hist_kernel<HIST_LDST><<<grid, kWarpsPerCta * 32, smem, stream>>>(args);
+  kernel_ptr(mode, kind)<<<grid, kWarpsPerCta * 32, smem, stream>>>(args);
   return cudaGetLastError();
 }
 

@@ -12,9 +12,13 @@ namespace dd {
 // (red.shared.add) or a load/add/store on its private column.
 enum HistMode : int { HIST_RED = 0, HIST_LDST = 1 };
 
+// log2 of the parts a launch splits its tiles into, for `warps` resident warps.
+uint32_t hist_split_log(uint64_t tiles, uint64_t warps);
 size_t hist_smem_bytes(uint32_t smem_bins, bool col_table);
-cudaError_t hist_occupancy(int mode, size_t smem, int* ctas_per_sm);
-cudaError_t launch_hist(int mode, const LaunchArgs& args, int grid, size_t smem, cudaStream_t stream);
+// kind: the JobKind of all the launch's jobs, or kMixedKinds.
+constexpr int kMixedKinds = -1;
+cudaError_t hist_occupancy(int mode, int kind, size_t smem, int* ctas_per_sm);
+cudaError_t launch_hist(int mode, int kind, const LaunchArgs& args, int grid, size_t smem, cudaStream_t stream);
 cudaError_t launch_popc_rate(uint32_t iters, int grid, uint32_t* sink, cudaStream_t stream);
 // pattern 0: per-thread columns (the single tcgen05 epilogue); 1: lane columns shared by all warps (the paired one)
 cudaError_t launch_red_rate(uint32_t iters, int grid, int threads, int pattern, uint32_t* sink, cudaStream_t stream);

@@ -146,13 +146,14 @@ extern "C" int dd_histogram_noalloc(int device, void* stream, const dd_request* 
   args.use_col_table = col_table ? 1u : 0u;
   const size_t smem = hist_smem_bytes(maxb, col_table);
   int occ = 0, sms = 0;
-  e = hist_occupancy(HIST_RED, smem, &occ);
+  e = hist_occupancy(HIST_RED, kMixedKinds, smem, &occ);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess || occ < 1) {
     set_error(std::string("dd_histogram_noalloc: launch set-up: ") + cudaGetErrorString(e));
     return DD_ERR_CUDA;
   }
-  const uint64_t want = (tiles + kWarpsPerCta - 1) / kWarpsPerCta;
+  args.split_log = hist_split_log(tiles, (uint64_t)sms * occ * kWarpsPerCta);
+  const uint64_t want = ((tiles << args.split_log) + kWarpsPerCta - 1) / kWarpsPerCta;
   const int grid = (int)(want < (uint64_t)sms * occ ? (want ? want : 1) : (uint64_t)sms * occ);
 
   // clear what must start at zero, upload the jobs, launch, read back
@@ -161,7 +162,7 @@ extern "C" int dd_histogram_noalloc(int device, void* stream, const dd_request* 
   e = cudaMemcpyAsync(scratch->jobs, table, count * sizeof(Job), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(scratch->bins, 0, count * sizeof(scratch->bins[0]), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(scratch->ctl, 0, sizeof(scratch->ctl), s);
-  if (e == cudaSuccess && tiles) e = launch_hist(HIST_RED, args, grid, smem, s);
+  if (e == cudaSuccess && tiles) e = launch_hist(HIST_RED, kMixedKinds, args, grid, smem, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(raw, scratch->bins, count * sizeof(raw[0]), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(ctl, scratch->ctl, sizeof(ctl), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
