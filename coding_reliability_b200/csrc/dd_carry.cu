@@ -51,19 +51,34 @@ constexpr int kStageCols = kStageThreads / 4;
 constexpr int kUnit = 16;           // residues between the staging kernel's rows and columns
 constexpr int kLeafThreads = 256;   // folding kernel reading popcounts
 constexpr int kFoldThreads = 192;   // folding kernel reading staged histograms
+constexpr size_t kStageCells = 32u << 20;  // staged histograms of one round of blocks (768 MB)
 constexpr int kLead = 8;            // rows above a step's own that its first level reads
 constexpr int kAhead = 3;           // rows loaded ahead
 constexpr int kSlots = kLead + 1 + kAhead;
 
-struct CarryArgs {
-  uint32_t A, psi, qinv, b, nq, many, slices;
-  uint32_t row0, rows, col0, cols;  // residues of this launch: [row0, row0+rows) x [col0, col0+cols)
-  uint32_t seg;                     // rows per CTA
+// One block of residue pairs of one job: [row0, row0+rows) x [col0, col0+cols).
+struct CarryEntry {
+  uint32_t A, psi, qinv, nq, slices, wide;
+  uint32_t row0, rows, col0, cols;
   uint32_t srows, scols;            // staged rows and columns (from row0, col0)
+  uint32_t seg, segs, strips;       // folding: rows per CTA, CTAs down and across
+  uint32_t stage_seg, stage_segs, stage_strips;
+  uint32_t fold_end, stage_end;     // CTAs of the launch up to and including this entry
   uint4* st16;                      // staged histograms: words e0 e1 e2 o0 ...
   uint2* st8;                       // ... and o1 o2
   unsigned long long* acc;          // [0, kMaxBins): residue pairs v < v'; then v = v'
 };
+
+// Entries of one launch, in its parameters (short instances share a launch, and so
+// fill the GPU together; 32 entries stay below the 4 KB every launch can pass).  64
+// instances of 8-bit A, k = 14: 0.33 ms, 2.0 ms launched one by one; 256 at k = 16:
+// 2.5 ms, popc kernel 123, tcgen05 81.
+constexpr uint32_t kEntries = 32;
+struct CarryBatch {
+  uint32_t n;
+  CarryEntry e[kEntries];
+};
+static_assert(sizeof(CarryBatch) <= 4096, "kernel parameters");
 
 // One step in a running column: exchange with column c + s, combine, rotate the ring entry y.
 template <int kLevel>
@@ -95,7 +110,7 @@ __host__ __device__ constexpr int exchange_bytes(int cols) {
 // fill sectors) and kStageCols consecutive w', of which the last 2^kLevels - 1
 // only feed their neighbours.
 template <int kLevels>
-__global__ void __launch_bounds__(kStageThreads) carry_stage_kernel(CarryArgs a) {
+__global__ void __launch_bounds__(kStageThreads) carry_stage_kernel(const __grid_constant__ CarryBatch batch) {
   constexpr int kFirst = 1 << (kLevels - 1);
   constexpr int kWarm = kFirst - 1;
   constexpr int kUseful = kStageCols - ((1 << kLevels) - 1);
@@ -103,16 +118,22 @@ __global__ void __launch_bounds__(kStageThreads) carry_stage_kernel(CarryArgs a)
   constexpr int kCols = kStageThreads + 4 * kFirst;
   __shared__ __align__(16) uint8_t ex[exchange_bytes<0, kLevels>(kCols) + 16];
 
+  uint32_t idx = 0;
+  while (blockIdx.x >= batch.e[idx].stage_end) ++idx;
+  const CarryEntry& a = batch.e[idx];
+  const uint32_t cta = blockIdx.x - (idx ? batch.e[idx - 1].stage_end : 0);
+  const uint32_t cx = cta % a.stage_strips, cy = cta / a.stage_strips;
+
   const int tid = threadIdx.x, sub = tid & 3, wi = tid >> 2;
-  const uint32_t rho = blockIdx.y % kUnit, seg = blockIdx.y / kUnit;
-  const uint32_t sigma = (blockIdx.x & 3) * 4 + sub, w0 = (blockIdx.x >> 2) * kUseful;
+  const uint32_t rho = cy % kUnit, seg = cy / kUnit;
+  const uint32_t sigma = (cx & 3) * 4 + sub, w0 = (cx >> 2) * kUseful;
   const uint32_t wrows = (a.srows - rho + kUnit - 1) / kUnit;  // rows of this rho in the block
-  const uint32_t wr0 = seg * a.seg;
+  const uint32_t wr0 = seg * a.stage_seg;
   if (wr0 >= wrows) return;
-  const uint32_t wr1 = min(wrows, wr0 + a.seg);
+  const uint32_t wr1 = min(wrows, wr0 + a.stage_seg);
   // residue pairs v' < v are their mirror images; a final row reads staged rows up to 15 above it
   {
-    const uint32_t vtop = a.col0 + (blockIdx.x & 3) * 4 + 3 + kUnit * (w0 + kUseful - 1);
+    const uint32_t vtop = a.col0 + (cx & 3) * 4 + 3 + kUnit * (w0 + kUseful - 1);
     if (vtop + 15 < a.row0 + rho + kUnit * wr0) return;
   }
   const uint32_t col = sigma + kUnit * (w0 + wi), vc = a.col0 + col;
@@ -180,7 +201,7 @@ constexpr size_t fold_smem(bool many) {
 // strip of columns (one per thread, the last 2^kLevels - 1 only feed their
 // neighbours) x a segment of rows.
 template <int kBefore, int kLevels, bool kMany>
-__global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carry_fold_kernel(CarryArgs a) {
+__global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carry_fold_kernel(const __grid_constant__ CarryBatch batch) {
   constexpr int kThreads = fold_threads<kBefore>();
   constexpr int kFirst = 1 << (kLevels - 1);
   constexpr int kWarm = kFirst - 1;
@@ -191,12 +212,16 @@ __global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carr
   constexpr int kLast = kBefore + kLevels;
   extern __shared__ __align__(16) uint8_t smem[];
 
+  uint32_t idx = 0;
+  while (blockIdx.x >= batch.e[idx].fold_end) ++idx;
+  const CarryEntry& a = batch.e[idx];
+  uint32_t cta = blockIdx.x - (idx ? batch.e[idx - 1].fold_end : 0);
+  const uint32_t c0 = cta % a.strips * kUseful;
+  cta /= a.strips;
+  const uint32_t r0 = cta % a.segs * a.seg, slice = cta / a.segs;
+
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t r0 = blockIdx.y * a.seg;
-  if (r0 >= a.rows) return;
   const uint32_t r1 = min(a.rows, r0 + a.seg);
-  const uint32_t c0 = blockIdx.x * kUseful;
-  if (c0 >= a.cols) return;
   if (a.col0 + min(a.cols, c0 + kUseful) <= a.row0 + r0) return;  // no v' >= v here
 
   // shared memory
@@ -301,14 +326,16 @@ __global__ void __launch_bounds__(fold_threads<kBefore>(), kBefore ? 2 : 1) carr
             if (c2) add_hist<kOne>(at + (__popc((qr + a.A) ^ (qc + a.A)) << 7), 1, g);
           }
         } else {
-          uint32_t* f = qd + tid;
-          for (uint32_t q = qr + blockIdx.z * a.A; q < a.nq; q += a.slices * a.A)
-            for (uint32_t p = qc; p < a.nq; p += a.A) f[__popc(q ^ p) * kThreads] += 1;
+          volatile uint32_t* f = qd + tid;
+          const uint32_t fa = (uint32_t)__cvta_generic_to_shared(qd + tid);
+          for (uint32_t q = qr + slice * a.A; q < a.nq; q += a.slices * a.A)
+            for (uint32_t p = qc; p < a.nq; p += a.A) red_add<0>(fa + __popc(q ^ p) * (kThreads * 4), 1);
           for (uint32_t d = 0; d <= 16; ++d) {
             const uint32_t x = f[d * kThreads];
             if (x) {
               f[d * kThreads] = 0;
-              add_hist<kWideProduct>(at + (d << 7), x, g);
+              if (a.wide) add_hist<kWideProduct>(at + (d << 7), x, g);
+              else add_hist<kNarrow>(at + (d << 7), x, g);
             }
           }
         }
@@ -342,31 +369,37 @@ __global__ void carry_finish_kernel(const Job* jobs, const unsigned long long* a
 }
 
 template <int kBefore, int kLevels, bool kMany>
-cudaError_t run_fold(const CarryArgs& a, uint32_t slices, cudaStream_t stream) {
-  constexpr int nt = fold_threads<kBefore>(), useful = nt - ((1 << kLevels) - 1);
+cudaError_t run_fold(const CarryBatch& b, cudaStream_t stream) {
+  constexpr int nt = fold_threads<kBefore>();
   constexpr size_t smem = fold_smem<kBefore, kLevels>(kMany);
   auto fn = carry_fold_kernel<kBefore, kLevels, kMany>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((a.cols + useful - 1) / useful, (a.rows + a.seg - 1) / a.seg, slices);
-  fn<<<grid, nt, smem, stream>>>(a);
+  fn<<<b.e[b.n - 1].fold_end, nt, smem, stream>>>(b);
   return cudaGetLastError();
 }
 
 template <int kBefore, int kLevels>
-cudaError_t run_fold(const CarryPlan& p, const CarryArgs& a, cudaStream_t stream) {
-  return p.many ? run_fold<kBefore, kLevels, true>(a, p.slices, stream)
-                : run_fold<kBefore, kLevels, false>(a, 1, stream);
+cudaError_t run_batch(const CarryBatch& b, bool many, cudaStream_t stream) {
+  if constexpr (kBefore > 0) {
+    carry_stage_kernel<kBefore><<<b.e[b.n - 1].stage_end, kStageThreads, 0, stream>>>(b);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return many ? run_fold<kBefore, kLevels, true>(b, stream) : run_fold<kBefore, kLevels, false>(b, stream);
 }
 
-template <int kLevels>
-cudaError_t run_stage(CarryArgs a, cudaStream_t stream) {
-  constexpr uint32_t useful = kStageCols - ((1 << kLevels) - 1);
-  const uint32_t w = (a.scols + kUnit - 1) / kUnit, wr = (a.srows + kUnit - 1) / kUnit;
-  a.seg = (wr + (wr + 63) / 64 - 1) / ((wr + 63) / 64);
-  const dim3 grid(4 * ((w + useful - 1) / useful), kUnit * ((wr + a.seg - 1) / a.seg));
-  carry_stage_kernel<kLevels><<<grid, kStageThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+cudaError_t run_batch(const CarryBatch& b, uint32_t levels, bool many, cudaStream_t stream) {
+  switch (levels) {
+    case 1: return run_batch<0, 1>(b, many, stream);
+    case 2: return run_batch<0, 2>(b, many, stream);
+    case 3: return run_batch<0, 3>(b, many, stream);
+    case 4: return run_batch<0, 4>(b, many, stream);
+    case 5: return run_batch<1, 4>(b, many, stream);
+    case 6: return run_batch<2, 4>(b, many, stream);
+    case 7: return run_batch<3, 4>(b, many, stream);
+    default: return run_batch<4, 4>(b, many, stream);
+  }
 }
 
 }  // namespace
@@ -387,7 +420,7 @@ bool carry_wins(const Job& j) {
   return j.n >= a + 4 && j.n >= 14;
 }
 
-void carry_plan(const Job& j, int num_sms, CarryPlan& p) {
+void carry_plan(const Job& j, CarryPlan& p) {
   p = CarryPlan();
   p.A = odd_part(j.A);
   p.k = j.n;
@@ -396,70 +429,103 @@ void carry_plan(const Job& j, int num_sms, CarryPlan& p) {
   p.staged = p.b > 4 ? p.b - 4 : 0;
   p.psi = (p.A - inverse_pow2(p.k, p.A)) % p.A;
   p.qinv = inverse_pow2(p.b, p.A);
-  const uint64_t nq = 1ull << p.s;
-  p.many = nq > 2ull * p.A;
+  p.many = (1ull << p.s) > 2ull * p.A;
+  p.side = p.A;
   if (p.staged) {
     const uint32_t useful = kStageCols - ((1u << p.staged) - 1);
-    p.side = std::min(p.A, kUnit * useful * 3 - 15);
-    p.pitch = p.side + 15;
-    p.cells = (size_t)p.pitch * p.pitch;
-  } else {
-    p.side = p.A;
-  }
-  // rows per CTA: long runs amortise the rows a segment computes twice; short ones
-  // where the residue square would leave SMs without a CTA
-  const uint32_t useful = p.staged ? kFoldThreads - 15 : kLeafThreads - ((1u << p.b) - 1);
-  const uint64_t strips = (p.side + useful - 1) / useful;
-  p.seg = 256;
-  while (p.seg > 16 && strips * ((p.side + p.seg - 1) / p.seg) < 8ull * num_sms) p.seg /= 2;
-  if (p.many) {
-    const uint64_t ctas = strips * ((p.side + p.seg - 1) / p.seg), per = (nq + p.A - 1) / p.A;
-    p.slices = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(per, 4096), std::max<uint64_t>(1, 8ull * num_sms / ctas));
+    p.side = std::min(p.A, kUnit * useful * 2 - 15);
+    p.cells = (size_t)(p.side + 15) * (p.side + 15);
   }
 }
 
-size_t carry_stage_bytes(const CarryPlan& p) { return p.staged ? p.cells * 24 + 256 : 0; }
-
-cudaError_t launch_carry(const CarryPlan& p, unsigned long long* acc, void* stage, cudaStream_t stream) {
-  cudaError_t e = cudaSuccess;
-  CarryArgs a{};
-  a.A = p.A;
-  a.psi = p.psi;
-  a.qinv = p.qinv;
-  a.b = p.b;
-  a.nq = 1u << p.s;
-  a.many = p.many;
-  a.slices = p.slices;
-  a.acc = acc;
-  a.seg = p.seg;
-  if (!p.staged) {
-    a.rows = a.cols = p.A;
-    switch (p.b) {
-      case 1: e = run_fold<0, 1>(p, a, stream); break;
-      case 2: e = run_fold<0, 2>(p, a, stream); break;
-      case 3: e = run_fold<0, 3>(p, a, stream); break;
-      default: e = run_fold<0, 4>(p, a, stream); break;
-    }
-  } else {
-    a.st16 = static_cast<uint4*>(stage);
-    a.st8 = reinterpret_cast<uint2*>(a.st16 + p.cells);
-    for (uint32_t r0 = 0; r0 < p.A && e == cudaSuccess; r0 += p.side)
-      for (uint32_t c0 = r0; c0 < p.A && e == cudaSuccess; c0 += p.side) {
-        a.row0 = r0;
-        a.col0 = c0;
-        a.rows = std::min(p.side, p.A - r0);
-        a.cols = std::min(p.side, p.A - c0);
-        a.srows = a.rows + 15;
-        a.scols = a.cols + 15;
-        switch (p.staged) {
-          case 1: e = run_stage<1>(a, stream); if (e == cudaSuccess) e = run_fold<1, 4>(p, a, stream); break;
-          case 2: e = run_stage<2>(a, stream); if (e == cudaSuccess) e = run_fold<2, 4>(p, a, stream); break;
-          case 3: e = run_stage<3>(a, stream); if (e == cudaSuccess) e = run_fold<3, 4>(p, a, stream); break;
-          default: e = run_stage<4>(a, stream); if (e == cudaSuccess) e = run_fold<4, 4>(p, a, stream); break;
-        }
-      }
+size_t carry_stage_bytes(const std::vector<CarryPlan>& plans) {
+  size_t all = 0, one = 0;
+  for (const CarryPlan& p : plans) {
+    const size_t blocks = (p.A + p.side - 1) / p.side;
+    all += p.cells * (blocks * (blocks + 1) / 2);
+    one = std::max(one, p.cells);
   }
-  return e;
+  // one round of blocks, at most kStageCells unless a single one is larger
+  return std::max(one, std::min(all, kStageCells)) * 24;
+}
+
+cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsigned long long* acc, void* stage,
+                         size_t stage_bytes, cudaStream_t stream) {
+  uint4* st16 = static_cast<uint4*>(stage);
+  const size_t cells = stage_bytes / 24;
+  uint2* st8 = reinterpret_cast<uint2*>(st16 + cells);
+  std::vector<bool> done(plans.size(), false);
+  for (size_t first = 0; first < plans.size(); ++first) {
+    if (done[first]) continue;
+    // the jobs that run the same kernels, their blocks in rounds that fit the staging memory
+    const uint32_t levels = plans[first].b, many = plans[first].many;
+    size_t alike = 0;
+    for (const CarryPlan& p : plans) alike += p.b == levels && p.many == many;
+    CarryBatch b{};
+    size_t used = 0;
+    for (size_t i = first; i < plans.size(); ++i) {
+      const CarryPlan& p = plans[i];
+      if (done[i] || p.b != levels || p.many != many) continue;
+      done[i] = true;
+      for (uint32_t r0 = 0; r0 < p.A; r0 += p.side)
+        for (uint32_t c0 = r0; c0 < p.A; c0 += p.side) {
+          CarryEntry e{};
+          e.A = p.A;
+          e.psi = p.psi;
+          e.qinv = p.qinv;
+          e.nq = 1u << p.s;
+          e.row0 = r0;
+          e.col0 = c0;
+          e.rows = std::min(p.side, p.A - r0);
+          e.cols = std::min(p.side, p.A - c0);
+          e.acc = acc + i * 2 * kMaxBins;
+          const uint32_t useful = p.staged ? kFoldThreads - 15 : kLeafThreads - ((1u << p.b) - 1);
+          e.strips = (e.cols + useful - 1) / useful;
+          // rows per CTA: long runs amortise the rows a segment computes twice; short
+          // ones where the launch would leave SMs without a CTA
+          const uint64_t want = std::max<uint64_t>(1, 8ull * num_sms / std::min<size_t>(alike, kEntries));
+          e.seg = 256;
+          while (e.seg > 16 && (uint64_t)e.strips * ((e.rows + e.seg - 1) / e.seg) < want) e.seg /= 2;
+          e.segs = (e.rows + e.seg - 1) / e.seg;
+          e.slices = 1;
+          if (p.many) {
+            // every slice computes the windows again, so only as many as fill the GPU once
+            // (A = 867, k = 21: 0.65 ms with four times as many, 0.32 ms)
+            const uint64_t per = (e.nq + p.A - 1) / p.A, ctas = (uint64_t)e.strips * e.segs;
+            e.slices = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(per, 4096), std::max<uint64_t>(1, want / 4 / ctas));
+            // a lane's 32-bit sums: rows x warps (x one lane) x q pairs x 4^b
+            const uint64_t sum = (uint64_t)e.seg * (kLeafThreads / 32) * ((per + e.slices - 1) / e.slices) * per << (2 * p.b);
+            e.wide = per > 4096 || sum > 0xFFFFFFFFull;
+          }
+          const size_t need = p.staged ? (size_t)(e.rows + 15) * (e.cols + 15) : 0;
+          if (b.n == kEntries || (b.n && used + need > cells)) {
+            const cudaError_t err = run_batch(b, levels, many != 0, stream);
+            if (err != cudaSuccess) return err;
+            b.n = 0;
+            used = 0;
+          }
+          if (p.staged) {
+            e.srows = e.rows + 15;
+            e.scols = e.cols + 15;
+            e.st16 = st16 + used;
+            e.st8 = st8 + used;
+            used += need;
+            const uint32_t su = kStageCols - ((1u << p.staged) - 1);
+            const uint32_t w = (e.scols + kUnit - 1) / kUnit, wr = (e.srows + kUnit - 1) / kUnit;
+            e.stage_strips = 4 * ((w + su - 1) / su);
+            e.stage_segs = (wr + 63) / 64;
+            e.stage_seg = (wr + e.stage_segs - 1) / e.stage_segs;
+          }
+          const CarryEntry* before = b.n ? &b.e[b.n - 1] : nullptr;
+          e.fold_end = (before ? before->fold_end : 0) + e.strips * e.segs * e.slices;
+          e.stage_end = (before ? before->stage_end : 0) + e.stage_strips * e.stage_segs * kUnit;
+          b.e[b.n++] = e;
+        }
+    }
+    const cudaError_t err = run_batch(b, levels, many != 0, stream);
+    if (err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_carry_finish(const Job* jobs, const unsigned long long* acc, uint32_t n, cudaStream_t stream) {

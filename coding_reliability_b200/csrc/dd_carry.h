@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "dd_jobs.h"
 
@@ -18,10 +19,7 @@ struct CarryPlan {
   uint32_t psi = 0;     // high word of t: psi * t mod A
   uint32_t qinv = 0;    // first q of residue v: qinv * v mod A
   uint32_t many = 0;    // a residue has more than two q
-  uint32_t slices = 1;  // many: CTAs that share a tile's q rows
-  uint32_t side = 0;    // residues per side of a staged block (staged > 0)
-  uint32_t pitch = 0;   // staged columns
-  uint32_t seg = 0;     // residue rows per CTA of the folding kernel
+  uint32_t side = 0;    // residues per side of a block
   size_t cells = 0;     // staged histograms of one block
 };
 
@@ -29,13 +27,13 @@ struct CarryPlan {
 bool carry_eligible(const Job& j);
 // The rule that picks this path for an eligible job under AUTO.
 bool carry_wins(const Job& j);
-void carry_plan(const Job& j, int num_sms, CarryPlan& p);
-// Bytes of staging memory a plan needs (0: none).
-size_t carry_stage_bytes(const CarryPlan& p);
-// Enqueues one job's kernels: its sums are added to acc (2 x kMaxBins uint64, zeroed
-// by the caller); stage is carry_stage_bytes(p) bytes, free for the next job in the
-// stream afterwards.
-cudaError_t launch_carry(const CarryPlan& p, unsigned long long* acc, void* stage, cudaStream_t stream);
+void carry_plan(const Job& j, CarryPlan& p);
+// Bytes of staging memory that serve any launch of these plans (0: none).
+size_t carry_stage_bytes(const std::vector<CarryPlan>& plans);
+// Enqueues the jobs' kernels: job i's sums are added to acc + i * 2 * kMaxBins (zeroed
+// by the caller).
+cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsigned long long* acc, void* stage,
+                         size_t stage_bytes, cudaStream_t stream);
 // acc of n jobs (2 x kMaxBins each) -> their bins; jobs: the device's table entries.
 cudaError_t launch_carry_finish(const Job* jobs, const unsigned long long* acc, uint32_t n, cudaStream_t stream);
 

@@ -190,8 +190,9 @@ __global__ void __launch_bounds__(Form<kTree>::kThreads, kTree ? 2 : 1) carry_ro
       if constexpr (!kMany) {
         for (uint32_t p = e0; p < e1; p += a.A) add_hist<kOne>(at + (__popc(e ^ p) << 7), 1, g);
       } else {
-        uint32_t* f = ed + tid;
-        for (uint32_t p = e0; p < e1; p += a.A) f[__popc(e ^ p) * F::kThreads] += 1;
+        volatile uint32_t* f = ed + tid;
+        const uint32_t fa = (uint32_t)__cvta_generic_to_shared(ed + tid);
+        for (uint32_t p = e0; p < e1; p += a.A) red_add<0>(fa + __popc(e ^ p) * (F::kThreads * 4), 1);
         for (uint32_t d = 0; d <= a.k - F::kB; ++d) {
           const uint32_t x = f[d * F::kThreads];
           if (x) {

@@ -116,14 +116,14 @@ static int ensure_capacity(dd_context* ctx, uint32_t slots, uint32_t njobs) {
 // when the device has no room for it (its jobs then take the pair kernels).
 static bool ensure_stage(dd_context* ctx, size_t bytes) {
   if (bytes <= ctx->stage_cap) return true;
-  drop_graph(ctx);
-  if (ctx->d_stage) cudaFree(ctx->d_stage);
-  ctx->d_stage = nullptr;
-  ctx->stage_cap = 0;
-  if (cudaMalloc(&ctx->d_stage, bytes) != cudaSuccess) {
+  void* mem = nullptr;
+  if (cudaMalloc(&mem, bytes) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
+  drop_graph(ctx);
+  if (ctx->d_stage) cudaFree(ctx->d_stage);
+  ctx->d_stage = mem;
   ctx->stage_cap = bytes;
   return true;
 }
@@ -172,8 +172,8 @@ static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel) {
 // (carry_wins) and its staging memory is to be had, else a pair kernel.
 static Route route_of(dd_context* ctx, const Job& j, uint32_t kernel) {
   if (carry_eligible(j) && (kernel == DD_KERNEL_CARRY || (kernel == DD_KERNEL_AUTO && carry_wins(j)))) {
-    CarryPlan p;
-    carry_plan(j, ctx->num_sms, p);
+    std::vector<CarryPlan> p(1);
+    carry_plan(j, p[0]);
     if (ensure_stage(ctx, carry_stage_bytes(p))) return ROUTE_CARRY;
   }
   RowsPlan rp;
@@ -205,7 +205,9 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.npopc = of_route[ROUTE_POPC];
   lp.nmma = of_route[ROUTE_MMA];
   lp.carry.resize(of_route[ROUTE_CARRY]);
-  for (size_t c = 0; c < lp.carry.size(); ++c) carry_plan(table[lp.npopc + lp.nmma + c], ctx->num_sms, lp.carry[c]);
+  for (size_t c = 0; c < lp.carry.size(); ++c) carry_plan(table[lp.npopc + lp.nmma + c], lp.carry[c]);
+  // room for several of them at once, where it is to be had (one fits: route_of)
+  ensure_stage(ctx, carry_stage_bytes(lp.carry));
   const uint32_t pair_jobs = lp.npopc + lp.nmma;
   lp.rows.resize(of_route[ROUTE_ROWS]);
   for (size_t c = 0; c < lp.rows.size(); ++c) rows_plan(table[pair_jobs + lp.carry.size() + c], ctx->num_sms, lp.rows[c]);
@@ -291,8 +293,7 @@ static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing)
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev0, s, evflags));
   if (lp.pgrid) DD_CUDA(launch_hist(ctx->hist_mode, lp.pkind, lp.pargs, lp.pgrid, lp.psmem, s));
   if (lp.mgrid) DD_CUDA(launch_mma(lp.margs, lp.mgrid, lp.msmem, s));
-  for (uint32_t c = 0; c < ncarry; ++c)
-    DD_CUDA(launch_carry(lp.carry[c], acc + (size_t)c * 2 * kMaxBins, ctx->d_stage, s));
+  if (ncarry) DD_CUDA(launch_carry(lp.carry, ctx->num_sms, acc, ctx->d_stage, ctx->stage_cap, s));
   if (ncarry) DD_CUDA(launch_carry_finish(ctx->d_jobs + lp.npopc + lp.nmma, acc, ncarry, s));
   for (uint32_t c = 0; c < nrows; ++c) DD_CUDA(launch_rows(ctx->h_jobs[njobs - nrows + c], lp.rows[c], s));
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev1, s, evflags));

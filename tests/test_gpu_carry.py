@@ -38,6 +38,19 @@ def test_carry_vs_tcgen05(ctx, A, k):
     assert res.raw == mma.raw and res.counts == mma.counts and res.minb == mma.minb
 
 
+def test_carry_batch(ctx):
+    """Jobs of one launch: more than a launch's 32 entries, every window length, few
+    and many q, and staged blocks that need several rounds."""
+    qs = [req(A, k, dd.KERNEL_CARRY) for k in (12, 13) for A in range(33, 33 + 2 * 40, 2)]
+    qs += [req(A, 14, dd.KERNEL_CARRY) for A in (1, 5, 17, 63, 255, 511, 1023, 2047, 4095, 8191)]
+    qs += [req(A, 17, dd.KERNEL_CARRY) for A in (4001, 4003, 4005, 4007)]
+    want = [ctx.histogram(req(q.A, q.n, dd.KERNEL_POPC)).raw for q in qs]
+    for graph in (False, True, True):
+        out = ctx.batch(qs, use_graph=graph, kernel=dd.KERNEL_CARRY)
+        for q, r, w in zip(qs, out, want):
+            assert r.kernel_used == dd.KERNEL_CARRY and r.raw == w, (q.A, q.n)
+
+
 def grid(A, k, m, kernel, **kw):
     return dd.Request(dd.CODE_AN, dd.MODE_GRID_1D, A, k, m=m, kernel=kernel, **kw)
 
