@@ -149,38 +149,68 @@ static uint32_t mma_epilogue_of(const dd_context* ctx) {
   return ctx->mma_epilogue == DD_MMA_EPILOGUE_AUTO ? ctx->mma_tuned_epilogue : ctx->mma_epilogue;
 }
 
-// Jobs below this many distance evaluations stay on the popc kernel under
-// AUTO: the tcgen05 kernel's fixed cost per launch (TMEM allocation, clearing
-// its ~180 KB of shared-memory table, barrier set-up) outweighs its rate there
-// (A = 641, k = 12, 8.4e6 pairs: popc 0.09 ms, tcgen05 0.44 ms; k = 16, 2.1e9
-// pairs, one launch each: tcgen05 0.41 ms, popc 0.57 ms).
-constexpr double kMmaMinPairs = 1073741824.0;  // 2^30
+// Under AUTO, jobs below these many distance evaluations stay on the popc kernel: the
+// tcgen05 kernel's fixed cost per launch (TMEM allocation, clearing and folding its
+// ~180 KB table) outweighs its rate there, and a triangle's diagonal strips weigh more
+// on it.  Exhaustive, one instance: k = 15, 5.4e8 pairs, popc 0.145 ms, tcgen05 0.129 ms;
+// k = 14 0.049 and 0.063 ms.  Grids: 1.6e8 pairs 0.18 and 0.10 ms.  In a launch of many
+// instances the fixed cost is shared: 16 of k = 14 0.53 and 0.42 ms, 64 of k = 12 0.15
+// and 0.21 ms.
+constexpr double kMmaMinTriangle = 536870912.0;  // 2^29
+constexpr double kMmaMinRect = 134217728.0;      // 2^27
+constexpr double kMmaMinShared = 67108864.0;     // 2^26, in a launch of
+constexpr double kMmaMinLaunch = 1073741824.0;   // 2^30 or more in such jobs
 
-// Which kernel runs a job: explicit MMA or POPC requests are honoured where
+static double pairs_of(const Job& j) {
+  return j.shape == SHAPE_TRIANGLE ? 0.5 * (double)j.rows * (double)j.rows : (double)j.rows * (double)j.cols;
+}
+
+// Which pair kernel runs a job: explicit MMA or POPC requests are honoured where
 // the job allows them; AUTO uses the context's measured preference for jobs
-// large enough to amortise the tcgen05 kernel's launch.
-static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel) {
+// large enough to amortise the tcgen05 kernel's launch.  launch_pairs: pairs of the
+// launch's jobs that could share one (0: unknown).
+static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel, double launch_pairs = 0) {
   if (!mma_eligible(j)) return false;
   if (kernel == DD_KERNEL_MMA) return true;
   if (kernel == DD_KERNEL_POPC) return false;
-  const double pairs = j.shape == SHAPE_TRIANGLE ? 0.5 * (double)j.rows * (double)j.rows
-                                                 : (double)j.rows * (double)j.cols;
-  return ctx->tuned == 2 && pairs >= kMmaMinPairs;  // autotuner's verdict for AN exhaustive shapes
+  const double least = launch_pairs >= kMmaMinLaunch ? kMmaMinShared
+                       : j.shape == SHAPE_TRIANGLE   ? kMmaMinTriangle
+                                                     : kMmaMinRect;
+  return ctx->tuned == 2 && pairs_of(j) >= least;  // autotuner's verdict for AN exhaustive shapes
 }
 
-// The route of a whole instance: the carry path where it is asked for or wins
-// (carry_wins) and its staging memory is to be had, else a pair kernel.
-static Route route_of(dd_context* ctx, const Job& j, uint32_t kernel) {
-  if (carry_eligible(j) && (kernel == DD_KERNEL_CARRY || (kernel == DD_KERNEL_AUTO && carry_wins(j)))) {
+// The jobs' routes: the carry path for each where it is asked for or wins and its
+// staging memory is to be had, a pair kernel for the others.
+static bool takes_carry(dd_context* ctx, const Job& j, uint32_t kernel, Route* route) {
+  if (kernel != DD_KERNEL_CARRY && kernel != DD_KERNEL_AUTO) return false;
+  const bool asked = kernel == DD_KERNEL_CARRY;
+  if (carry_eligible(j) && (asked || carry_wins(j))) {
     std::vector<CarryPlan> p(1);
     carry_plan(j, p[0]);
-    if (ensure_stage(ctx, carry_stage_bytes(p))) return ROUTE_CARRY;
+    if (ensure_stage(ctx, carry_stage_bytes(p))) {
+      *route = ROUTE_CARRY;
+      return true;
+    }
   }
   RowsPlan rp;
-  if ((kernel == DD_KERNEL_CARRY || kernel == DD_KERNEL_AUTO) && rows_plan(j, ctx->num_sms, rp) &&
-      (kernel == DD_KERNEL_CARRY || rows_win(j, rp)))
-    return ROUTE_ROWS;
-  return want_mma(ctx, j, kernel) ? ROUTE_MMA : ROUTE_POPC;
+  if (rows_plan(j, ctx->num_sms, rp) && (asked || rows_win(j, rp))) {
+    *route = ROUTE_ROWS;
+    return true;
+  }
+  return false;
+}
+static std::vector<Route> routes_of(dd_context* ctx, const std::vector<Job>& jobs, const dd_request* reqs) {
+  std::vector<Route> routes(jobs.size(), ROUTE_POPC);
+  std::vector<bool> carry(jobs.size());
+  double shared = 0;
+  for (size_t i = 0; i < jobs.size(); ++i) {
+    carry[i] = takes_carry(ctx, jobs[i], reqs[i].kernel, &routes[i]);
+    if (!carry[i] && reqs[i].kernel != DD_KERNEL_POPC && mma_eligible(jobs[i]) && pairs_of(jobs[i]) >= kMmaMinShared)
+      shared += pairs_of(jobs[i]);
+  }
+  for (size_t i = 0; i < jobs.size(); ++i)
+    if (!carry[i]) routes[i] = want_mma(ctx, jobs[i], reqs[i].kernel, shared) ? ROUTE_MMA : ROUTE_POPC;
+  return routes;
 }
 
 // Orders the job table (popc jobs, MMA jobs, then the two kinds of carry jobs), assigns
@@ -206,7 +236,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.nmma = of_route[ROUTE_MMA];
   lp.carry.resize(of_route[ROUTE_CARRY]);
   for (size_t c = 0; c < lp.carry.size(); ++c) carry_plan(table[lp.npopc + lp.nmma + c], lp.carry[c]);
-  // room for several of them at once, where it is to be had (one fits: route_of)
+  // room for several of them at once, where it is to be had (one fits: takes_carry)
   ensure_stage(ctx, carry_stage_bytes(lp.carry));
   const uint32_t pair_jobs = lp.npopc + lp.nmma;
   lp.rows.resize(of_route[ROUTE_ROWS]);
@@ -255,7 +285,8 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.margs.timeout_ns = ctx->mma_timeout_ns;
   lp.margs.packed = mma_epilogue_of(ctx) == DD_MMA_EPILOGUE_PAIRED ? 1u : 0u;
   lp.margs.pk_cells = 0;
-  lp.margs.pad = 0;
+  lp.margs.small_claim = 1;
+  lp.margs.big_claims = 0;
   if (lp.nmma && tm) {
     if (lp.margs.packed) {
       // one joint table for the launch, sized for its largest S; each job's
@@ -270,6 +301,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
     }
     lp.msmem = mma_smem_bytes(lp.margs.hist_rows, lp.margs.b_bufs, lp.margs.packed != 0, lp.margs.pk_cells);
     lp.mgrid = (int)std::min<uint64_t>((uint64_t)ctx->num_sms, tm);  // one CTA (one TMEM owner) per SM
+    mma_claims(lp.margs, lp.mgrid);
   }
   std::memcpy(ctx->h_jobs, table.data(), table.size() * sizeof(Job));
   return DD_OK;
@@ -545,8 +577,7 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
   }
   int st = ensure_capacity(ctx, count, count);
   if (st != DD_OK) return st;
-  std::vector<Route> routes(count);
-  for (uint32_t i = 0; i < count; ++i) routes[i] = route_of(ctx, jobs[i], reqs[i].kernel);
+  const std::vector<Route> routes = routes_of(ctx, jobs, reqs);
   LaunchPlan lp;
   st = plan_launch(ctx, jobs, routes, lp);
   if (st != DD_OK) return st;

@@ -109,8 +109,10 @@ constexpr int kColsPerWarp = kN / (kEpiWarps / 4);  // columns of a tile each ep
 constexpr int kLoads = kColsPerWarp / 32;           // 32-column TMEM loads per warp and tile
 static_assert(kEpiWarps % 4 == 0 && kColsPerWarp % 32 == 0, "whole 32-column TMEM loads per warp and tile");
 // Strips a generator claim takes: 4 super tiles, which in the column-by-column
-// tile order share their column operand (written once per claim and column).
-constexpr int kClaimStrips = 4 * kStrips;
+// tile order share their column operand (written once per claim and column).  The
+// last strips of a launch go in smaller claims, so that the CTAs end together
+// (mma_claims).
+constexpr uint32_t kClaimStrips = 4 * kStrips;
 // pair-packed epilogue
 constexpr int kPkHalf = kSuper / 2;                 // packed columns of a strip: p holds columns 2p, 2p + 1
 constexpr int kPkTilesPerStrip = kPkHalf / kN;      // 2 MMA tiles of 256 packed columns per strip
@@ -338,7 +340,7 @@ struct Shared {
   uint32_t abort;         // set by whichever wait ran out; every other wait then gives up too
   uint32_t gflag;         // generators: result of their thread 0's wait
   uint32_t pad;
-  // generators: first strip of claim c in gclaim[c & 1].  Thread 0 rewrites an entry
+  // generators: number of their claim c in gclaim[c & 1].  Thread 0 rewrites an entry
   // two claims later, past the barrier of the claim in between, which every thread
   // reaches only after reading the entry (a single word could be overwritten first
   // when every strip of a claim is skipped)
@@ -494,14 +496,14 @@ __global__ void __launch_bounds__(kThreads, 1) mma_hist_kernel(MmaArgs args) {
     bool normal = false;
     for (;;) {
       if (t >= end) {
-        if (gtid == 0) sh->gclaim[nclaim & 1] = atomicAdd(args.counter, (unsigned long long)kClaimStrips);
+        if (gtid == 0) sh->gclaim[nclaim & 1] = atomicAdd(args.counter, 1ull);
         gen_bar();
-        const unsigned long long base = sh->gclaim[nclaim & 1];
+        const unsigned long long c = sh->gclaim[nclaim & 1], big = args.big_claims;
         ++nclaim;
-        if (base >= args.total_tiles) { normal = true; break; }
-        t = base;
-        end = base + kClaimStrips < args.total_tiles ? base + (unsigned long long)kClaimStrips
-                                                     : (unsigned long long)args.total_tiles;
+        const uint64_t size = c < big ? kClaimStrips : args.small_claim;
+        t = c < big ? c * kClaimStrips : big * kClaimStrips + (c - big) * args.small_claim;
+        if (t >= args.total_tiles) { normal = true; break; }
+        end = t + size < args.total_tiles ? t + size : (uint64_t)args.total_tiles;
       }
       const unsigned long long tt = t++;
       const uint32_t jn = find_job(args.jobs, args.njobs, tt);
@@ -826,6 +828,17 @@ __global__ void __launch_bounds__(kThreads, 1) mma_hist_kernel(MmaArgs args) {
           const int64_t dhi = (int64_t)(rect ? es.cols : es.n) - (int64_t)cbase;  // o < dhi
           const int32_t lo_o = i < es.n ? (int32_t)(dlo < -1 ? -1 : (dlo > 64 ? 64 : dlo)) : 64;
           const int32_t hi_o = (int32_t)(dhi < 0 ? 0 : (dhi > 64 ? 64 : dhi));
+          // Most halves of a partial strip hold no pair that counts, or only such
+          // pairs: of the 512 of a diagonal super tile 32 hold both kinds.  64 instances of
+          // k = 16: 19.9 ms with every half checked, 18.4 ms.  (Sharing the full strips'
+          // windowed branch for them made its loop 2-3 % slower, a non-inlined checked
+          // loop 4 %.)
+          if (__all_sync(0xffffffffu, lo_o + 1 >= hi_o)) return;
+          if (pkall && __all_sync(0xffffffffu, lo_o < 0 && hi_o == 64)) {
+#pragma unroll
+            for (int u = 0; u < 32; ++u) red_shared(pk_lane + (x[u] << 7));
+            return;
+          }
 #pragma unroll
           for (int u = 0; u < 32; ++u) {
             const bool v1 = 2 * u > lo_o && 2 * u < hi_o;
@@ -1025,6 +1038,16 @@ size_t mma_smem_bytes(uint32_t hist_rows, uint32_t b_bufs, bool packed, uint32_t
 
 uint32_t mma_b_bufs(uint32_t hist_rows) {
   return mma_smem_bytes(hist_rows, 2, false, 0) <= smem_optin() ? 2u : 1u;
+}
+
+// Claims of 32 strips up to the last two super tiles per CTA, then of 8 (one super
+// tile's columns); launches with less work than that go in two claims per CTA.  Against
+// claims of 32 throughout: A = 58659, k = 13 0.205 -> 0.041 ms, k = 15 0.21 -> 0.126 ms,
+// 2-D grid of 33333 x 100001 points 0.84 -> 0.67 ms.
+void mma_claims(MmaArgs& args, int grid) {
+  const uint64_t tail = (uint64_t)grid * kStrips * 2;
+  args.big_claims = args.total_tiles > tail ? (args.total_tiles - tail) / kClaimStrips : 0;
+  args.small_claim = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kStrips, args.total_tiles / (2 * (uint64_t)grid)));
 }
 
 cudaError_t launch_mma(const MmaArgs& args, int grid, size_t smem, cudaStream_t stream) {

@@ -19,7 +19,8 @@ struct MmaArgs {
   uint32_t b_bufs;           // column-operand buffers in shared memory: 2 when they fit next to the bins, else 1
   uint32_t packed;           // 1: pair-packed epilogue (two distances per MMA column, joint-bin table)
   uint32_t pk_cells;         // pair-packed: joint-table cells of this launch (S x window rows of its jobs)
-  uint32_t pad;
+  uint32_t small_claim;      // strips of a claim after the first big_claims (mma_claims)
+  unsigned long long big_claims;
 };
 
 // True if the job can run on the MMA path: all pairs of a codeword progression or
@@ -43,6 +44,8 @@ void mma_pack_setup(Job& j, uint32_t cells);
 // Column-operand buffers that fit in shared memory next to the bins (single epilogue).
 uint32_t mma_b_bufs(uint32_t hist_rows);
 size_t mma_smem_bytes(uint32_t hist_rows, uint32_t b_bufs, bool packed, uint32_t pk_cells);
+// Sets the sizes of the strips' claims for a grid of CTAs.
+void mma_claims(MmaArgs& args, int grid);
 cudaError_t launch_mma(const MmaArgs& args, int grid, size_t smem, cudaStream_t stream);
 
 }  // namespace dd
