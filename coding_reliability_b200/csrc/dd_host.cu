@@ -29,7 +29,11 @@ struct dd_context {
   bool own_stream = false;
   int num_sms = 0;
   // device state
-  unsigned long long* d_bins = nullptr;  // bin_slots x kMaxBins, then the carry path's sums (2 x kMaxBins a slot)
+  // one buffer, so that a launch clears it with one memset and reads it back with one
+  // copy: control words, the launch's bins (kMaxBins a slot), then the carry path's
+  // sums (2 x kMaxBins a job)
+  unsigned long long* d_mem = nullptr;
+  unsigned long long* d_bins = nullptr;  // bin_slots x kMaxBins
   uint32_t bin_slots = 0;
   unsigned long long* d_ctl = nullptr;   // [0] popc work counter, [1] MMA work counter, [2] status, [3..15] diagnostics
   dd::Job* d_jobs = nullptr;
@@ -37,10 +41,13 @@ struct dd_context {
   void* d_stage = nullptr;               // carry path: staged histograms of one block
   size_t stage_cap = 0;
   // pinned host mirrors
+  unsigned long long* h_mem = nullptr;   // control words, bins
   unsigned long long* h_bins = nullptr;
   unsigned long long* h_ctl = nullptr;
   dd::Job* h_jobs = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // resident popc CTAs per SM by bin increment, job kind, bins and column table (0: not asked yet)
+  int occupancy[2][4][dd::kMaxBins + 1][2] = {};
   // tuning
   int hist_mode = dd::HIST_RED;
   int tuned = 0;
@@ -86,15 +93,19 @@ static int ensure_capacity(dd_context* ctx, uint32_t slots, uint32_t njobs) {
   DD_CUDA(cudaSetDevice(ctx->device));
   if (slots > ctx->bin_slots || njobs > ctx->job_cap) drop_graph(ctx);
   if (slots > ctx->bin_slots) {
-    if (ctx->d_bins) cudaFree(ctx->d_bins);
-    if (ctx->h_bins) cudaFreeHost(ctx->h_bins);
-    ctx->d_bins = nullptr;
-    ctx->h_bins = nullptr;
+    if (ctx->d_mem) cudaFree(ctx->d_mem);
+    if (ctx->h_mem) cudaFreeHost(ctx->h_mem);
+    ctx->d_mem = ctx->d_ctl = ctx->d_bins = nullptr;
+    ctx->h_mem = ctx->h_ctl = ctx->h_bins = nullptr;
     ctx->bin_slots = 0;
     const uint32_t cap = std::max<uint32_t>(slots, 64);
-    cudaError_t e = cudaMalloc(&ctx->d_bins, (size_t)cap * 3 * kMaxBins * sizeof(unsigned long long));
+    cudaError_t e = cudaMalloc(&ctx->d_mem, (kCtlWords + (size_t)cap * 3 * kMaxBins) * sizeof(unsigned long long));
     if (e != cudaSuccess) { set_error("bins: cudaMalloc failed"); return DD_ERR_OUT_OF_MEMORY; }
-    DD_CUDA(cudaMallocHost(&ctx->h_bins, (size_t)cap * kMaxBins * sizeof(unsigned long long)));
+    DD_CUDA(cudaMallocHost(&ctx->h_mem, (kCtlWords + (size_t)cap * kMaxBins) * sizeof(unsigned long long)));
+    ctx->d_ctl = ctx->d_mem;
+    ctx->d_bins = ctx->d_mem + kCtlWords;
+    ctx->h_ctl = ctx->h_mem;
+    ctx->h_bins = ctx->h_mem + kCtlWords;
     ctx->bin_slots = cap;
   }
   if (njobs > ctx->job_cap) {
@@ -266,8 +277,8 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.pargs.split_log = 0;
   if (lp.npopc && tp) {
     lp.psmem = hist_smem_bytes(maxb, col_table);
-    int occ = 0;
-    DD_CUDA(hist_occupancy(ctx->hist_mode, lp.pkind, lp.psmem, &occ));
+    int& occ = ctx->occupancy[ctx->hist_mode == HIST_RED][lp.pkind + 1][maxb][col_table];
+    if (!occ) DD_CUDA(hist_occupancy(ctx->hist_mode, lp.pkind, lp.psmem, &occ));
     if (occ < 1) { set_error("kernel does not fit on an SM"); return DD_ERR_UNSUPPORTED; }
     lp.pargs.split_log = hist_split_log(tp, (uint64_t)ctx->num_sms * occ * kWarpsPerCta);
     const uint64_t want = ((tp << lp.pargs.split_log) + kWarpsPerCta - 1) / kWarpsPerCta;
@@ -314,10 +325,9 @@ static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing)
   const uint32_t ncarry = (uint32_t)lp.carry.size(), nrows = (uint32_t)lp.rows.size();
   const uint32_t njobs = lp.npopc + lp.nmma + ncarry + nrows;
   DD_CUDA(cudaMemcpyAsync(ctx->d_jobs, ctx->h_jobs, njobs * sizeof(Job), cudaMemcpyHostToDevice, s));
-  unsigned long long* acc = ctx->d_bins + (size_t)ctx->bin_slots * kMaxBins;
-  if (ncarry) DD_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncarry * 2 * kMaxBins * sizeof(unsigned long long), s));
-  DD_CUDA(cudaMemsetAsync(ctx->d_bins, 0, (size_t)lp.nslots * kMaxBins * sizeof(unsigned long long), s));
-  DD_CUDA(cudaMemsetAsync(ctx->d_ctl, 0, kCtlWords * sizeof(unsigned long long), s));
+  unsigned long long* acc = ctx->d_bins + (size_t)lp.nslots * kMaxBins;
+  const size_t result_bytes = (kCtlWords + (size_t)lp.nslots * kMaxBins) * sizeof(unsigned long long);
+  DD_CUDA(cudaMemsetAsync(ctx->d_mem, 0, result_bytes + (size_t)ncarry * 2 * kMaxBins * sizeof(unsigned long long), s));
   // Inside a stream capture the records must be external so that they become
   // event-record nodes of the graph (the kernel time is then measurable on
   // every replay); outside a capture the flag is not accepted.
@@ -329,9 +339,7 @@ static int enqueue_launch(dd_context* ctx, const LaunchPlan& lp, bool capturing)
   if (ncarry) DD_CUDA(launch_carry_finish(ctx->d_jobs + lp.npopc + lp.nmma, acc, ncarry, s));
   for (uint32_t c = 0; c < nrows; ++c) DD_CUDA(launch_rows(ctx->h_jobs[njobs - nrows + c], lp.rows[c], s));
   DD_CUDA(cudaEventRecordWithFlags(ctx->ev1, s, evflags));
-  DD_CUDA(cudaMemcpyAsync(ctx->h_bins, ctx->d_bins, (size_t)lp.nslots * kMaxBins * sizeof(unsigned long long),
-                          cudaMemcpyDeviceToHost, s));
-  DD_CUDA(cudaMemcpyAsync(ctx->h_ctl, ctx->d_ctl, kCtlWords * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+  DD_CUDA(cudaMemcpyAsync(ctx->h_mem, ctx->d_mem, result_bytes, cudaMemcpyDeviceToHost, s));
   return DD_OK;
 }
 
@@ -454,8 +462,6 @@ int dd_context_create(int device, void* stream, dd_context** out) {
     if (stream) ctx->stream = (cudaStream_t)stream;
     else { e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking); ctx->own_stream = true; }
   }
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_ctl, kCtlWords * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_ctl, kCtlWords * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
   if (e != cudaSuccess) {
@@ -480,12 +486,10 @@ int dd_context_destroy(dd_context* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-  if (ctx->d_bins) cudaFree(ctx->d_bins);
-  if (ctx->d_ctl) cudaFree(ctx->d_ctl);
-  if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
+  if (ctx->d_mem) cudaFree(ctx->d_mem);
   if (ctx->d_jobs) cudaFree(ctx->d_jobs);
   if (ctx->d_stage) cudaFree(ctx->d_stage);
-  if (ctx->h_bins) cudaFreeHost(ctx->h_bins);
+  if (ctx->h_mem) cudaFreeHost(ctx->h_mem);
   if (ctx->h_jobs) cudaFreeHost(ctx->h_jobs);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
