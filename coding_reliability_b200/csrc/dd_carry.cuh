@@ -151,9 +151,8 @@ __device__ __forceinline__ H8 first_level(uint32_t ra, uint32_t rb, uint32_t ca,
   return add_z(same.bytes(), cross.bytes());
 }
 
-__device__ __forceinline__ uint32_t mul_mod(uint32_t a, uint32_t v, uint32_t A) {
-  return (uint32_t)((uint64_t)a * v % A);
-}
+// a v mod A for a < A < 2^16 (32-bit divisions only)
+__device__ __forceinline__ uint32_t mul_mod(uint32_t a, uint32_t v, uint32_t A) { return a * (v % A) % A; }
 __device__ __forceinline__ uint32_t sub_mod(uint32_t x, uint32_t d, uint32_t A) { return x >= d ? x - d : x + A - d; }
 
 template <int kOffset>
