@@ -37,11 +37,13 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
 // acc of n jobs (2 x kMaxBins each) -> their bins; jobs: the device's table entries.
 cudaError_t launch_carry_finish(const Job* jobs, const unsigned long long* acc, uint32_t n, cudaStream_t stream);
 
-// One 1-D grid job as carry_rows_kernel runs it.
+// One 1-D grid job as carry_rows_kernel or carry_ring_kernel runs it.
 struct RowsPlan {
   uint32_t A = 0;           // odd part of the multiplier
   uint32_t tree = 0;        // rows with a power-of-two stride, in blocks
   uint32_t stride_log = 0;  // tree: log2 of the stride
+  uint32_t ring = 0;        // window bits of carry_ring_kernel (0: carry_rows_kernel)
+  uint32_t groups = 0;      // ring: rows side by side
   uint32_t many = 0;        // a residue stands for more columns than are worth visiting one by one
   uint32_t per = 0;         // columns of a residue per CTA
   uint32_t slices = 1;      // CTAs that share a residue's columns

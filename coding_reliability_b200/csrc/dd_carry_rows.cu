@@ -18,8 +18,8 @@
 // from level to level, so that a block of 64 rows costs about 64 first levels.
 //
 // Measured on B200 against the tcgen05 kernel: A = 62307, k = 24, m = 65536 14.8 ms
-// against 126 ms, A = 867 0.40 against 116 ms; listed rows: A = 867, k = 24, m = 10001
-// 1.5 against 18.7 ms, A = 62307, m = 1001 1.65 against 3.4 ms.  Bound by instruction
+// against 126 ms, A = 867 0.35 against 116 ms; listed rows: A = 867, k = 24, m = 10001
+// 0.43 against 18.7 ms, A = 62307, m = 1001 1.65 against 3.4 ms.  Bound by instruction
 // issue, as the exhaustive form; DRAM carries nothing.
 //
 // Thread = column residue; the neighbour u' + s comes through shared memory.  The
@@ -47,7 +47,8 @@ struct RowsArgs {
   uint64_t rows;             // rows (list), blocks (tree)
   uint64_t mult;             // list: odd part of the multiplier, 64-bit product with the lattice point
   double step;               // list: lattice point i is (uint64)(i * step)
-  uint32_t shift[9];         // shift[L] = psi * 2^(kB-L) mod A
+  uint32_t shift[17];        // shift[L] = psi * 2^(kB-L) mod A (ring: 2^(b-L) mod A)
+  uint32_t b, groups;        // ring: window bits, rows side by side in a CTA
   unsigned long long* bins;
 };
 
@@ -92,15 +93,17 @@ struct Exchange {
   uint32_t bytes, turn;
   int tid;
   template <class H>
-  __device__ __forceinline__ H with(const H& own, int s) {
+  __device__ __forceinline__ H at(const H& own, int index) {
     uint8_t* row = rows + (turn ? bytes : 0);
     turn ^= 1;
     put(row, tid, own);
     __syncthreads();
     H nb;
-    get(row, tid + s, nb);
+    get(row, index, nb);
     return nb;
   }
+  template <class H>
+  __device__ __forceinline__ H with(const H& own, int s) { return at(own, tid + s); }
 };
 
 // Level L of the tree over the rows whose high words are c + (multiples of shift[1..L]).
@@ -212,6 +215,75 @@ __global__ void __launch_bounds__(Form<kTree>::kThreads, kTree ? 2 : 1) carry_ro
   }
 }
 
+// Listed rows of a short multiplier: the columns of all A residues fit a CTA, so the
+// window closes on itself (no thread only feeds its neighbours) and may be as long as
+// b = k - bits(A) bits (at most 16), which leaves about two columns a residue to visit
+// instead of 2^(k-8) / A.  Several rows run side by side where A is at most half the CTA.
+// A = 867, k = 24, 10,001 rows: 1.35 ms with a window of 8 bits, 0.43 ms.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) carry_ring_kernel(const __grid_constant__ RowsArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint32_t* tab = reinterpret_cast<uint32_t*>(smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < kTabRows * 32; i += kThreads) tab[i] = 0;
+  Exchange ex{smem + kTabBytes, 48u * kThreads, 0, tid};
+  const uint32_t group = tid / a.A, u = tid - group * a.A, first = group * a.A;
+  const uint32_t ca = mul_mod(a.psi, u, a.A), cb = mul_mod(a.psi, u + (1u << (a.b - 1)), a.A);
+  const uint32_t e0 = mul_mod(a.einv, u, a.A);
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(tab) + lane * 4u;
+  __syncthreads();
+  auto next = [&](uint32_t L) {  // thread of the column shift[L] on
+    const uint32_t v = u + a.shift[L];
+    return (int)min(first + (v >= a.A ? v - a.A : v), (uint32_t)kThreads - 1);
+  };
+  const uint64_t i0 = (uint64_t)blockIdx.x * a.seg, i1 = min(a.rows, i0 + a.seg);
+  for (uint64_t base = i0; base < i1; base += a.groups) {
+    const uint64_t i = base + group;
+    const uint64_t y = a.mult * (uint64_t)((double)i * a.step);
+    const uint32_t t = (uint32_t)(y & ((1ull << a.k) - 1)), c = (uint32_t)(y >> a.k);
+    const uint32_t r = t >> (a.k - a.b), e = t & (a.ne - 1);
+    Nibbles same, cross;
+    const bool set = (r >> (a.b - 1)) & 1;
+    same.count(__popc(c ^ (set ? cb : ca)));
+    cross.count(__popc(c ^ (set ? ca : cb)));
+    H8 h = add_z(same.bytes(), cross.bytes());
+    uint32_t L = 2;
+#pragma unroll 1
+    for (; L <= a.b && L <= 7; ++L) {
+      const H8 nb = ex.at(h, next(L));
+      h = (r >> (a.b - L)) & 1 ? add_z(nb, h) : add_z(h, nb);
+    }
+    H16 g = widen(h);
+    if (L <= a.b) {
+      const H16 nb = widen(ex.at(h, next(L)));
+      g = (r >> (a.b - L)) & 1 ? add_z(nb, g) : add_z(g, nb);
+#pragma unroll 1
+      for (++L; L <= a.b; ++L) {
+        const H16 n = ex.at(g, next(L));
+        g = (r >> (a.b - L)) & 1 ? add_z(n, g) : add_z(g, n);
+      }
+    }
+    if (group < a.groups && i < i1)
+      for (uint32_t p = e0; p < a.ne; p += a.A) add_hist<kOne>(at + (__popc(e ^ p) << 7), 1, g);
+  }
+  __syncthreads();
+  for (int d = warp; d < kTabRows; d += kThreads / 32) {
+    const uint32_t x = tab[d * 32 + lane];
+    const unsigned long long t = (unsigned long long)__reduce_add_sync(0xffffffffu, x & 0xFFFFu) +
+                                 ((unsigned long long)__reduce_add_sync(0xffffffffu, x >> 16) << 16);
+    if (lane == 0 && t) atomicAdd(a.bins + d, t);
+  }
+}
+
+template <int kThreads>
+cudaError_t run_ring(const RowsArgs& a, cudaStream_t stream) {
+  constexpr int smem = kTabBytes + 2 * 48 * kThreads;
+  cudaError_t e = cudaFuncSetAttribute(carry_ring_kernel<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  carry_ring_kernel<kThreads><<<(uint32_t)((a.rows + a.seg - 1) / a.seg), kThreads, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
 template <bool kTree, bool kMany>
 cudaError_t run_rows(const RowsArgs& a, const RowsPlan& p, cudaStream_t stream) {
   using F = Form<kTree>;
@@ -243,6 +315,19 @@ bool rows_plan(const Job& j, int num_sms, RowsPlan& p) {
   const uint64_t st = stride >= 1 && stride < 4294967296.0 ? (uint64_t)stride : 0;
   p.tree = st && (double)st == stride && (st & (st - 1)) == 0 && j.rows == j.cols / st &&
            j.rows >= 1u << Form<true>::kB;
+  if (!p.tree && p.A <= 1024 && j.n <= 24 && j.n > bits + 1) {
+    // one wave of CTAs (two of 512 threads or one of 1024 an SM); a lane's column adds
+    // the residue's columns x 2^16 a round of rows and warp (of 32), below 2^32
+    p.ring = std::min<uint32_t>(16, j.n - bits);
+    p.rows = j.rows;
+    const uint32_t threads = p.A <= 512 ? 512 : 1024;
+    p.groups = threads / p.A;
+    const uint64_t ctas = (uint64_t)num_sms * (1024 / threads);
+    const uint64_t columns = ((1ull << (j.n - p.ring)) + p.A - 1) / p.A;  // at most 256
+    const uint64_t rounds = std::min<uint64_t>(2047 / columns, (p.rows + p.groups * ctas - 1) / (p.groups * ctas));
+    p.seg = (uint32_t)rounds * p.groups;
+    return true;
+  }
   const uint32_t kb = p.tree ? Form<true>::kB : Form<false>::kB;
   while (p.tree && (1ull << p.stride_log) < st) ++p.stride_log;
   const uint64_t ne = 1ull << (j.n - kb), most = (ne + p.A - 1) / p.A;
@@ -268,14 +353,15 @@ bool rows_plan(const Job& j, int num_sms, RowsPlan& p) {
 // The tree's residue pairs cost about as much as 30 codeword pairs of the tcgen05 kernel
 // (A = 62307, m = 65536: k = 21, 34 a residue, 13.9 ms here and 15.8 ms there; k = 20,
 // 13.9 and 7.9 ms), the list's about 170 (m = 10007: A = 62307, k = 22, 67 a residue,
-// 13.8 and 5.2 ms; A = 8191, 512 a residue, 2.3 and 4.7 ms); below 2^28 pairs the popc
+// 13.8 and 5.2 ms; A = 8191, 512 a residue, 2.3 and 4.7 ms), the ring's as many (A = 867,
+// m = 10001: k = 18, 302 a residue, 0.26 and 0.34 ms; k = 17, 0.23 and 0.19 ms); below 2^28 pairs the popc
 // kernel's single launch is as fast.
 bool rows_win(const Job& j, const RowsPlan& p) {
-  return (double)j.rows * (double)j.cols >= 268435456.0 && j.cols >= (uint64_t)p.A * (p.tree ? 32 : 256);
+  return (double)j.rows * (double)j.cols >= 268435456.0 && j.cols >= (uint64_t)p.A * (p.tree ? 32 : p.ring ? 192 : 256);
 }
 
 cudaError_t launch_rows(const Job& j, const RowsPlan& p, cudaStream_t stream) {
-  const uint32_t kb = p.tree ? Form<true>::kB : Form<false>::kB;
+  const uint32_t kb = p.ring ? p.ring : p.tree ? Form<true>::kB : Form<false>::kB;
   RowsArgs a{};
   a.A = p.A;
   a.k = j.n;
@@ -290,8 +376,16 @@ cudaError_t launch_rows(const Job& j, const RowsPlan& p, cudaStream_t stream) {
   a.stride_log = p.stride_log;
   // block q: e = 2^stride_log q, u = 2^-(k-kb) e
   a.uinv = inverse_pow2(j.n - kb - (p.tree ? p.stride_log : 0), p.A);
-  for (uint32_t L = 1; L <= kb; ++L) a.shift[L] = (uint32_t)((uint64_t)a.psi * (1ull << (kb - L)) % p.A);
+  for (uint32_t L = 1; L <= kb; ++L) {
+    const uint64_t s = (1ull << (kb - L)) % p.A;
+    a.shift[L] = (uint32_t)(p.ring ? s : a.psi * s % p.A);
+  }
   a.bins = j.bins;
+  if (p.ring) {
+    a.b = p.ring;
+    a.groups = p.groups;
+    return p.A <= 512 ? run_ring<512>(a, stream) : run_ring<1024>(a, stream);
+  }
   if (p.tree) return p.many ? run_rows<true, true>(a, p, stream) : run_rows<true, false>(a, p, stream);
   return p.many ? run_rows<false, true>(a, p, stream) : run_rows<false, false>(a, p, stream);
 }

@@ -4,7 +4,8 @@ kernel, bit-exact: every window length (k - bits(A) = 1..8 levels, one kernel up
 edges of the column strips (112 and 177 useful columns), row segments and staged
 blocks (5409 and 6081 residues a side).  The 1-D grid form (dd_carry_rows.cu): rows
 in blocks of a power-of-two stride and listed rows, strips of 449 and 769 useful
-columns, few and many columns a residue, several slices of them."""
+columns, few and many columns a residue, several slices of them, and all residues in
+one CTA (A <= 512 and <= 1024)."""
 import pytest
 
 import coding_reliability_b200 as dd
@@ -56,7 +57,8 @@ def grid(A, k, m, kernel, **kw):
 
 
 @pytest.mark.parametrize("A,k,m", [(1, 12, 64), (3, 12, 13), (5, 13, 4096), (61, 12, 4096), (449, 12, 65), (451, 13, 64),
-                                   (641, 14, 1000), (769, 13, 3), (771, 12, 17), (1021, 15, 333), (976, 14, 128)])
+                                   (641, 14, 1000), (1023, 13, 3), (771, 12, 17), (1021, 15, 333), (976, 14, 128),
+                                   (1, 13, 100), (33, 14, 777), (511, 13, 2047), (513, 12, 1001), (1537, 13, 99)])
 def test_grid_vs_oracle(ctx, A, k, m):
     q = grid(A, k, m, dd.KERNEL_CARRY)
     nb, h, Aeff = dd.request_shape(q)
@@ -66,7 +68,8 @@ def test_grid_vs_oracle(ctx, A, k, m):
 
 
 @pytest.mark.parametrize("A,k,m", [(65535, 16, 256), (65535, 20, 100), (32769, 24, 128), (8191, 22, 1 << 12),
-                                   (1283, 24, 99), (61, 24, 1 << 10), (33, 27, 64), (35, 25, 21), (65535, 27, 64)])
+                                   (1283, 24, 99), (61, 24, 1 << 10), (33, 27, 64), (35, 25, 21), (65535, 27, 64), (127, 24, 301),
+                                   (33, 23, 1001), (867, 22, 333), (1027, 22, 333)])
 def test_grid_vs_tcgen05(ctx, A, k, m):
     res = ctx.histogram(grid(A, k, m, dd.KERNEL_CARRY))
     mma = ctx.histogram(grid(A, k, m, dd.KERNEL_MMA))
