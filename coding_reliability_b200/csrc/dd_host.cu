@@ -298,6 +298,8 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   lp.margs.pk_cells = 0;
   lp.margs.small_claim = 1;
   lp.margs.big_claims = 0;
+  lp.margs.big_claim = 1;
+  lp.margs.pad = 0;
   if (lp.nmma && tm) {
     if (lp.margs.packed) {
       // one joint table for the launch, sized for its largest S; each job's

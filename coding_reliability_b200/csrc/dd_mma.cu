@@ -41,10 +41,10 @@
 // runs while the epilogue bins tile t.  (Four buffers of N = 128 measured 17 %
 // slower for the single epilogue: every tile costs each epilogue warp a barrier
 // poll and an arrive through the shared-memory pipe that its atomics saturate,
-// so fewer, wider tiles win over deeper buffering.)  Generator warps claim 32
-// strips at a time (four super tiles when the job's tile range is aligned,
-// which in the column-by-column order mostly share one column) and write the
-// column operand only when the column super tile changes, into the second of
+// so fewer, wider tiles win over deeper buffering.)  Generator warps claim up
+// to 256 strips at a time (32 super tiles, which in the column-by-column order
+// mostly share one column; smaller claims in short launches and at the end) and
+// write the column operand only when the column super tile changes, into the second of
 // two buffers when both fit beside the bins, so the next operand is written
 // while the current one's MMAs run; the row operand is double-buffered by
 // strip.  One CTA per SM (16 epilogue warps, 1 issuer warp, 3 generator
@@ -75,7 +75,7 @@ namespace {
 constexpr int kEpiWarps = 16;                          // epilogue warps
 constexpr int kEpiThreads = kEpiWarps * 32;            // 512: bin columns per bin row
 constexpr int kIssuerWarp = kEpiWarps;                 // warp 16: its lane 0 issues every MMA
-constexpr int kGenWarps = 3;                           // warps 17..19: claim, decode, write operands
+constexpr int kGenWarps = 3;                           // warps 17..20: claim, decode, write operands
 constexpr int kGenThreads = kGenWarps * 32;
 constexpr int kThreads = kEpiThreads + 32 + kGenThreads;
 constexpr int kM = 128;                 // rows per strip (UMMA M)
@@ -108,11 +108,11 @@ constexpr unsigned kGenPollNs = 0;
 constexpr int kColsPerWarp = kN / (kEpiWarps / 4);  // columns of a tile each epilogue warp reads
 constexpr int kLoads = kColsPerWarp / 32;           // 32-column TMEM loads per warp and tile
 static_assert(kEpiWarps % 4 == 0 && kColsPerWarp % 32 == 0, "whole 32-column TMEM loads per warp and tile");
-// Strips a generator claim takes: 4 super tiles, which in the column-by-column
-// tile order share their column operand (written once per claim and column).  The
-// last strips of a launch go in smaller claims, so that the CTAs end together
-// (mma_claims).
-constexpr uint32_t kClaimStrips = 4 * kStrips;
+// Strips a generator claim takes at most: 32 super tiles, which in the
+// column-by-column tile order mostly share their column operand (written once per
+// claim and column).  Short launches take smaller claims, and so do the last strips of
+// any, so that the CTAs end together (mma_claims).
+constexpr uint64_t kMaxClaim = 32 * kStrips;
 // pair-packed epilogue
 constexpr int kPkHalf = kSuper / 2;                 // packed columns of a strip: p holds columns 2p, 2p + 1
 constexpr int kPkTilesPerStrip = kPkHalf / kN;      // 2 MMA tiles of 256 packed columns per strip
@@ -427,7 +427,7 @@ __device__ __noinline__ void pk_fallback(uint32_t P, uint32_t S, float inv_s, in
 }
 
 // Warp roles: warps 0..15 bin (epilogue), warp 16 issues the MMAs (lane 0),
-// warps 17..19 claim strips and write their operands.  Hand-offs go through
+// warps 17..20 claim strips and write their operands.  Hand-offs go through
 // mbarriers only: slot_full/slot_free (a strip's operands written / its MMAs
 // done), full[b] (the MMA result in TMEM buffer b is ready, and for a strip's
 // first tile the strip's StripInfo),
@@ -494,61 +494,96 @@ __global__ void __launch_bounds__(kThreads, 1) mma_hist_kernel(MmaArgs args) {
     uint32_t nclaim = 0;           // claims taken
     unsigned long long t = 0, end = 0;
     bool normal = false;
+    // The current job's fields, read when a strip leaves its tile range, and the decoded
+    // position of its last strip.  A strip's operands are due every ~4,000 cycles, and
+    // the job table is a chain of dependent loads away (its search, too, in a launch of
+    // several jobs): looked up for every strip, the generators, not the epilogue, set
+    // the pace (A = 3999, k = 20 58.2 -> 50.0 ms, 256 instances of k = 16 75.9 -> 58.8 ms;
+    // a fourth generator warp costs more registers than it gains: 57 ms).
+    uint32_t jn = 0xffffffffu;
+    const Job* jp = args.jobs;
+    uint64_t tb = 0, tiles = 0, N = 0, NC = 0, offset = 0, col_tiles = 0, row_tiles = 0;
+    bool rect = false;
+    int L = 0;
+    uint32_t S = 1;
+    int32_t lo = 0;
+    uint64_t A = 0;
+    bool row_prog = false, col_prog = false;  // codewords A * index
+    uint64_t last = ~0ull - 1, sr = 0, sc = 0;  // last decoded tile of the instance, its row tile (super tile) and column tile
     for (;;) {
       if (t >= end) {
         if (gtid == 0) sh->gclaim[nclaim & 1] = atomicAdd(args.counter, 1ull);
         gen_bar();
         const unsigned long long c = sh->gclaim[nclaim & 1], big = args.big_claims;
         ++nclaim;
-        const uint64_t size = c < big ? kClaimStrips : args.small_claim;
-        t = c < big ? c * kClaimStrips : big * kClaimStrips + (c - big) * args.small_claim;
+        const uint64_t size = c < big ? args.big_claim : args.small_claim;
+        t = c < big ? c * args.big_claim : big * args.big_claim + (c - big) * args.small_claim;
         if (t >= args.total_tiles) { normal = true; break; }
         end = t + size < args.total_tiles ? t + size : (uint64_t)args.total_tiles;
       }
       const unsigned long long tt = t++;
-      const uint32_t jn = find_job(args.jobs, args.njobs, tt);
-      if (jn >= args.njobs) {
-        if (gtid == 0) atomicOr(args.status, KSTATUS_BAD_JOB);
-        continue;
+      if (jn == 0xffffffffu || tt < tb || tt - tb >= tiles) {
+        jn = find_job(args.jobs, args.njobs, tt);
+        if (jn >= args.njobs) {
+          if (gtid == 0) atomicOr(args.status, KSTATUS_BAD_JOB);
+          jn = 0xffffffffu;
+          continue;
+        }
+        jp = args.jobs + jn;
+        tb = __ldg(&jp->tile_begin);
+        tiles = __ldg(&jp->tiles);
+        N = __ldg(&jp->rows);
+        NC = __ldg(&jp->cols);
+        offset = __ldg(&jp->tile_offset);
+        col_tiles = __ldg(&jp->col_tiles);
+        row_tiles = (N + kM - 1) / kM;
+        rect = __ldg(&jp->shape) == SHAPE_RECT;
+        S = __ldg(&jp->pk_s);
+        lo = __ldg(&jp->pk_lo);
+        A = __ldg(&jp->A);
+        row_prog = __ldg(&jp->row_kind) == ROW_PROGRESSION;
+        col_prog = __ldg(&jp->col_kind) == COL_PROGRESSION;
+        // every AN codeword of the job lies below A * 2^n (lattice points are indices
+        // < 2^n); an extended Hamming codeword has nbins - 1 bits
+        if (__ldg(&jp->row_kind) == ROW_HAMMING_EXT) {
+          L = (int)__ldg(&jp->nbins) - 1;
+        } else {
+          const uint64_t maxcw = A * ((1ull << __ldg(&jp->n)) - 1ull);
+          L = 64 - __clzll((long long)(maxcw | 1));
+        }
+        L = (L + 3) & ~3;
+        last = ~0ull - 1;
       }
-      const Job* jp = args.jobs + jn;
-      const uint64_t tb = __ldg(&jp->tile_begin), tiles = __ldg(&jp->tiles);
       if (tt < tb || tt - tb >= tiles) {
         if (gtid == 0) atomicOr(args.status, KSTATUS_BAD_JOB);
         continue;
       }
-      const uint64_t A = __ldg(&jp->A), N = __ldg(&jp->rows), NC = __ldg(&jp->cols);
-      const uint64_t lt = tt - tb + __ldg(&jp->tile_offset);
-      const bool rect = __ldg(&jp->shape) == SHAPE_RECT;
-      uint64_t r0, c0, sc;
+      const uint64_t lt = tt - tb + offset;
+      uint64_t r0, c0;
       bool full;
       if (rect) {
         // grid job: 128 rows x 1024 columns per tile, column tile by column tile,
         // so that consecutive tiles share the column operand
         static_assert(kM == 128 && kSuper == 1024, "rect_decode's tile shape");
-        rect_decode(lt, (N + kM - 1) / kM, r0, c0);
-        sc = c0 / kSuper;
+        if (lt == last + 1) {
+          if (++sr == row_tiles) { sr = 0; ++sc; }
+        } else {
+          rect_decode(lt, row_tiles, sr, sc);
+          sr /= kM;
+          sc /= kSuper;
+        }
+        r0 = sr * kM;
+        c0 = sc * kSuper;
         full = (r0 + kM <= N) && (c0 + kSuper <= NC);
       } else {
-        uint64_t sr;
-        tri_decode(lt / kStrips, __ldg(&jp->col_tiles), sr, sc);
+        if (lt != last + 1) tri_decode(lt / kStrips, col_tiles, sr, sc);
+        else if (lt % kStrips == 0 && ++sr > sc) { sr = 0; ++sc; }
         r0 = sr * kSuper + (lt % kStrips) * kM;
         c0 = sc * kSuper;
         full = (r0 + kM <= N) && (c0 + kSuper <= N) && sr != sc;
       }
+      last = lt;
       if (r0 >= N) continue;  // uniform over the group
-      // every AN codeword of the job lies below A * 2^n (lattice points are indices
-      // < 2^n); an extended Hamming codeword has nbins - 1 bits
-      int L;
-      if (__ldg(&jp->row_kind) == ROW_HAMMING_EXT) {
-        L = (int)__ldg(&jp->nbins) - 1;
-      } else {
-        const uint64_t maxcw = A * ((1ull << __ldg(&jp->n)) - 1ull);
-        L = 64 - __clzll((long long)(maxcw | 1));
-      }
-      L = (L + 3) & ~3;
-      const uint32_t S = __ldg(&jp->pk_s);
-      const int32_t lo = __ldg(&jp->pk_lo);
       const uint32_t slot = (uint32_t)(s & 1);
       const bool need_b = jn != bjob || sc != bsc;
       // this slot's row operand may be rewritten once every MMA of strip s-2 is
@@ -578,14 +613,16 @@ __global__ void __launch_bounds__(kThreads, 1) mma_hist_kernel(MmaArgs args) {
 #pragma unroll 1
           for (int cc = gtid; cc < kPkHalf; cc += kGenThreads) {
             const uint64_t j = c0 + 2 * (uint64_t)cc, j2 = j + 1;
-            write_col_pk(bb + (cc / kN) * kBTileBytes, cc % kN, j < ncols ? mma_col_value(jp, j) : 0,
-                         j2 < ncols ? mma_col_value(jp, j2) : 0, L, S, lo);
+            write_col_pk(bb + (cc / kN) * kBTileBytes, cc % kN,
+                         j < ncols ? (col_prog ? A * j : mma_col_value(jp, j)) : 0,
+                         j2 < ncols ? (col_prog ? A * j2 : mma_col_value(jp, j2)) : 0, L, S, lo);
           }
         } else {
 #pragma unroll 1
           for (int cc = gtid; cc < kSuper; cc += kGenThreads) {
             const uint64_t j = c0 + cc;
-            write_operand(bb + (cc / kN) * kBTileBytes, cc % kN, j < ncols ? mma_col_value(jp, j) : 0, L, false);
+            write_operand(bb + (cc / kN) * kBTileBytes, cc % kN,
+                          j < ncols ? (col_prog ? A * j : mma_col_value(jp, j)) : 0, L, false);
           }
         }
         bjob = jn;
@@ -595,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, 1) mma_hist_kernel(MmaArgs args) {
 #pragma unroll 1
       for (int rr = gtid; rr < kM; rr += kGenThreads) {
         const uint64_t i = r0 + rr;
-        const uint64_t x = i < N ? mma_row_value(jp, i) : 0;
+        const uint64_t x = i < N ? (row_prog ? A * i : mma_row_value(jp, i)) : 0;
         if constexpr (kPk) write_row_pk(a, rr, x, L, S);
         else write_operand(a, rr, x, L, true);
       }
@@ -1040,14 +1077,20 @@ uint32_t mma_b_bufs(uint32_t hist_rows) {
   return mma_smem_bytes(hist_rows, 2, false, 0) <= smem_optin() ? 2u : 1u;
 }
 
-// Claims of 32 strips up to the last two super tiles per CTA, then of 8 (one super
-// tile's columns); launches with less work than that go in two claims per CTA.  Against
-// claims of 32 throughout: A = 58659, k = 13 0.205 -> 0.041 ms, k = 15 0.21 -> 0.126 ms,
-// 2-D grid of 33333 x 100001 points 0.84 -> 0.67 ms.
+// Big claims (a quarter of a CTA's share, at most kMaxClaim) up to the last one per CTA,
+// then claims of an eighth of that, at least one super tile; launches of few strips go
+// in two claims per CTA.  The column operand that a claim begins with is written while
+// the pipeline drains: claims of 32 strips throughout, 64, 128, 256 and 512 take 58.8,
+// 57.1, 56.2, 54.1 and 53.3 ms (256 instances of k = 16), 5.13, 4.94, 4.93, 4.91 and
+// 5.60 ms (1-D grid, A = 40001, k = 22, m = 10007; 256 with smaller claims at the end);
+// A = 58659, k = 13 0.205 ms with claims of 32, 0.041 ms.
 void mma_claims(MmaArgs& args, int grid) {
-  const uint64_t tail = (uint64_t)grid * kStrips * 2;
-  args.big_claims = args.total_tiles > tail ? (args.total_tiles - tail) / kClaimStrips : 0;
-  args.small_claim = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kStrips, args.total_tiles / (2 * (uint64_t)grid)));
+  const uint64_t share = args.total_tiles / (uint64_t)grid;
+  args.big_claim = (uint32_t)std::min<uint64_t>(kMaxClaim, std::max<uint64_t>(1, share / 4 / kStrips) * kStrips);
+  const uint64_t tail = (uint64_t)grid * args.big_claim;
+  args.big_claims = args.total_tiles > tail ? (args.total_tiles - tail) / args.big_claim : 0;
+  args.small_claim = (uint32_t)std::max<uint64_t>(
+      1, std::min<uint64_t>(std::max<uint64_t>(kStrips, args.big_claim / 8 / kStrips * kStrips), share / 2));
 }
 
 cudaError_t launch_mma(const MmaArgs& args, int grid, size_t smem, cudaStream_t stream) {

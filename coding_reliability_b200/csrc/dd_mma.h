@@ -20,7 +20,9 @@ struct MmaArgs {
   uint32_t packed;           // 1: pair-packed epilogue (two distances per MMA column, joint-bin table)
   uint32_t pk_cells;         // pair-packed: joint-table cells of this launch (S x window rows of its jobs)
   uint32_t small_claim;      // strips of a claim after the first big_claims (mma_claims)
-  unsigned long long big_claims;
+  unsigned long long big_claims;  // ... of big_claim strips each
+  uint32_t big_claim;
+  uint32_t pad;
 };
 
 // True if the job can run on the MMA path: all pairs of a codeword progression or
