@@ -18,11 +18,12 @@
 // With b = k - bits(A) that is about b A^2 / 2 small steps instead of 4^k / 2 pairs
 // (A = 58659, k = 22: 1.0e10 against 8.8e12), all in integers.
 //
-// Measured on B200 against the tcgen05 kernel: A = 62307, k = 22: 70 ms against 965 ms,
-// k = 20: 20.6 against 63.5 ms; A = 867, k = 21: 0.32 against 231 ms, k = 16: 0.066
-// against 0.37 ms.  Bound by instruction issue and its latencies at 12 warps an SM, the
-// ALU and shared-memory pipes each a bit over half busy; DRAM carries nothing up to 4
-// window bits and the staged histograms (24 bytes a residue pair, once each way) above.
+// Measured on B200 against the tcgen05 kernel: A = 62307, k = 22: 50 ms against 941 ms
+// (965 ms before its generators were mended), k = 20: 20.6 against 59.5 ms; A = 867,
+// k = 21: 0.31 against 193 ms, k = 16: 0.055 against 0.29 ms.  Bound by instruction
+// issue and its latencies at 12 to 18 warps an SM, the ALU and shared-memory pipes each
+// a bit over half busy; DRAM carries nothing up to 4 window bits and the staged
+// histograms (24 bytes a residue pair, once each way) above.
 //
 // A histogram lives in registers, packed: four 8-bit counts per word while the
 // counts stay within 4^4, two 16-bit counts per word up to 4^8.  The count 4^4 (4^8)
@@ -33,11 +34,11 @@
 // Columns v' lie across threads, rows v are time, descending.  A step needs the
 // neighbour column v'+s of the same row and both of row v+s, which are kept as
 // Y = H(v, v'+s) + z H(v, v') in a ring of s rows.  Windows of up to 4 bits run in one
-// kernel from the popcounts to the bins (carry_quad_kernel).  Longer ones run their
-// largest steps first, in a kernel whose rows and columns are 16 residues apart, and
-// stage the 8-bit histograms in memory; there a thread holds one column in words of
-// every second (every fourth) bin, so that multiplying by z renames words and shifts
-// only one word in two (in four).
+// kernel from the popcounts to the bins (carry_quad_kernel).  For longer ones the same
+// four steps run first, in a kernel whose rows and columns are 2^(b-4) residues apart,
+// and stage their 8-bit histograms in memory (carry_stage_kernel); the remaining small
+// steps hold one column a thread in words of every fourth bin, so that multiplying by
+// z renames words and shifts only one in four (carry_fold_kernel).
 #include <algorithm>
 
 #include "dd_carry.cuh"
@@ -45,33 +46,32 @@
 namespace dd {
 namespace {
 
-constexpr int kStageThreads = 512;  // staging kernel: 4 column residues mod 16 x 128 columns 16 apart
-constexpr int kStageCols = kStageThreads / 4;
-constexpr int kUnit = 16;           // residues between the staging kernel's rows and columns
-constexpr int kFoldThreads = 192;   // folding kernel reading staged histograms
 constexpr size_t kStageCells = 32u << 20;  // staged histograms of one round of blocks (768 MB)
-constexpr int kLead = 8;            // rows above a step's own that its first level reads
-constexpr int kAhead = 3;           // rows loaded ahead
-constexpr int kSlots = kLead + 1 + kAhead;
+constexpr uint32_t kStageSide = 3584;      // residues per side of a staged block, with the windows' overhang
+constexpr int kAhead = 3;           // rows the folding kernels load ahead
+constexpr int kFoldThreads = 192;
+constexpr int kQuadWarps = 6;       // warps of a CTA where each works alone
 
 // One block of residue pairs of one job: [row0, row0+rows) x [col0, col0+cols).
 struct CarryEntry {
   uint32_t A, psi, qinv, nq, slices, wide;
   uint32_t row0, rows, col0, cols;
-  uint32_t srows, scols;            // staged rows and columns (from row0, col0)
+  uint32_t unit;                    // residues between the staging kernel's rows and columns: 2^(b-4)
+  uint32_t srows, scols, pitch;     // staged rows and columns (from row0, col0); columns of one residue mod unit
   uint32_t seg, segs, strips;       // folding: rows per CTA, CTAs down and across
   uint32_t stage_seg, stage_segs, stage_strips;
   uint32_t fold_end, stage_end;     // CTAs of the launch up to and including this entry
-  uint4* st16;                      // staged histograms: words e0 e1 e2 o0 ...
+  // staged histograms, row by row, a row's columns by their residue mod unit:
+  uint4* st16;                      // words e0 e1 e2 o0 ...
   uint2* st8;                       // ... and o1 o2
   unsigned long long* acc;          // [0, kMaxBins): residue pairs v < v'; then v = v'
 };
 
 // Entries of one launch, in its parameters (short instances share a launch, and so
-// fill the GPU together; 32 entries stay below the 4 KB every launch can pass).  64
+// fill the GPU together; 31 entries stay below the 4 KB every launch can pass).  64
 // instances of 8-bit A, k = 14: 0.33 ms, 2.0 ms launched one by one; 256 at k = 16:
 // 2.5 ms, popc kernel 123, tcgen05 81.
-constexpr uint32_t kEntries = 32;
+constexpr uint32_t kEntries = 31;
 struct CarryBatch {
   uint32_t n;
   CarryEntry e[kEntries];
@@ -92,81 +92,6 @@ __device__ __forceinline__ Hist<kLevel> level(const Hist<kLevel - 1>& own, uint8
   return r;
 }
 
-// Shared bytes of the exchange rows: one per level after the first; with a single
-// one, two that take turns (a row's only barrier then separates them).
-template <int kBefore, int kLevels>
-__host__ __device__ constexpr int exchange_bytes(int cols) {
-  int n = 0;
-  for (int i = 1; i < kLevels; ++i) n += (kBefore + i <= 4 ? 24 : 48) * cols;
-  return kLevels == 2 ? 2 * n : n;
-}
-
-// ---------------------------------------------------------------- staging kernel
-// The kLevels largest steps (s = 16 * 2^(kLevels-1) .. 16) for a block of residue
-// pairs.  CTA: rows v = row0 + rho + 16 w for one rho and a run of w; columns v' =
-// col0 + sigma + 16 w' for four neighbouring sigma (so that the stores of a warp
-// fill sectors) and kStageCols consecutive w', of which the last 2^kLevels - 1
-// only feed their neighbours.
-template <int kLevels>
-__global__ void __launch_bounds__(kStageThreads) carry_stage_kernel(const __grid_constant__ CarryBatch batch) {
-  constexpr int kFirst = 1 << (kLevels - 1);
-  constexpr int kWarm = kFirst - 1;
-  constexpr int kUseful = kStageCols - ((1 << kLevels) - 1);
-  constexpr int kUnroll = kLevels >= 3 ? kFirst / 2 : 1;
-  constexpr int kCols = kStageThreads + 4 * kFirst;
-  __shared__ __align__(16) uint8_t ex[exchange_bytes<0, kLevels>(kCols) + 16];
-
-  uint32_t idx = 0;
-  while (blockIdx.x >= batch.e[idx].stage_end) ++idx;
-  const CarryEntry& a = batch.e[idx];
-  const uint32_t cta = blockIdx.x - (idx ? batch.e[idx - 1].stage_end : 0);
-  const uint32_t cx = cta % a.stage_strips, cy = cta / a.stage_strips;
-
-  const int tid = threadIdx.x, sub = tid & 3, wi = tid >> 2;
-  const uint32_t rho = cy % kUnit, seg = cy / kUnit;
-  const uint32_t sigma = (cx & 3) * 4 + sub, w0 = (cx >> 2) * kUseful;
-  const uint32_t wrows = (a.srows - rho + kUnit - 1) / kUnit;  // rows of this rho in the block
-  const uint32_t wr0 = seg * a.stage_seg;
-  if (wr0 >= wrows) return;
-  const uint32_t wr1 = min(wrows, wr0 + a.stage_seg);
-  // residue pairs v' < v are their mirror images; a final row reads staged rows up to 15 above it
-  {
-    const uint32_t vtop = a.col0 + (cx & 3) * 4 + 3 + kUnit * (w0 + kUseful - 1);
-    if (vtop + 15 < a.row0 + rho + kUnit * wr0) return;
-  }
-  const uint32_t col = sigma + kUnit * (w0 + wi), vc = a.col0 + col;
-  const bool store = wi < kUseful && col < a.scols;
-  const uint32_t ca = mul_mod(a.psi, vc, a.A), cb = mul_mod(a.psi, vc + kUnit * kFirst, a.A);
-  const int total = ((int)(wr1 - wr0) + kWarm + kUnroll - 1) / kUnroll * kUnroll;
-  uint32_t w = wr0 + total - 1;  // descending
-  const uint32_t step = mul_mod(a.psi, kUnit, a.A);
-  uint32_t ra = mul_mod(a.psi, a.row0 + rho + kUnit * w, a.A);
-  uint32_t rb = mul_mod(a.psi, a.row0 + rho + kUnit * (w + kFirst), a.A);
-
-  H8 y4[4], y2[2], y1;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) zero(y4[i]);
-  zero(y2[0]); zero(y2[1]); zero(y1);
-  for (int it = 0; it < total; it += kUnroll) {
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u, --w) {
-      H8 h = first_level(ra, rb, ca, cb);
-      ra = sub_mod(ra, step, a.A);
-      rb = sub_mod(rb, step, a.A);
-      uint8_t* row = ex;
-      if constexpr (kLevels >= 4) { h = level<2>(h, row, tid, 4 * 4, y4[u & 3]); row += 24 * kCols; }
-      if constexpr (kLevels >= 3) { h = level<2>(h, row, tid, 4 * 2, y2[u & 1]); row += 24 * kCols; }
-      if constexpr (kLevels == 2) row += ((it + u) & 1) * 24 * kCols;
-      if constexpr (kLevels >= 2) h = level<2>(h, row, tid, 4, y1);
-      if (store && w < wr1) {
-        const size_t at = (size_t)(rho + kUnit * w) * a.scols + col;
-        a.st16[at] = make_uint4(h.e[0], h.e[1], h.e[2], h.o[0]);
-        a.st8[at] = make_uint2(h.o[1], h.o[2]);
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------- folding kernel
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -180,30 +105,64 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int kPending>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-// Shared memory of the folding kernel: tables (U and D, twice for wide products),
+// One column's bins to the cells from at (and at2) on, in all words alike: most hold
+// counts, and a test per word costs more than the empty additions.
+template <int kBin>
+__device__ __forceinline__ void fold_word(uint32_t w, uint32_t at, uint32_t at2, bool twice) {
+  const uint32_t lo = w & 0xFFFFu, hi = w >> 16;
+  red_add<kBin * 128>(at, lo);
+  red_add<(kBin + 4) * 128>(at, hi);
+  if (twice) {
+    red_add<kBin * 128>(at2, lo);
+    red_add<(kBin + 4) * 128>(at2, hi);
+  }
+}
+template <bool kTwice>
+__device__ __forceinline__ void fold_column(const H16& g, uint32_t at, uint32_t at2) {
+  fold_word<0>(g.p0[0], at, at2, kTwice); fold_word<1>(g.p1[0], at, at2, kTwice);
+  fold_word<2>(g.p2[0], at, at2, kTwice); fold_word<3>(g.p3[0], at, at2, kTwice);
+  fold_word<8>(g.p0[1], at, at2, kTwice); fold_word<9>(g.p1[1], at, at2, kTwice);
+  fold_word<10>(g.p2[1], at, at2, kTwice); fold_word<11>(g.p3[1], at, at2, kTwice);
+  fold_word<16>(g.p0[2], at, at2, kTwice); fold_word<17>(g.p1[2], at, at2, kTwice);
+  fold_word<18>(g.p2[2], at, at2, kTwice); fold_word<19>(g.p3[2], at, at2, kTwice);
+  red_add<24 * 128>(at, g.p0[3]);  // bin 28 does not occur
+  if (kTwice) red_add<24 * 128>(at2, g.p0[3]);
+}
+
+// The first level of the last kLevels reads its own row only, with a ring in registers;
+// 8 rows of 16-bit histograms do not fit there, so kLevels = 4 reads row v + 8, too.
+template <int kLevels>
+__host__ __device__ constexpr int fold_lead() { return kLevels == 4 ? 8 : 0; }
+template <int kLevels>
+__host__ __device__ constexpr int fold_slots() { return fold_lead<kLevels>() + 1 + kAhead; }
+// Exchange rows, one per level after the first; a single one has two that take turns
+// (a row's only barrier then separates them).
+template <int kLevels>
+__host__ __device__ constexpr int fold_exchanges() { return kLevels == 2 ? 2 : kLevels - 1; }
+
+// Shared memory of the folding kernel: tables (U, D and a spare; U and D twice for wide products),
 // exchange rows, the ring of staged rows, and the q-distance counts of each thread (many).
-template <int kBefore, int kLevels>
+template <int kLevels>
 constexpr size_t fold_smem(bool many) {
   constexpr int cols = kFoldThreads + (1 << (kLevels - 1));
-  return (size_t)kTabBytes * (many ? 4 : 2) + exchange_bytes<kBefore, kLevels>(cols) + (size_t)kSlots * cols * 24 +
+  return (size_t)kTabBytes * (many ? 4 : 3) + (size_t)(48 * fold_exchanges<kLevels>() + 24 * fold_slots<kLevels>()) * cols +
          (many ? (size_t)(16 + 1) * kFoldThreads * 4 : 0);
 }
 
-// The last four steps (s = 8 .. 1) and the sum over q, q'.  kBefore: levels already in
-// the staged input.  CTA: a
-// strip of columns (one per thread, the last 2^kLevels - 1 only feed their
-// neighbours) x a segment of rows.
-template <int kBefore, int kLevels, bool kMany>
-__global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __grid_constant__ CarryBatch batch) {
+// The last kLevels steps (s = 2^(kLevels-1) .. 1), from the staged 8-bit histograms to
+// 16-bit ones, and the sum over q, q'.  CTA: a strip of columns (one per thread, the
+// last 2^kLevels - 1 only feed their neighbours) x a segment of rows.  Measured and
+// dropped: a warp alone with shuffles and two 16-bit counts folded as one word (k = 22
+// 58.7 against 52.9 ms: fewer warps for its tables), CTAs of 256 threads (57 ms).
+template <int kLevels, bool kMany>
+__global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold_kernel(const __grid_constant__ CarryBatch batch) {
   constexpr int kThreads = kFoldThreads;
   constexpr int kFirst = 1 << (kLevels - 1);
-  constexpr int kWarm = kFirst - 1;
+  constexpr int kLead = fold_lead<kLevels>(), kSlots = fold_slots<kLevels>();
+  constexpr int kWarm = (kLead ? kFirst : 2 * kFirst) - 1;
   constexpr int kUseful = kThreads - ((1 << kLevels) - 1);
-  static_assert(kLevels == 4 && kFirst == kLead, "the staged input leaves four levels");
-  constexpr int kUnroll = kFirst / 2;
+  constexpr int kUnroll = kLevels == 4 ? 4 : kFirst;  // the longest ring in registers
   constexpr int kCols = kThreads + kFirst;
-  constexpr int kL1 = kBefore + 1;
-  constexpr int kLast = kBefore + kLevels;
   extern __shared__ __align__(16) uint8_t smem[];
 
   uint32_t idx = 0;
@@ -220,8 +179,8 @@ __global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __gri
 
   // shared memory
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);  // U, D (and their high parts)
-  uint8_t* ex = smem + kTabBytes * (kMany ? 4 : 2);
-  uint4* in16 = reinterpret_cast<uint4*>(ex + exchange_bytes<kBefore, kLevels>(kCols));
+  uint8_t* ex = smem + kTabBytes * (kMany ? 4 : 3);
+  uint4* in16 = reinterpret_cast<uint4*>(ex + 48 * fold_exchanges<kLevels>() * kCols);
   uint2* in8 = reinterpret_cast<uint2*>(in16 + kSlots * kCols);
   uint32_t* qd = reinterpret_cast<uint32_t*>(in8 + kSlots * kCols);
   for (int i = tid; i < kTabBytes * (kMany ? 4 : 2) / 4; i += kThreads) tab[i] = 0;
@@ -235,23 +194,23 @@ __global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __gri
   uint32_t r = r0 + total - 1;  // descending, from row0
   uint32_t qr = mul_mod(a.qinv, a.row0 + r, a.A);
   const uint32_t tab_u = (uint32_t)__cvta_generic_to_shared(tab) + lane * 4u;
+  const bool two = qc + a.A < a.nq, second = __any_sync(0xffffffffu, two);  // a second q: here, in this warp
+  const uint32_t spare = tab_u + 2 * kTabBytes;  // few q: the third table is not read
 
   // input: staged rows through a ring of kSlots rows
   int slot = 0;  // ring slot of load number it (row r + kLead of that step)
-  const uint32_t scol = min(col, a.scols - 1);
+  const uint32_t scol = min(col, a.scols - 1), cell = scol % a.unit * a.pitch + scol / a.unit;
   auto load = [&](int sl, uint32_t row) {
-    const size_t at = (size_t)min(row, a.srows - 1) * a.scols;
-    copy_async16(in16 + sl * kCols + tid, a.st16 + at + scol);
-    copy_async8(in8 + sl * kCols + tid, a.st8 + at + scol);
+    const size_t at = (size_t)min(row, a.srows - 1) * (a.unit * a.pitch) + cell;
+    copy_async16(in16 + sl * kCols + tid, a.st16 + at);
+    copy_async8(in8 + sl * kCols + tid, a.st8 + at);
     copy_commit();
   };
   for (int l = 0; l < kLead + kAhead; ++l) load(l, r + kLead - l);
   copy_wait<kAhead - 1>();
   __syncthreads();
 
-  Hist<kLast - 2> y4[4];
-  Hist<kLast - 1> y2[2];
-  Hist<kLast> y1;
+  H16 y4[4], y2[2], y1;  // the rings of the steps 4, 2, 1
 #pragma unroll
   for (int i = 0; i < 4; ++i) zero(y4[i]);
   zero(y2[0]); zero(y2[1]); zero(y1);
@@ -263,11 +222,18 @@ __global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __gri
       auto fetch = [&](int sl, int c) {
         const uint4 x = in16[sl * kCols + c];
         const uint2 w = in8[sl * kCols + c];
-        return as_level<kL1>(H8{{x.x, x.y, x.z}, {x.w, w.x, w.y}});
+        return widen(H8{{x.x, x.y, x.z}, {x.w, w.x, w.y}});
       };
       const int lo = slot, hi = slot + kLead < kSlots ? slot + kLead : slot + kLead - kSlots;
-      const Hist<kL1> h1 =
-          add_z(add(fetch(hi, tid), fetch(lo, tid + kFirst)), add(fetch(hi, tid + kFirst), fetch(lo, tid)));
+      H16 g;
+      if constexpr (kLevels == 4) {
+        g = add_z(add(fetch(hi, tid), fetch(lo, tid + kFirst)), add(fetch(hi, tid + kFirst), fetch(lo, tid)));
+      } else {
+        const H16 own = fetch(hi, tid), nb = fetch(hi, tid + kFirst);
+        H16& y = kLevels == 3 ? y4[u & 3] : kLevels == 2 ? y2[u & 1] : y1;
+        g = add(add_z(own, nb), y);
+        y = add_z(nb, own);
+      }
       int nx = slot + kLead + kAhead;
       if (nx >= kSlots) nx -= kSlots;
       // row r + kLead - (kLead + kAhead); rows below the block's first are never used
@@ -276,24 +242,26 @@ __global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __gri
       copy_wait<kAhead - 1>();
       // remaining levels
       uint8_t* row = ex;
-      const Hist<kLast - 2> h2 = level<kLast - 2>(h1, row, tid, 4, y4[u & 3]);
-      row += slot_bytes<Hist<kL1>>() * kCols;
-      const Hist<kLast - 1> h3 = level<kLast - 1>(h2, row, tid, 2, y2[u & 1]);
-      row += slot_bytes<Hist<kLast - 2>>() * kCols;
-      const Hist<kLast> g = level<kLast>(h3, row, tid, 1, y1);
+      if constexpr (kLevels == 4) { g = level<6>(g, row, tid, 4, y4[u & 3]); row += 48 * kCols; }
+      if constexpr (kLevels >= 3) { g = level<6>(g, row, tid, 2, y2[u & 1]); row += 48 * kCols; }
+      if constexpr (kLevels == 2) row += ((it + u) & 1) * 48 * kCols;
+      if constexpr (kLevels >= 2) g = level<6>(g, row, tid, 1, y1);
+      else __syncthreads();  // the row loaded ahead is complete for the neighbours
       // fold: every q of row residue v with every q' of column residue v'
       const uint32_t v = a.row0 + r;
-      if (mine && r < r1 && vc >= v) {
-        const uint32_t at = tab_u + (vc == v ? kTabBytes : 0);
-        if constexpr (!kMany) {
-          const bool c2 = qc + a.A < a.nq;
-          add_hist<kOne>(at + (__popc(qr ^ qc) << 7), 1, g);
-          if (c2) add_hist<kOne>(at + (__popc(qr ^ (qc + a.A)) << 7), 1, g);
-          if (qr + a.A < a.nq) {
-            add_hist<kOne>(at + (__popc((qr + a.A) ^ qc) << 7), 1, g);
-            if (c2) add_hist<kOne>(at + (__popc((qr + a.A) ^ (qc + a.A)) << 7), 1, g);
+      if constexpr (!kMany) {
+        if (r < r1)
+#pragma unroll 1
+          for (uint32_t q = qr; q < a.nq; q += a.A) {
+            // columns that do not count here go to a spare column of the table
+            const uint32_t to = !mine || vc < v ? spare : vc == v ? tab_u + kTabBytes : tab_u;
+            const uint32_t at = to + (__popc(q ^ qc) << 7);
+            if (second) fold_column<true>(g, at, (two ? to : spare) + (__popc(q ^ (qc + a.A)) << 7));
+            else fold_column<false>(g, at, at);
           }
-        } else {
+      } else if (mine && r < r1 && vc >= v) {
+        const uint32_t at = tab_u + (vc == v ? kTabBytes : 0);
+        {
           volatile uint32_t* f = qd + tid;
           const uint32_t fa = (uint32_t)__cvta_generic_to_shared(qd + tid);
           for (uint32_t q = qr + slice * a.A; q < a.nq; q += a.slices * a.A)
@@ -327,7 +295,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __gri
   }
 }
 
-// ---------------------------------------------------------------- windows of up to 4 bits
+// ---------------------------------------------------------------- four steps in a warp
 // Everything in one warp: a lane holds four neighbouring columns, one byte each, in
 // one word per bin, so that z renames words, a step costs two additions per word for
 // four residue pairs, and the neighbour columns come by shuffles (no barrier, no
@@ -338,7 +306,6 @@ __global__ void __launch_bounds__(kFoldThreads, 2) carry_fold_kernel(const __gri
 // instructions per 32 residue pairs, neighbours through shared memory and a barrier a
 // step), 20.6 ms (about 200); with the first ring in registers, too, 29 ms (254
 // registers, 8 warps an SM, an unrolled loop past the instruction cache).
-constexpr int kQuadWarps = 6;
 constexpr int kCells = 37;                 // q distance <= 16, bins 0, 2, .. 20
 constexpr int kDiscard = 21;               // cells for columns that do not count
 constexpr int kPackedRows = 16;            // x 4 columns x 4 q pairs x 255 stays below 2^16
@@ -431,6 +398,107 @@ __device__ __forceinline__ void fold_quad(const Quad<kN>& g, const uint32_t (&at
     for (int i = 0; i < 4; ++i) {
       red_at(at[i] + d * 128, v[i]);
       if constexpr (kTwice) red_at(at2[i] + d * 128, v[i]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- windows of 5 to 8 bits
+// Their four largest steps, in the same way, for a block of residue pairs whose rows
+// and columns are `unit` = 2^(b-4) apart: work of a warp is the rows v = row0 + rho +
+// unit w, for one rho and a run of w, and the columns col0 + sigma + unit w' for one
+// sigma and 128 consecutive w'.  The finished 8-bit histograms are stored column by
+// column (a 4 x 4 byte transpose per four bins), 32 bytes a store.  159 warp
+// instructions per 32 residue pairs at 62 % issue, the ALU pipe 70 % busy (A = 7151,
+// k = 19).  Staging b - 4 levels and folding four took 70 ms where four staged and b - 4
+// folded ones take 50 ms (A = 62307, k = 22).
+constexpr int kStageRing = 4 * 5 * 16 * 32;  // a warp's first ring
+constexpr int kStageBytes = kQuadWarps * kStageRing;
+
+__device__ __forceinline__ void transpose_bytes(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t (&col)[4]) {
+  const uint32_t a = __byte_perm(w0, w1, 0x5140), b = __byte_perm(w2, w3, 0x5140);
+  const uint32_t c = __byte_perm(w0, w1, 0x7362), d = __byte_perm(w2, w3, 0x7362);
+  col[0] = __byte_perm(a, b, 0x5410);
+  col[1] = __byte_perm(a, b, 0x7632);
+  col[2] = __byte_perm(c, d, 0x5410);
+  col[3] = __byte_perm(c, d, 0x7632);
+}
+__device__ __forceinline__ void store32(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f,
+                                        uint32_t g, uint32_t h) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d),
+               "r"(e), "r"(f), "r"(g), "r"(h)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kQuadWarps * 32, 2) carry_stage_kernel(const __grid_constant__ CarryBatch batch) {
+  constexpr uint32_t kUseful = quad_useful<4>();
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint32_t idx = 0;
+  while (blockIdx.x >= batch.e[idx].stage_end) ++idx;
+  const CarryEntry& a = batch.e[idx];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t work = (blockIdx.x - (idx ? batch.e[idx - 1].stage_end : 0)) * kQuadWarps + warp;
+  const uint32_t w0 = work % a.stage_strips * kUseful;
+  work /= a.stage_strips;
+  const uint32_t sigma = work % a.unit;
+  work /= a.unit;
+  const uint32_t rho = work % a.unit, seg = work / a.unit;
+  if (seg >= a.stage_segs) return;
+  const uint32_t wrows = (a.srows - rho + a.unit - 1) / a.unit;  // rows of this rho in the block
+  const uint32_t wr0 = seg * a.stage_seg, wr1 = min(wrows, wr0 + a.stage_seg);
+  // residue pairs v' < v are their mirror images; a finished window reads unit - 1 past its own
+  if (wr0 >= wr1 || a.col0 + sigma + a.unit * (w0 + kUseful) < a.row0 + rho + a.unit * wr0) return;
+  uint4* ring = reinterpret_cast<uint4*>(smem + warp * kStageRing) + lane;
+
+  const uint32_t w4 = w0 + 4u * lane;
+  uint32_t c[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] = mul_mod(a.psi, a.col0 + sigma + a.unit * (w4 + i), a.A);
+  const bool store = 4u * lane < kUseful && w4 < a.pitch;
+  const int total = ((int)(wr1 - wr0) + 7 + 1) / 2 * 2;
+  uint32_t w = wr0 + total - 1;  // descending
+  const uint32_t step = mul_mod(a.psi, a.unit, a.A);
+  uint32_t ra = mul_mod(a.psi, a.row0 + rho + a.unit * w, a.A), rb = mul_mod(a.psi, a.row0 + rho + a.unit * (w + 8), a.A);
+  size_t at = ((size_t)(rho + a.unit * w) * a.unit + sigma) * a.pitch + w4;
+  const size_t row_cells = (size_t)a.unit * a.unit * a.pitch;
+
+  Quad<20> y2[2];
+  Quad<21> y1;
+#pragma unroll
+  for (int d = 0; d < 20; ++d) y2[0].w[d] = y2[1].w[d] = 0;
+#pragma unroll
+  for (int d = 0; d < 21; ++d) y1.w[d] = 0;
+  for (int it = 0; it < total; it += 2) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u, --w, at -= row_cells) {
+      const uint32_t ha = distances(ra, c), hd = distances(rb, c);
+      Quad<18> h1;
+#pragma unroll
+      for (int d = 0; d < 18; ++d) h1.w[d] = 0;
+      count_bytes<0>(ha, h1);
+      count_bytes<1>(columns_at<8>(ha), h1);
+      count_bytes<1>(hd, h1);
+      count_bytes<0>(columns_at<8>(hd), h1);
+      ra = sub_mod(ra, step, a.A);
+      rb = sub_mod(rb, step, a.A);
+      uint4* row = ring + ((it + u) & 3) * (5 * 32);
+      Quad<19> y4;
+      load_quad(row, y4);
+      const Quad<19> h2 = quad_level<4>(h1, y4);
+      store_quad(row, y4);
+      const Quad<20> h3 = quad_level<2>(h2, y2[u & 1]);
+      const Quad<21> g = quad_level<1>(h3, y1);
+      if (store && w < wr1) {
+        uint32_t e[3][4], o[3][4];
+        transpose_bytes(g.w[0], g.w[2], g.w[4], g.w[6], e[0]);
+        transpose_bytes(g.w[1], g.w[3], g.w[5], g.w[7], o[0]);
+        transpose_bytes(g.w[8], g.w[10], g.w[12], g.w[14], e[1]);
+        transpose_bytes(g.w[9], g.w[11], g.w[13], g.w[15], o[1]);
+        transpose_bytes(g.w[16], g.w[18], g.w[20], 0u, e[2]);
+        transpose_bytes(g.w[17], g.w[19], 0u, 0u, o[2]);
+        store32(a.st16 + at, e[0][0], e[1][0], e[2][0], o[0][0], e[0][1], e[1][1], e[2][1], o[0][1]);
+        store32(a.st16 + at + 2, e[0][2], e[1][2], e[2][2], o[0][2], e[0][3], e[1][3], e[2][3], o[0][3]);
+        store32(a.st8 + at, o[1][0], o[2][0], o[1][1], o[2][1], o[1][2], o[2][2], o[1][3], o[2][3]);
+      }
     }
   }
 }
@@ -582,22 +650,17 @@ __global__ void carry_finish_kernel(const Job* jobs, const unsigned long long* a
   j.bins[d] = t[d] + (t[kMaxBins + d] - (d == 0 ? 1ull << j.n : 0ull)) / 2;
 }
 
-template <int kBefore, int kLevels, bool kMany>
-cudaError_t run_fold(const CarryBatch& b, cudaStream_t stream) {
-  constexpr size_t smem = fold_smem<kBefore, kLevels>(kMany);
-  auto fn = carry_fold_kernel<kBefore, kLevels, kMany>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int kLevels, bool kMany>
+cudaError_t run_staged(const CarryBatch& b, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(carry_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
   if (e != cudaSuccess) return e;
+  carry_stage_kernel<<<b.e[b.n - 1].stage_end, kQuadWarps * 32, kStageBytes, stream>>>(b);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  constexpr size_t smem = fold_smem<kLevels>(kMany);
+  auto fn = carry_fold_kernel<kLevels, kMany>;
+  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
   fn<<<b.e[b.n - 1].fold_end, kFoldThreads, smem, stream>>>(b);
   return cudaGetLastError();
-}
-
-template <int kBefore, int kLevels>
-cudaError_t run_batch(const CarryBatch& b, bool many, cudaStream_t stream) {
-  carry_stage_kernel<kBefore><<<b.e[b.n - 1].stage_end, kStageThreads, 0, stream>>>(b);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return many ? run_fold<kBefore, kLevels, true>(b, stream) : run_fold<kBefore, kLevels, false>(b, stream);
 }
 
 template <int kLevels>
@@ -609,17 +672,17 @@ cudaError_t run_quad(const CarryBatch& b, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-// With up to 4 window bits 2^s < 2 A, so a residue has at most two q (many is false).
+// With fewer than 8 window bits 2^s < 2 A, so a residue has at most two q (many is false).
 cudaError_t run_batch(const CarryBatch& b, uint32_t levels, bool many, cudaStream_t stream) {
   switch (levels) {
     case 1: return run_quad<1>(b, stream);
     case 2: return run_quad<2>(b, stream);
     case 3: return run_quad<3>(b, stream);
     case 4: return run_quad<4>(b, stream);
-    case 5: return run_batch<1, 4>(b, many, stream);
-    case 6: return run_batch<2, 4>(b, many, stream);
-    case 7: return run_batch<3, 4>(b, many, stream);
-    default: return run_batch<4, 4>(b, many, stream);
+    case 5: return run_staged<1, false>(b, stream);
+    case 6: return run_staged<2, false>(b, stream);
+    case 7: return run_staged<3, false>(b, stream);
+    default: return many ? run_staged<4, true>(b, stream) : run_staged<4, false>(b, stream);
   }
 }
 
@@ -641,6 +704,16 @@ bool carry_wins(const Job& j) {
   return j.n >= a + 4 && j.n >= 14;
 }
 
+// Staged columns of one residue mod unit (a lane stores four), and the histograms of a
+// block of finished rows x cols.
+static uint32_t staged_pitch(const CarryPlan& p, uint32_t cols) {
+  const uint32_t unit = 1u << p.staged;
+  return ((cols + unit - 1 + unit - 1) / unit + 3) / 4 * 4;
+}
+static size_t staged_cells(const CarryPlan& p, uint32_t rows, uint32_t cols) {
+  return (size_t)(rows + (1u << p.staged) - 1) * (staged_pitch(p, cols) << p.staged);
+}
+
 void carry_plan(const Job& j, CarryPlan& p) {
   p = CarryPlan();
   p.A = odd_part(j.A);
@@ -653,9 +726,8 @@ void carry_plan(const Job& j, CarryPlan& p) {
   p.many = (1ull << p.s) > 2ull * p.A;
   p.side = p.A;
   if (p.staged) {
-    const uint32_t useful = kStageCols - ((1u << p.staged) - 1);
-    p.side = std::min(p.A, kUnit * useful * 2 - 15);
-    p.cells = (size_t)(p.side + 15) * (p.side + 15);
+    p.side = std::min(p.A, kStageSide - ((1u << p.staged) - 1));
+    p.cells = staged_cells(p, p.side, p.side);
   }
 }
 
@@ -707,7 +779,7 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
           e.rows = std::min(p.side, p.A - r0);
           e.cols = std::min(p.side, p.A - c0);
           e.acc = acc + i * 2 * kMaxBins;
-          const uint32_t useful = p.staged ? kFoldThreads - 15 : (128 - ((1u << p.b) - 1)) / 4 * 4;
+          const uint32_t useful = p.staged ? kFoldThreads - ((1u << p.staged) - 1) : (128 - ((1u << p.b) - 1)) / 4 * 4;
           e.strips = (e.cols + useful - 1) / useful;
           // rows per CTA: long runs amortise the rows a segment computes twice; short
           // ones where the launch would leave SMs without a CTA
@@ -727,7 +799,7 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
             const uint64_t sum = (uint64_t)e.seg * (kFoldThreads / 32) * ((per + e.slices - 1) / e.slices) * per << (2 * p.b);
             e.wide = per > 4096 || sum > 0xFFFFFFFFull;
           }
-          const size_t need = p.staged ? (size_t)(e.rows + 15) * (e.cols + 15) : 0;
+          const size_t need = p.staged ? staged_cells(p, e.rows, e.cols) : 0;
           if (b.n == kEntries || (b.n && used + need > cells)) {
             const cudaError_t err = run_batch(b, levels, many != 0, stream);
             if (err != cudaSuccess) return err;
@@ -735,21 +807,26 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
             used = 0;
           }
           if (p.staged) {
-            e.srows = e.rows + 15;
-            e.scols = e.cols + 15;
+            e.unit = 1u << p.staged;
+            e.srows = e.rows + e.unit - 1;
+            e.scols = e.cols + e.unit - 1;
+            e.pitch = staged_pitch(p, e.cols);
             e.st16 = st16 + used;
             e.st8 = st8 + used;
             used += need;
-            const uint32_t su = kStageCols - ((1u << p.staged) - 1);
-            const uint32_t w = (e.scols + kUnit - 1) / kUnit, wr = (e.srows + kUnit - 1) / kUnit;
-            e.stage_strips = 4 * ((w + su - 1) / su);
-            e.stage_segs = (wr + 63) / 64;
-            e.stage_seg = (wr + e.stage_segs - 1) / e.stage_segs;
+            const uint32_t wr = (e.srows + e.unit - 1) / e.unit, su = quad_useful<4>();
+            e.stage_strips = (e.pitch + su - 1) / su;
+            e.stage_seg = 128;
+            while (e.stage_seg > 16 &&
+                   (uint64_t)e.stage_strips * e.unit * e.unit * ((wr + e.stage_seg - 1) / e.stage_seg) < want * 3 / 2)
+              e.stage_seg /= 2;
+            e.stage_segs = (wr + e.stage_seg - 1) / e.stage_seg;
           }
           const CarryEntry* before = b.n ? &b.e[b.n - 1] : nullptr;
           const uint32_t ctas = e.strips * e.segs * e.slices;
           e.fold_end = (before ? before->fold_end : 0) + (p.staged ? ctas : (ctas + kQuadWarps - 1) / kQuadWarps);
-          e.stage_end = (before ? before->stage_end : 0) + e.stage_strips * e.stage_segs * kUnit;
+          e.stage_end = (before ? before->stage_end : 0) +
+                        (e.stage_strips * e.stage_segs * e.unit * e.unit + kQuadWarps - 1) / kQuadWarps;
           b.e[b.n++] = e;
         }
     }
