@@ -742,6 +742,21 @@ size_t carry_stage_bytes(const std::vector<CarryPlan>& plans) {
   return std::max(one, std::min(all, kStageCells)) * 24;
 }
 
+// Rows of a segment: long runs amortise the 7 to 15 rows a segment computes twice, down
+// to 16 where the launch has fewer than want pieces.  A launch that does not fill the GPU
+// once with 16 waits for one segment's chain of rows, so it goes on to 4 while it stays
+// within one wave of few pieces (folding kernel, a residue with many q: A = 581, k = 21
+// 0.31 -> 0.20 ms; quad kernels: A = 867, k = 14 0.046 -> 0.031 ms); more than a wave
+// only computes rows again (A = 867, k = 18 0.078 -> 0.102 ms, 256 instances of an 8-bit
+// A at k = 16 1.85 -> 2.07 ms; A = 1019, k = 21 0.299 -> 0.310 ms), and a few rows split
+// badly (A = 9, k = 22 5.0 -> 6.2 ms).  Half of a block's pieces lie below its diagonal.
+static uint32_t rows_per(uint32_t most, uint32_t rows, uint64_t across, uint64_t want, uint64_t few) {
+  uint32_t seg = most;
+  while (seg > 16 && across * ((rows + seg - 1) / seg) < want) seg /= 2;
+  while (seg > 4 && seg <= 16 && rows > 10 && 2 * across * ((rows + seg - 1) / seg) <= few) seg /= 2;
+  return seg;
+}
+
 cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsigned long long* acc, void* stage,
                          size_t stage_bytes, cudaStream_t stream) {
   uint4* st16 = static_cast<uint4*>(stage);
@@ -781,13 +796,11 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
           e.acc = acc + i * 2 * kMaxBins;
           const uint32_t useful = p.staged ? kFoldThreads - ((1u << p.staged) - 1) : (128 - ((1u << p.b) - 1)) / 4 * 4;
           e.strips = (e.cols + useful - 1) / useful;
-          // rows per CTA: long runs amortise the rows a segment computes twice; short
-          // ones where the launch would leave SMs without a CTA
-          // (strips x segments are CTAs of the folding kernel, warps of the other)
-          const uint64_t want =
-              std::max<uint64_t>(1, (p.staged ? 8ull : 24ull) * num_sms / std::min<size_t>(std::max<size_t>(alike, 1), kEntries));
-          e.seg = 256;
-          while (e.seg > 16 && (uint64_t)e.strips * ((e.rows + e.seg - 1) / e.seg) < want) e.seg /= 2;
+          // rows per CTA (of the folding kernel; per warp of the others)
+          const uint64_t share = std::min<size_t>(std::max<size_t>(alike, 1), kEntries);
+          const uint64_t want = std::max<uint64_t>(1, (p.staged ? 8ull : 24ull) * num_sms / share);
+          const uint64_t warps = 10ull * num_sms / share;  // one wave of the quad kernels, nearly
+          e.seg = rows_per(256, e.rows, e.strips, want, p.staged ? (p.many ? 4ull : 2ull) * num_sms / share : warps);
           e.segs = (e.rows + e.seg - 1) / e.seg;
           e.slices = 1;
           if (p.many) {
@@ -816,10 +829,7 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
             used += need;
             const uint32_t wr = (e.srows + e.unit - 1) / e.unit, su = quad_useful<4>();
             e.stage_strips = (e.pitch + su - 1) / su;
-            e.stage_seg = 128;
-            while (e.stage_seg > 16 &&
-                   (uint64_t)e.stage_strips * e.unit * e.unit * ((wr + e.stage_seg - 1) / e.stage_seg) < want * 3 / 2)
-              e.stage_seg /= 2;
+            e.stage_seg = rows_per(128, wr, (uint64_t)e.stage_strips * e.unit * e.unit, want * 3 / 2, warps);
             e.stage_segs = (wr + e.stage_seg - 1) / e.stage_seg;
           }
           const CarryEntry* before = b.n ? &b.e[b.n - 1] : nullptr;

@@ -39,6 +39,16 @@ def test_carry_vs_tcgen05(ctx, A, k):
     assert res.raw == mma.raw and res.counts == mma.counts and res.minb == mma.minb
 
 
+@pytest.mark.parametrize("A,k", [(9, 14), (11, 12), (11, 17), (13, 14), (17, 13), (23, 12), (31, 16), (61, 19), (129, 18),
+                                 (301, 13), (581, 20), (867, 14), (723, 15)])
+def test_carry_short_segments(ctx, A, k):
+    """Segments of 4 and 8 rows: shorter than the rows a segment computes twice."""
+    res = ctx.histogram(req(A, k, dd.KERNEL_CARRY))
+    popc = ctx.histogram(req(A, k, dd.KERNEL_POPC))
+    assert (res.kernel_used, popc.kernel_used) == (dd.KERNEL_CARRY, dd.KERNEL_POPC)
+    assert res.raw == popc.raw and res.counts == popc.counts
+
+
 def test_carry_batch(ctx):
     """Jobs of one launch: more than a launch's 32 entries, every window length, few
     and many q, and staged blocks that need several rounds."""
