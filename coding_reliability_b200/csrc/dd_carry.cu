@@ -129,6 +129,45 @@ __device__ __forceinline__ void fold_column(const H16& g, uint32_t at, uint32_t 
   if (kTwice) red_add<24 * 128>(at2, g.p0[3]);
 }
 
+// The additions to the tables are the larger part of this kernel's shared-memory traffic
+// (nearly every warp has a column with a second q, so 48 a row).  With up to six window
+// bits a count stays below 2^12, so a word of an H16 (bins d and d + 4) goes to a cell as
+// it is: cell e of a lane's packed table holds distances e and e + 4 and is unpacked
+// every two rows of the CTA (24 additions a row, and 9 to unpack).  k = 22, A = 58659
+// 45.3 -> 40.6 ms, A = 40001 23.8 -> 20.4 ms; k = 21, A = 40001 20.1 -> 17.2 ms.  Seven
+// window bits would need unpacking within a row.  A field holds the counts of 12 warps'
+// rows; should it overflow all the same (4 q pairs of equal distance, most of a window's
+// pairs in one bin), the bins' sum is wrong, and the caller counts on another kernel.
+constexpr int kPackCells = 36;  // q distance <= 16, bins 0 .. 3, 8 .. 11, 16 .. 19 (and 4 more)
+template <int kLevels, bool kMany>
+__host__ __device__ constexpr bool fold_packed() { return kLevels <= 2 && !kMany; }
+template <bool kTwice, int kBin>
+__device__ __forceinline__ void pack_word(uint32_t w, uint32_t at, uint32_t at2) {
+  red_add<kBin * 128>(at, w);
+  if (kTwice) red_add<kBin * 128>(at2, w);
+}
+template <bool kTwice>
+__device__ __forceinline__ void pack_column(const H16& g, uint32_t at, uint32_t at2) {
+  pack_word<kTwice, 0>(g.p0[0], at, at2); pack_word<kTwice, 1>(g.p1[0], at, at2);
+  pack_word<kTwice, 2>(g.p2[0], at, at2); pack_word<kTwice, 3>(g.p3[0], at, at2);
+  pack_word<kTwice, 8>(g.p0[1], at, at2); pack_word<kTwice, 9>(g.p1[1], at, at2);
+  pack_word<kTwice, 10>(g.p2[1], at, at2); pack_word<kTwice, 11>(g.p3[1], at, at2);
+  pack_word<kTwice, 16>(g.p0[2], at, at2); pack_word<kTwice, 17>(g.p1[2], at, at2);
+  pack_word<kTwice, 18>(g.p2[2], at, at2); pack_word<kTwice, 19>(g.p3[2], at, at2);
+}
+// A warp's share of a packed table to the 32-bit one; other warps may go on adding.
+__device__ __forceinline__ void unpack_cells(uint32_t cells, uint32_t tab, int warp) {
+#pragma unroll
+  for (int i = 0; i < kPackCells / (kFoldThreads / 32); ++i) {
+    const uint32_t e = (uint32_t)(i * (kFoldThreads / 32) + warp) * 128;
+    uint32_t x;
+    asm volatile("atom.shared.exch.b32 %0, [%1], 0;" : "=r"(x) : "r"(cells + e) : "memory");
+    red_add<0>(tab + e, x & 0xFFFFu);
+    red_add<4 * 128>(tab + e, x >> 16);
+  }
+}
+static_assert(kPackCells % (kFoldThreads / 32) == 0 && kPackCells + 4 <= kTabRows, "a warp's cells, unpacked");
+
 // The first level of the last kLevels reads its own row only, with a ring in registers;
 // 8 rows of 16-bit histograms do not fit there, so kLevels = 4 reads row v + 8, too.
 template <int kLevels>
@@ -140,20 +179,24 @@ __host__ __device__ constexpr int fold_slots() { return fold_lead<kLevels>() + 1
 template <int kLevels>
 __host__ __device__ constexpr int fold_exchanges() { return kLevels == 2 ? 2 : kLevels - 1; }
 
-// Shared memory of the folding kernel: tables (U, D and a spare; U and D twice for wide products),
-// exchange rows, the ring of staged rows, and the q-distance counts of each thread (many).
-template <int kLevels>
-constexpr size_t fold_smem(bool many) {
+// Shared memory of the folding kernel: tables (U, D and a spare, which a q' past the last
+// reaches at distances up to 17; U and D twice for wide products), exchange rows, the ring of staged rows, and the q-distance counts of each thread (many).
+template <int kLevels, bool kMany>
+__host__ __device__ constexpr int fold_tables() {
+  return kTabBytes * (kMany ? 4 : fold_packed<kLevels, kMany>() ? 2 : 3) + (fold_packed<kLevels, kMany>() ? (3 * kPackCells + 1) * 128 : 0);
+}
+template <int kLevels, bool kMany>
+constexpr size_t fold_smem() {
   constexpr int cols = kFoldThreads + (1 << (kLevels - 1));
-  return (size_t)kTabBytes * (many ? 4 : 3) + (size_t)(48 * fold_exchanges<kLevels>() + 24 * fold_slots<kLevels>()) * cols +
-         (many ? (size_t)(16 + 1) * kFoldThreads * 4 : 0);
+  return (size_t)fold_tables<kLevels, kMany>() + (size_t)(48 * fold_exchanges<kLevels>() + 24 * fold_slots<kLevels>()) * cols +
+         (kMany ? (size_t)(16 + 1) * kFoldThreads * 4 : 0);
 }
 
 // The last kLevels steps (s = 2^(kLevels-1) .. 1), from the staged 8-bit histograms to
 // 16-bit ones, and the sum over q, q'.  CTA: a strip of columns (one per thread, the
 // last 2^kLevels - 1 only feed their neighbours) x a segment of rows.  Measured and
-// dropped: a warp alone with shuffles and two 16-bit counts folded as one word (k = 22
-// 58.7 against 52.9 ms: fewer warps for its tables), CTAs of 256 threads (57 ms).
+// dropped: a warp alone with shuffles and tables of its own (k = 22 58.7 against 52.9 ms:
+// fewer warps), CTAs of 256 threads (57 ms).
 template <int kLevels, bool kMany>
 __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold_kernel(const __grid_constant__ CarryBatch batch) {
   constexpr int kThreads = kFoldThreads;
@@ -179,11 +222,11 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
 
   // shared memory
   uint32_t* tab = reinterpret_cast<uint32_t*>(smem);  // U, D (and their high parts)
-  uint8_t* ex = smem + kTabBytes * (kMany ? 4 : 3);
+  uint8_t* ex = smem + fold_tables<kLevels, kMany>();
   uint4* in16 = reinterpret_cast<uint4*>(ex + 48 * fold_exchanges<kLevels>() * kCols);
   uint2* in8 = reinterpret_cast<uint2*>(in16 + kSlots * kCols);
   uint32_t* qd = reinterpret_cast<uint32_t*>(in8 + kSlots * kCols);
-  for (int i = tid; i < kTabBytes * (kMany ? 4 : 2) / 4; i += kThreads) tab[i] = 0;
+  for (int i = tid; i < fold_tables<kLevels, kMany>() / 4; i += kThreads) tab[i] = 0;
   if constexpr (kMany)
     for (int i = tid; i < 17 * kThreads; i += kThreads) qd[i] = 0;
 
@@ -195,7 +238,10 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
   uint32_t qr = mul_mod(a.qinv, a.row0 + r, a.A);
   const uint32_t tab_u = (uint32_t)__cvta_generic_to_shared(tab) + lane * 4u;
   const bool two = qc + a.A < a.nq, second = __any_sync(0xffffffffu, two);  // a second q: here, in this warp
-  const uint32_t spare = tab_u + 2 * kTabBytes;  // few q: the third table is not read
+  // few q: the third table is not read
+  constexpr bool kPacked = fold_packed<kLevels, kMany>();
+  constexpr uint32_t kNext = kPacked ? kPackCells * 128 : kTabBytes;  // from U to D to the spare
+  const uint32_t to_u = kPacked ? tab_u + 2 * kTabBytes : tab_u, spare = to_u + 2 * kNext;
 
   // input: staged rows through a ring of kSlots rows
   int slot = 0;  // ring slot of load number it (row r + kLead of that step)
@@ -254,9 +300,12 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
 #pragma unroll 1
           for (uint32_t q = qr; q < a.nq; q += a.A) {
             // columns that do not count here go to a spare column of the table
-            const uint32_t to = !mine || vc < v ? spare : vc == v ? tab_u + kTabBytes : tab_u;
+            const uint32_t to = !mine || vc < v ? spare : vc == v ? to_u + kNext : to_u;
             const uint32_t at = to + (__popc(q ^ qc) << 7);
-            if (second) fold_column<true>(g, at, (two ? to : spare) + (__popc(q ^ (qc + a.A)) << 7));
+            if constexpr (kPacked) {
+              if (second) pack_column<true>(g, at, (two ? to : spare) + (__popc(q ^ (qc + a.A)) << 7));
+              else pack_column<false>(g, at, at);
+            } else if (second) fold_column<true>(g, at, (two ? to : spare) + (__popc(q ^ (qc + a.A)) << 7));
             else fold_column<false>(g, at, at);
           }
       } else if (mine && r < r1 && vc >= v) {
@@ -278,9 +327,18 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
       }
       qr = sub_mod(qr, a.qinv, a.A);
     }
+    if constexpr (kPacked) {
+      if (kUnroll == 2 || (it & 1)) unpack_cells(to_u, tab_u, warp);
+      if ((it & 31) >= 32 - kUnroll) unpack_cells(to_u + kNext, tab_u + kTabBytes, warp);  // a row has one v = v'
+    }
   }
   copy_wait<0>();
   __syncthreads();
+  if constexpr (kPacked) {
+    unpack_cells(to_u, tab_u, warp);
+    unpack_cells(to_u + kNext, tab_u + kTabBytes, warp);
+    __syncthreads();
+  }
   // tables -> global sums
   for (int d = warp; d < 2 * kTabRows; d += kThreads / 32) {
     const uint32_t x = tab[d * 32 + lane];
@@ -656,7 +714,7 @@ cudaError_t run_staged(const CarryBatch& b, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   carry_stage_kernel<<<b.e[b.n - 1].stage_end, kQuadWarps * 32, kStageBytes, stream>>>(b);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  constexpr size_t smem = fold_smem<kLevels>(kMany);
+  constexpr size_t smem = fold_smem<kLevels, kMany>();
   auto fn = carry_fold_kernel<kLevels, kMany>;
   if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
   fn<<<b.e[b.n - 1].fold_end, kFoldThreads, smem, stream>>>(b);

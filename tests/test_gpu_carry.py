@@ -49,6 +49,17 @@ def test_carry_short_segments(ctx, A, k):
     assert res.raw == popc.raw and res.counts == popc.counts
 
 
+@pytest.mark.parametrize("A,k", [(33, 11), (33, 12), (63, 11), (63, 12), (129, 13), (255, 14), (4095, 17), (4095, 18), (3583, 18),
+                                 (16385, 20), (32767, 21), (32769, 21), (65535, 21), (58659, 21), (65521, 22)])
+def test_carry_packed_fold(ctx, A, k):
+    """Windows of 5 and 6 bits: one and two folded levels, one and two q per residue,
+    16-bit q (whose last neighbour is past the table's distances)."""
+    res = ctx.histogram(req(A, k, dd.KERNEL_CARRY))
+    mma = ctx.histogram(req(A, k, dd.KERNEL_MMA))
+    assert (res.kernel_used, mma.kernel_used) == (dd.KERNEL_CARRY, dd.KERNEL_MMA)
+    assert res.raw == mma.raw and res.counts == mma.counts
+
+
 def test_carry_batch(ctx):
     """Jobs of one launch: more than a launch's 32 entries, every window length, few
     and many q, and staged blocks that need several rounds."""
