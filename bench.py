@@ -14,11 +14,12 @@ region the headline histogram is computed once more on the other kernel and
 must be identical (`parity`).
 
 Reported per the harness contract: one JSON line on rank 0.
-  value   pairs/s from the kernel's own CUDA events (codewords are generated
+  value   pairs/s from the kernels' own CUDA events (codewords are generated
           on the device: the inputs are scalars already resident)
   e2e     pairs/s measured around the whole dd_histogram call on the stream
-          (job-table H2D, bin reset, kernel, bins D2H)
-  roofline  POPC-pipe fraction: pairs/s x popc-per-pair / measured POPC rate
+          (job-table H2D, bin reset, kernels, bins D2H)
+  roofline  fraction of the bound of the route that ran: instruction issue
+          (residue pairs), shared-memory atomics (tcgen05), POPC rate (popc)
   cpu_baseline  the reference's own CPU path (-c) on a bounded sample
 
 `--impl reference` times the reference's own CPU implementation (its `codrel -c`
@@ -59,8 +60,14 @@ MMA_K_PAD = 64  # int8 K of every tcgen05 tile (operand bit planes padded to 64)
 UNIT = "pairs/s"
 
 
-# residue-pair kernels (k=24 runs 4 staged and 4 folded levels, as the capture does)
-NCU_WARP_INST_PER_RESIDUE_PAIR = (137859072 + 328428147) / (5409 * 5410 // 2)
+# residue-pair kernels (k=24 runs 4 staged and 4 folded levels, as the capture does):
+# warp instructions (smsp__inst_executed.sum) and DRAM bytes of the staging and the
+# folding launch of A=5409, k=21, over its residue pairs
+NCU_CARRY_PAIRS = 5409 * 5410 // 2
+NCU_WARP_INST_PER_RESIDUE_PAIR = (148741596 + 300484621) / NCU_CARRY_PAIRS
+NCU_DRAM_BYTES_PER_RESIDUE_PAIR = (43776 + 431059200 + 382256384 + 6925312) / NCU_CARRY_PAIRS
+JOB_BYTES = 160               # one job-table entry, host to device
+RESULT_BYTES = 16 * 8 + 64 * 8  # control words and one slot of 64 bins, device to host
 
 
 def issue_roofline(pairs_per_s: float, epilogue: str, sm_mhz, num_sms: int) -> dict:
@@ -119,10 +126,21 @@ class ClockSampler:
         try:
             self.f = open(path, "w")
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={index}", f"--query-gpu={q}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"],
+                                          "--format=csv,noheader,nounits", "-lms", "20"],
                                          stdout=self.f, stderr=subprocess.DEVNULL)
         except Exception:
             self.proc = None
+
+    def samples(self) -> int:
+        """Complete samples so far."""
+        return self.path.read_text().count("\n") if self.proc else 0
+
+    def load_until(self, samples: int, step, limit_s: float = 5.0) -> None:
+        """Runs untimed steps until that many samples are there (or the time is up): a
+        timed region of a few milliseconds is shorter than nvidia-smi's own query."""
+        end = time.perf_counter() + limit_s
+        while self.proc and self.samples() < samples and time.perf_counter() < end:
+            step()
 
     def stop(self) -> dict:
         if not self.proc:
@@ -241,10 +259,24 @@ def counts_digest(counts: list[int]) -> str:
     return hashlib.sha256(",".join(str(c) for c in counts).encode()).hexdigest()
 
 
+def kernel_launches(step) -> int:
+    """Kernels that one (untimed) step launches, counted by the profiler; 1 where it
+    records none."""
+    try:
+        from torch.profiler import ProfilerActivity, profile
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            step()
+        names = [e.name for e in prof.events()]
+    except Exception as e:  # no profiler on this machine
+        print(f"kernel launches not counted: {e}", file=sys.stderr)
+        names = []
+    return sum("kernel" in n and not n.startswith("cuda") for n in names) or 1
+
+
 def cross_kernel_check(ctx, dd, A: int, k: int, timed) -> dict:
     """Recomputes the timed histogram on another kernel (popc for tcgen05, tcgen05
-    for popc and for the residue-pair kernels) and requires the identical raw bins and counts: two independent
-    implementations of the same exact histogram."""
+    for popc and for the residue-pair kernels) and requires the identical raw bins
+    and counts: two independent implementations of the same exact histogram."""
     other = dd.KERNEL_POPC if timed.kernel_used == dd.KERNEL_MMA else dd.KERNEL_MMA
     o = ctx.histogram(dd.Request(dd.CODE_AN, dd.MODE_EXHAUSTIVE, A, k, kernel=other))
     assert o.kernel_used == other
@@ -314,6 +346,7 @@ def main() -> None:
 
     clocks_dir = Path(args.clocks_dir) if args.clocks_dir else Path(tempfile.gettempdir())
     clocks = ClockSampler(local, clocks_dir / f"clocks_rank{rank}.csv")
+    clocks.load_until(2, lambda: ctx.histogram(req))
     barrier()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     ev0.record(stream)
@@ -327,12 +360,15 @@ def main() -> None:
     ev1.record(stream)
     barrier()
     total_ms = ev0.elapsed_time(ev1)
+    clocks.load_until(clocks.samples() + 3, lambda: ctx.histogram(req))  # the same load, still under way
     clk = clocks.stop()
 
     t_kernel, t_total = max_over_ranks([kernel_ms, total_ms], world, "cuda")
     # every step must produce the same exact histogram
     assert all(r.counts == results[0].counts for r in results)
     assert sum(results[0].raw) == P
+
+    launches_per_step = kernel_launches(lambda: ctx.histogram(req)) if rank == 0 else 1
 
     # the same histogram once more on the other kernel, outside the timed region
     parity = None
@@ -346,18 +382,22 @@ def main() -> None:
     mma = results[0].kernel_used == dd.KERNEL_MMA
     if results[0].kernel_used == dd.KERNEL_CARRY:
         # residue-pair kernels: A^2 / 2 pairs of residues stand for the 4^k / 2 pairs of
-        # codewords; the bound is instruction issue
+        # codewords; the bounds are instruction issue (staging kernel) and the
+        # shared-memory pipe (folding kernel)
         rpairs = A * (A + 1) // 2 * args.steps / (kernel_ms * 1e-3)
         peak = ISSUE_PER_CLOCK_PER_SM * torch.cuda.get_device_properties(local).multi_processor_count * \
             (clk.get("sm_mhz") or 0) * 1e6
         roofline = {"bound": "issue", "achieved": rpairs * NCU_WARP_INST_PER_RESIDUE_PAIR / 1e9,
                     "peak": peak / 1e9 if peak else None, "unit": "Ginst/s",
                     "frac": rpairs * NCU_WARP_INST_PER_RESIDUE_PAIR / peak if peak else None,
-                    "traffic": None, "residue_pairs_per_s": rpairs, "codeword_pairs_per_residue_pair": P / (A * (A + 1) // 2),
+                    "traffic": NCU_DRAM_BYTES_PER_RESIDUE_PAIR * A * (A + 1) / 2,
+                    "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum per residue pair of the captured "
+                                      "launches (staged histograms, written once and read once), x this step's residue pairs",
+                    "residue_pairs_per_s": rpairs, "codeword_pairs_per_residue_pair": P / (A * (A + 1) // 2),
                     "warp_inst_per_residue_pair": NCU_WARP_INST_PER_RESIDUE_PAIR,
-                    "peak_source": "4 warp instructions per clock per SM at the median SM clock sampled in the timed "
-                                   "region; instructions per residue pair from sm__inst_executed.sum of the staging and "
-                                   "folding kernels of one block (A=5409, k=21), ncu capture"}
+                    "peak_source": "4 warp instructions per clock per SM at the median SM clock sampled over the timed "
+                                   "steps and the untimed ones around them; instructions per residue pair from "
+                                   "smsp__inst_executed.sum of the staging and folding kernels, ncu capture (A=5409, k=21)"}
     elif mma:
         # tcgen05 path: the tensor core computes the distances; the bound is the
         # histogram epilogue's shared-memory atomics: one per pair (single
@@ -405,10 +445,11 @@ def main() -> None:
         "scaling": "weak", "vs_baseline": None, "dtype": "u64", "data": "synthetic",
         "config": {"workload": f"an_exhaustive_A{A}_k{k}", "A": A, "k": k, "codeword_bits": 40, "bins": 41,
                    "pairs": P, "parallelism": f"replicas x{world}",
-                   "cold_l2": "n/a: codewords generated in registers, no HBM input"},
+                   "cold_l2": "n/a: codewords generated in registers, no HBM input (the residue-pair "
+                              "route writes and reads its staged histograms, more than L2 per step)"},
         "roofline": roofline,
-        "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": 256, "d2h_bytes_per_step": 64 * 8 * 8},
-        "gpu_launches": args.steps,
+        "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": JOB_BYTES, "d2h_bytes_per_step": RESULT_BYTES},
+        "gpu_launches": args.steps * launches_per_step,
         "clocks": clk,
         "kernel_used": kname(results[0]),
         "autotune": tuning,
