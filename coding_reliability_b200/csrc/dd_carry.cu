@@ -754,11 +754,16 @@ bool carry_eligible(const Job& j) {
   return a <= 16 && j.n > a;
 }
 
-// Residue pairs cost about as much as the tcgen05 kernel's 16^2 codeword pairs
-// (16-bit A: k = 19, 17.9 ms here and 15.3 ms there; k = 20, 26.8 and 63.5 ms); below
-// k = 14 a launch of the popc kernel takes no longer than this path's three.
+// A residue pair costs about as much as the tcgen05 kernel's 11^2 codeword pairs, so with
+// three bits more than A's it depends on A itself (A of 16 bits, k = 19: A = 34407
+// 7.0 ms here and 12.5 ms there, 42599 9.5, 49153 12.2, 55705 15.3; 15 bits, k = 18:
+// 17203 2.1 and 3.2 ms, 21299 2.8, 24577 3.4; from 17 down a launch fills the GPU less,
+// 14 bits, k = 17, A = 10649 1.02 and 0.90 ms), with four it always does (A = 62307,
+// k = 20 20.6 and 59.2 ms).  Below k = 14 a launch of the popc kernel takes no longer
+// than this path's three.
 bool carry_wins(const Job& j) {
-  const uint32_t a = bits_of(odd_part(j.A));
+  const uint32_t odd = odd_part(j.A), a = bits_of(odd);
+  if (j.n == a + 3 && j.n >= 18) return 5ull * odd <= 7ull << (a - 1);
   return j.n >= a + 4 && j.n >= 14;
 }
 

@@ -114,3 +114,14 @@ def test_route(ctx):
         for q, r in zip(qs, out):
             p = ctx.histogram(dd.Request(q.code, q.mode, q.A, q.n, m=q.m, convention=q.convention, kernel=dd.KERNEL_POPC))
             assert r.raw == p.raw and r.counts == p.counts and r.pairs == p.pairs
+
+
+@pytest.mark.parametrize("A,k,carry", [(32769, 19, True), (45875, 19, True), (45877, 19, False), (65535, 19, False), (22937, 18, True),
+                                       (22939, 18, False), (2 * 22937, 18, True), (8193, 17, False), (32769, 18, False)])
+def test_route_three_bits(ctx, A, k, carry):
+    """k three bits above A's: the residues of the shorter multipliers, codewords for the others."""
+    ctx.autotune()
+    res = ctx.histogram(req(A, k, dd.KERNEL_AUTO))
+    assert res.kernel_used == (dd.KERNEL_CARRY if carry else dd.KERNEL_MMA)
+    other = ctx.histogram(req(A, k, dd.KERNEL_MMA if carry else dd.KERNEL_CARRY))
+    assert res.raw == other.raw and res.counts == other.counts
