@@ -18,12 +18,13 @@
 // With b = k - bits(A) that is about b A^2 / 2 small steps instead of 4^k / 2 pairs
 // (A = 58659, k = 22: 1.0e10 against 8.8e12), all in integers.
 //
-// Measured on B200 against the tcgen05 kernel: A = 62307, k = 22: 50 ms against 941 ms
-// (965 ms before its generators were mended), k = 20: 20.6 against 59.5 ms; A = 867,
-// k = 21: 0.31 against 193 ms, k = 16: 0.055 against 0.29 ms.  Bound by instruction
-// issue and its latencies at 12 to 18 warps an SM, the ALU and shared-memory pipes each
-// a bit over half busy; DRAM carries nothing up to 4 window bits and the staged
-// histograms (24 bytes a residue pair, once each way) above.
+// Measured on B200 against the tcgen05 kernel: A = 58659, k = 22: 40.6 ms against 941 ms
+// (965 ms before its generators were mended), k = 24: 85 ms against 15 s; A = 62307,
+// k = 20: 20.6 against 59.2 ms; A = 867, k = 21: 0.25 against 193 ms, k = 16: 0.046
+// against 0.28 ms.  Bound by instruction issue and its latencies at 12 to 18 warps an
+// SM, the ALU (staging) and shared-memory (folding) pipes three quarters busy; DRAM
+// carries nothing up to 4 window bits and the staged histograms (24 bytes a residue
+// pair, once each way) above.
 //
 // A histogram lives in registers, packed: four 8-bit counts per word while the
 // counts stay within 4^4, two 16-bit counts per word up to 4^8.  The count 4^4 (4^8)
@@ -69,8 +70,8 @@ struct CarryEntry {
 
 // Entries of one launch, in its parameters (short instances share a launch, and so
 // fill the GPU together; 31 entries stay below the 4 KB every launch can pass).  64
-// instances of 8-bit A, k = 14: 0.33 ms, 2.0 ms launched one by one; 256 at k = 16:
-// 2.5 ms, popc kernel 123, tcgen05 81.
+// instances of 8-bit A, k = 14: 0.18 ms (0.33 when they first shared one, 2.0 launched one
+// by one); 256 at k = 16: 1.9 ms, popc kernel 123, tcgen05 54.
 constexpr uint32_t kEntries = 31;
 struct CarryBatch {
   uint32_t n;
@@ -180,10 +181,11 @@ template <int kLevels>
 __host__ __device__ constexpr int fold_exchanges() { return kLevels == 2 ? 2 : kLevels - 1; }
 
 // Shared memory of the folding kernel: tables (U, D and a spare, which a q' past the last
-// reaches at distances up to 17; U and D twice for wide products), exchange rows, the ring of staged rows, and the q-distance counts of each thread (many).
+// reaches at distances up to 17; U and D twice for wide products), exchange rows, the
+// ring of staged rows, and the q-distance counts of each thread (many).
 template <int kLevels, bool kMany>
 __host__ __device__ constexpr int fold_tables() {
-  return kTabBytes * (kMany ? 4 : fold_packed<kLevels, kMany>() ? 2 : 3) + (fold_packed<kLevels, kMany>() ? (3 * kPackCells + 1) * 128 : 0);
+  return fold_packed<kLevels, kMany>() ? kTabBytes * 2 + (3 * kPackCells + 1) * 128 : kTabBytes * (kMany ? 4 : 3);
 }
 template <int kLevels, bool kMany>
 constexpr size_t fold_smem() {
@@ -362,8 +364,9 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
 // holds distances e and e + 1 in its halves and is unpacked to 32 bits every
 // kPackedRows rows.  A = 62307, k = 20: 28.5 ms with one column a thread (367 warp
 // instructions per 32 residue pairs, neighbours through shared memory and a barrier a
-// step), 20.6 ms (about 200); with the first ring in registers, too, 29 ms (254
-// registers, 8 warps an SM, an unrolled loop past the instruction cache).
+// step), 20.6 ms so (229 at A = 30011, k = 19, margins included); with the first ring in
+// registers, too, 29 ms (254 registers, 8 warps an SM, an unrolled loop past the
+// instruction cache).
 constexpr int kCells = 37;                 // q distance <= 16, bins 0, 2, .. 20
 constexpr int kDiscard = 21;               // cells for columns that do not count
 constexpr int kPackedRows = 16;            // x 4 columns x 4 q pairs x 255 stays below 2^16
@@ -868,7 +871,7 @@ cudaError_t launch_carry(const std::vector<CarryPlan>& plans, int num_sms, unsig
           e.slices = 1;
           if (p.many) {
             // every slice computes the windows again, so only as many as fill the GPU once
-            // (A = 867, k = 21: 0.65 ms with four times as many, 0.32 ms)
+            // (A = 867, k = 21: 0.65 ms with four times as many, 0.32 ms so, with segments of 16)
             const uint64_t per = (e.nq + p.A - 1) / p.A, ctas = (uint64_t)e.strips * e.segs;
             e.slices = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(per, 4096), std::max<uint64_t>(1, want / 4 / ctas));
             // a lane's 32-bit sums: rows x warps (x one lane) x q pairs x 4^b
