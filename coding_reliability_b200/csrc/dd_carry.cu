@@ -20,7 +20,7 @@
 //
 // Measured on B200 against the tcgen05 kernel: A = 58659, k = 22: 40.6 ms against 941 ms
 // (965 ms before its generators were mended), k = 24: 85 ms against 15 s; A = 62307,
-// k = 20: 20.6 against 59.2 ms; A = 867, k = 21: 0.25 against 193 ms, k = 16: 0.046
+// k = 20: 20.6 against 59.2 ms; A = 867, k = 21: 0.18 against 193 ms, k = 16: 0.046
 // against 0.28 ms.  Bound by instruction issue and its latencies at 12 to 18 warps an
 // SM, the ALU (staging) and shared-memory (folding) pipes three quarters busy; DRAM
 // carries nothing up to 4 window bits and the staged histograms (24 bytes a residue
@@ -41,6 +41,7 @@
 // steps hold one column a thread in words of every fourth bin, so that multiplying by
 // z renames words and shifts only one in four (carry_fold_kernel).
 #include <algorithm>
+#include <utility>
 
 #include "dd_carry.cuh"
 
@@ -168,6 +169,41 @@ __device__ __forceinline__ void unpack_cells(uint32_t cells, uint32_t tab, int w
   }
 }
 static_assert(kPackCells % (kFoldThreads / 32) == 0 && kPackCells + 4 <= kTabRows, "a warp's cells, unpacked");
+
+// Many q: the counts of the 17 q distances (f, a stride of kStride words) times kN bins of
+// a window from kFrom on.  The products are summed in registers, so that a residue pair
+// costs 57 additions to the table in two parts (both at once would spill) instead of up to
+// 17 x 25: A = 1019, k = 21 0.298 -> 0.188 ms, A = 867, k = 20 0.200 -> 0.128 ms, A = 61
+// 0.133 -> 0.106 ms; shorter multipliers spend their time on the pairs of q.  The host
+// sends sums that do not fit 32 bits to the wide products.
+template <int kBin>
+__device__ __forceinline__ uint32_t bin_of(const H16& g) {
+  constexpr int j = kBin / 8, m = kBin % 4;
+  const uint32_t w = m == 0 ? g.p0[j] : m == 1 ? g.p1[j % 3] : m == 2 ? g.p2[j % 3] : g.p3[j % 3];
+  return kBin % 8 < 4 ? w & 0xFFFFu : w >> 16;
+}
+template <int kFrom, int... kI>
+__device__ __forceinline__ void take_bins(const H16& g, uint32_t* x, std::integer_sequence<int, kI...>) {
+  ((x[kI] = bin_of<kFrom + kI>(g)), ...);
+}
+template <int kFrom, int... kI>
+__device__ __forceinline__ void add_sums(uint32_t at, const uint32_t* x, std::integer_sequence<int, kI...>) {
+  (red_add<(kFrom + kI) * 128>(at, x[kI]), ...);
+}
+template <int kFrom, int kN, int kStride>
+__device__ __forceinline__ void add_product(const volatile uint32_t* f, const H16& g, uint32_t at) {
+  uint32_t x[kN], sum[kN + 16];
+  take_bins<kFrom>(g, x, std::make_integer_sequence<int, kN>());
+#pragma unroll
+  for (int e = 0; e < kN + 16; ++e) sum[e] = 0;
+#pragma unroll
+  for (int d = 0; d <= 16; ++d) {
+    const uint32_t n = f[d * kStride];
+#pragma unroll
+    for (int i = 0; i < kN; ++i) sum[d + i] += n * x[i];
+  }
+  add_sums<kFrom>(at, sum, std::make_integer_sequence<int, kN + 16>());
+}
 
 // The first level of the last kLevels reads its own row only, with a ring in registers;
 // 8 rows of 16-bit histograms do not fit there, so kLevels = 4 reads row v + 8, too.
@@ -317,12 +353,18 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
           const uint32_t fa = (uint32_t)__cvta_generic_to_shared(qd + tid);
           for (uint32_t q = qr + slice * a.A; q < a.nq; q += a.slices * a.A)
             for (uint32_t p = qc; p < a.nq; p += a.A) red_add<0>(fa + __popc(q ^ p) * (kThreads * 4), 1);
-          for (uint32_t d = 0; d <= 16; ++d) {
-            const uint32_t x = f[d * kThreads];
-            if (x) {
-              f[d * kThreads] = 0;
-              if (a.wide) add_hist<kWideProduct>(at + (d << 7), x, g);
-              else add_hist<kNarrow>(at + (d << 7), x, g);
+          if (!a.wide) {
+            add_product<0, 13, kThreads>(f, g, at);
+            add_product<13, 12, kThreads>(f, g, at);
+#pragma unroll
+            for (uint32_t d = 0; d <= 16; ++d) f[d * kThreads] = 0;
+          } else {
+            for (uint32_t d = 0; d <= 16; ++d) {
+              const uint32_t x = f[d * kThreads];
+              if (x) {
+                f[d * kThreads] = 0;
+                add_hist<kWideProduct>(at + (d << 7), x, g);
+              }
             }
           }
         }

@@ -60,6 +60,16 @@ def test_carry_packed_fold(ctx, A, k):
     assert res.raw == mma.raw and res.counts == mma.counts
 
 
+@pytest.mark.parametrize("A,k", [(3, 14), (3, 18), (5, 20), (31, 15), (33, 15), (63, 20), (65, 16), (255, 18), (511, 19), (1019, 21),
+                                 (1023, 20), (2047, 21), (8191, 23)])
+def test_carry_many_q(ctx, A, k):
+    """Many q per residue: sums in registers, and the wide products of the shortest A."""
+    res = ctx.histogram(req(A, k, dd.KERNEL_CARRY))
+    mma = ctx.histogram(req(A, k, dd.KERNEL_MMA))
+    assert (res.kernel_used, mma.kernel_used) == (dd.KERNEL_CARRY, dd.KERNEL_MMA)
+    assert res.raw == mma.raw and res.counts == mma.counts
+
+
 def test_carry_batch(ctx):
     """Jobs of one launch: more than a launch's 32 entries, every window length, few
     and many q, and staged blocks that need several rounds."""
