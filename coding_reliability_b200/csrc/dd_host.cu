@@ -163,31 +163,66 @@ static uint32_t mma_epilogue_of(const dd_context* ctx) {
 // Under AUTO, jobs below these many distance evaluations stay on the popc kernel: the
 // tcgen05 kernel's fixed cost per launch (TMEM allocation, clearing and folding its
 // ~180 KB table) outweighs its rate there, and a triangle's diagonal strips weigh more
-// on it.  Exhaustive, one instance: k = 15, 5.4e8 pairs, popc 0.145 ms, tcgen05 0.129 ms;
-// k = 14 0.049 and 0.063 ms.  Grids: 1.6e8 pairs 0.18 and 0.10 ms.  In a launch of many
-// instances the fixed cost is shared: 16 of k = 14 0.53 and 0.42 ms, 64 of k = 12 0.15
-// and 0.21 ms.
+// on it.  Exhaustive, one instance: k = 15, 5.4e8 pairs, popc 0.144 ms, tcgen05 0.117 ms;
+// k = 14 0.049 and 0.061 ms.  2-D grids, whose lattice columns the popc kernel computes
+// one by one: 1.3e8 pairs (1000 x 134217) 0.164 and 0.080 ms.  In a launch of many
+// instances the fixed cost is shared: 8 of k = 14 0.280 and 0.289 ms, 12 0.400 and 0.342,
+// 16 0.53 and 0.41; 16 of k = 13 0.152 and 0.186 ms.
 constexpr double kMmaMinTriangle = 536870912.0;  // 2^29
 constexpr double kMmaMinRect = 134217728.0;      // 2^27
 constexpr double kMmaMinShared = 67108864.0;     // 2^26, in a launch of
-constexpr double kMmaMinLaunch = 1073741824.0;   // 2^30 or more in such jobs
+constexpr double kMmaMinLaunch = 1342177280.0;   // 1.25 x 2^30 or more in such jobs
+constexpr double kMmaAlways = 1073741824.0;      // 2^30
 
 static double pairs_of(const Job& j) {
   return j.shape == SHAPE_TRIANGLE ? 0.5 * (double)j.rows * (double)j.rows : (double)j.rows * (double)j.cols;
 }
 
+// 1-D grids below kMmaAlways: their columns are codewords in sequence, which the popc
+// kernel bins at its full rate where a tile has all of its 128 rows (a count of rows that
+// is no multiple of 128 leaves one row tile on the checked loop, and the two loops
+// together run slower), while the tcgen05 kernel writes an operand for every column tile
+// whether 128 rows use it or 4096.  So the two costs, in microseconds of a launch, or of
+// one more job of a launch that is shared: fixed, for each column tile, for each full
+// tile, for each checked one.  The coefficients fit 450 measured shapes (k = 13 .. 24, m
+// of 2^25.5 .. 2^30 / 2^k in whole and ragged tiles, A of 7, 11 and 16 bits); where the
+// rule decides, its choice takes 1.005 times the faster kernel's time in the mean and 1.05 times
+// the popc kernel's at most (A = 62307, popc and tcgen05: k = 20, m = 128 0.045 and 0.084
+// ms, m = 512 0.136 and 0.131; k = 17, m = 1024 0.044 and 0.062, m = 4096 0.136 and 0.103;
+// k = 16, m = 2805 0.088 and 0.070; 16 jobs of k = 18, m = 256 0.26 and 0.36, of k = 14,
+// m = 4096 0.26 and 0.24).
+static bool progression_on_mma(const Job& j, bool shared) {
+  const double tiles = (double)j.col_tiles, full = (double)(j.rows / kWarpRows);
+  const uint32_t rest = (uint32_t)(j.rows % kWarpRows);
+  double popc = shared ? 0.0 : 13.0, mma = shared ? 4.0 : 36.0;
+  if (rest) {
+    popc += tiles * (0.048 * full + 0.066 + 0.013 * ((rest + 31) / 32));
+    mma += tiles * (0.045 + 0.0135 * full + (rest % 32 ? 0.042 : 0.022));
+  } else {
+    popc += tiles * 0.0295 * full;
+    mma += tiles * (0.045 + 0.0135 * full);
+  }
+  return mma < popc;
+}
+
+// Whether a job that AUTO leaves to the pair kernels is one for the tcgen05 kernel where the
+// autotuner prefers that.  launch_pairs: pairs of the launch's jobs that could share one
+// (0: unknown).
+static bool large_for_mma(const Job& j, double launch_pairs) {
+  const bool shared = launch_pairs >= kMmaMinLaunch;
+  const double pairs = pairs_of(j);
+  if (pairs < (shared ? kMmaMinShared : j.shape == SHAPE_TRIANGLE ? kMmaMinTriangle : kMmaMinRect)) return false;
+  return pairs >= kMmaAlways || j.shape == SHAPE_TRIANGLE || j.col_kind != COL_PROGRESSION || progression_on_mma(j, shared);
+}
+
 // Which pair kernel runs a job: explicit MMA or POPC requests are honoured where
 // the job allows them; AUTO uses the context's measured preference for jobs
-// large enough to amortise the tcgen05 kernel's launch.  launch_pairs: pairs of the
-// launch's jobs that could share one (0: unknown).
+// large enough to amortise the tcgen05 kernel's launch.
 static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel, double launch_pairs = 0) {
   if (!mma_eligible(j)) return false;
   if (kernel == DD_KERNEL_MMA) return true;
   if (kernel == DD_KERNEL_POPC) return false;
-  const double least = launch_pairs >= kMmaMinLaunch ? kMmaMinShared
-                       : j.shape == SHAPE_TRIANGLE   ? kMmaMinTriangle
-                                                     : kMmaMinRect;
-  return ctx->tuned == 2 && pairs_of(j) >= least;  // autotuner's verdict for AN exhaustive shapes
+  return ctx->tuned == 2 && large_for_mma(j, launch_pairs);  // autotuner's verdict for AN exhaustive shapes
 }
 
 // The jobs' routes: the carry path for each where it is asked for or wins and its

@@ -70,7 +70,8 @@ typedef enum dd_mode {
 typedef enum dd_kernel {
   DD_KERNEL_AUTO = 0,  /* the carry kernels where they win (dd_carry.cu), else the autotuner's choice
                           for the shape; jobs too small for the tcgen05 kernel's fixed cost (2^29 pairs
-                          exhaustive, 2^27 in a grid) stay on the popc kernel */
+                          exhaustive, 2^27 in a grid; 1-D grids below 2^30 by an estimate of both
+                          kernels' times) stay on the popc kernel */
   DD_KERNEL_POPC = 1,  /* XOR + POPC, warp-private shared-memory bins */
   DD_KERNEL_MMA = 2,   /* tcgen05 kind::i8 bit-plane MMA, histogram epilogue from TMEM */
   DD_KERNEL_CARRY = 3  /* residues of A (odd part of at most 16 bits) instead of codewords, whole
