@@ -134,12 +134,18 @@ __device__ __forceinline__ void fold_column(const H16& g, uint32_t at, uint32_t 
 // The additions to the tables are the larger part of this kernel's shared-memory traffic
 // (nearly every warp has a column with a second q, so 48 a row).  With up to six window
 // bits a count stays below 2^12, so a word of an H16 (bins d and d + 4) goes to a cell as
-// it is: cell e of a lane's packed table holds distances e and e + 4 and is unpacked
-// every two rows of the CTA (24 additions a row, and 9 to unpack).  k = 22, A = 58659
-// 45.3 -> 40.6 ms, A = 40001 23.8 -> 20.4 ms; k = 21, A = 40001 20.1 -> 17.2 ms.  Seven
-// window bits would need unpacking within a row.  A field holds the counts of 12 warps'
-// rows; should it overflow all the same (4 q pairs of equal distance, most of a window's
-// pairs in one bin), the bins' sum is wrong, and the caller counts on another kernel.
+// it is: cell e of a lane's packed table holds distances e and e + 4 (24 additions a row,
+// and 9 to unpack).  k = 22, A = 58659 45.3 -> 40.3 ms, A = 40001 23.8 -> 20.2 ms; k = 21,
+// A = 40001 20.1 -> 17.2 ms.  Seven window bits would need unpacking within a row.
+// Two tables take turns of two rows; the one of the turn before is unpacked at the end of a
+// turn, when every warp has left it (a barrier of this turn) and none has come back (the next
+// turn's first).  So a field holds the counts of 6 warps x 2 rows; one table that is unpacked
+// while others go on adding can hold 17 warps' rows, as their timing has it.  With five
+// window bits a field is at most 12 x 4 q pairs x 4^5.  With six, an overflow takes four q
+// pairs of one distance and most of every window's pairs in one bin: the fullest fields are
+// those of A = 2^j + 1, 44,000 of 65,535 (62,600 with 17 rows), and as the rows of a turn are
+// an odd one and the one below it, whatever the segments, they are the same in every run.
+// An overflow would make the bins' sum wrong, and the caller counts on another kernel.
 constexpr int kPackCells = 36;  // q distance <= 16, bins 0 .. 3, 8 .. 11, 16 .. 19 (and 4 more)
 template <int kLevels, bool kMany>
 __host__ __device__ constexpr bool fold_packed() { return kLevels <= 2 && !kMany; }
@@ -157,7 +163,8 @@ __device__ __forceinline__ void pack_column(const H16& g, uint32_t at, uint32_t 
   pack_word<kTwice, 16>(g.p0[2], at, at2); pack_word<kTwice, 17>(g.p1[2], at, at2);
   pack_word<kTwice, 18>(g.p2[2], at, at2); pack_word<kTwice, 19>(g.p3[2], at, at2);
 }
-// A warp's share of a packed table to the 32-bit one; other warps may go on adding.
+// A warp's share of a packed table to the 32-bit one; other warps may go on adding.  (An
+// exchange also where none does: a load and a store take longer, k = 22 40.7 against 40.3 ms.)
 __device__ __forceinline__ void unpack_cells(uint32_t cells, uint32_t tab, int warp) {
 #pragma unroll
   for (int i = 0; i < kPackCells / (kFoldThreads / 32); ++i) {
@@ -217,11 +224,12 @@ template <int kLevels>
 __host__ __device__ constexpr int fold_exchanges() { return kLevels == 2 ? 2 : kLevels - 1; }
 
 // Shared memory of the folding kernel: tables (U, D and a spare, which a q' past the last
-// reaches at distances up to 17; U and D twice for wide products), exchange rows, the
-// ring of staged rows, and the q-distance counts of each thread (many).
+// reaches at distances up to 17; U and D twice for wide products; packed tables, two for U,
+// beside U and D), exchange rows, the ring of staged rows, and the q-distance counts of each
+// thread (many).
 template <int kLevels, bool kMany>
 __host__ __device__ constexpr int fold_tables() {
-  return fold_packed<kLevels, kMany>() ? kTabBytes * 2 + (3 * kPackCells + 1) * 128 : kTabBytes * (kMany ? 4 : 3);
+  return fold_packed<kLevels, kMany>() ? kTabBytes * 2 + (4 * kPackCells + 1) * 128 : kTabBytes * (kMany ? 4 : 3);
 }
 template <int kLevels, bool kMany>
 constexpr size_t fold_smem() {
@@ -278,8 +286,10 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
   const bool two = qc + a.A < a.nq, second = __any_sync(0xffffffffu, two);  // a second q: here, in this warp
   // few q: the third table is not read
   constexpr bool kPacked = fold_packed<kLevels, kMany>();
-  constexpr uint32_t kNext = kPacked ? kPackCells * 128 : kTabBytes;  // from U to D to the spare
-  const uint32_t to_u = kPacked ? tab_u + 2 * kTabBytes : tab_u, spare = to_u + 2 * kNext;
+  constexpr uint32_t kNext = kPacked ? kPackCells * 128 : kTabBytes;  // from a table to the next
+  const uint32_t to_u0 = kPacked ? tab_u + 2 * kTabBytes : tab_u;     // U (packed: and U of the other turn)
+  const uint32_t to_d = to_u0 + (kPacked ? 2 : 1) * kNext, spare = to_d + kNext;
+  uint32_t to_u = to_u0;
 
   // input: staged rows through a ring of kSlots rows
   int slot = 0;  // ring slot of load number it (row r + kLead of that step)
@@ -331,6 +341,7 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
       if constexpr (kLevels == 2) row += ((it + u) & 1) * 48 * kCols;
       if constexpr (kLevels >= 2) g = level<6>(g, row, tid, 1, y1);
       else __syncthreads();  // the row loaded ahead is complete for the neighbours
+      if constexpr (kPacked) to_u = to_u0 + ((it + u) & 2 ? kNext : 0u);
       // fold: every q of row residue v with every q' of column residue v'
       const uint32_t v = a.row0 + r;
       if constexpr (!kMany) {
@@ -338,7 +349,7 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
 #pragma unroll 1
           for (uint32_t q = qr; q < a.nq; q += a.A) {
             // columns that do not count here go to a spare column of the table
-            const uint32_t to = !mine || vc < v ? spare : vc == v ? to_u + kNext : to_u;
+            const uint32_t to = !mine || vc < v ? spare : vc == v ? to_d : to_u;
             const uint32_t at = to + (__popc(q ^ qc) << 7);
             if constexpr (kPacked) {
               if (second) pack_column<true>(g, at, (two ? to : spare) + (__popc(q ^ (qc + a.A)) << 7));
@@ -372,15 +383,18 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
       qr = sub_mod(qr, a.qinv, a.A);
     }
     if constexpr (kPacked) {
-      if (kUnroll == 2 || (it & 1)) unpack_cells(to_u, tab_u, warp);
-      if ((it & 31) >= 32 - kUnroll) unpack_cells(to_u + kNext, tab_u + kTabBytes, warp);  // a row has one v = v'
+      // the other turn's table: every warp left it before a barrier of this turn, and enters
+      // it past one that waits for this warp
+      if (kUnroll == 2 || (it & 1)) unpack_cells(to_u0 + (it & 2 ? 0u : kNext), tab_u, warp);
+      if ((it & 31) >= 32 - kUnroll) unpack_cells(to_d, tab_u + kTabBytes, warp);  // a row has one v = v', a lane every 32nd
     }
   }
   copy_wait<0>();
   __syncthreads();
   if constexpr (kPacked) {
-    unpack_cells(to_u, tab_u, warp);
-    unpack_cells(to_u + kNext, tab_u + kTabBytes, warp);
+    unpack_cells(to_u0, tab_u, warp);
+    unpack_cells(to_u0 + kNext, tab_u, warp);
+    unpack_cells(to_d, tab_u + kTabBytes, warp);
     __syncthreads();
   }
   // tables -> global sums
