@@ -676,21 +676,10 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
     r.total_ms = total;
     r.user_tag = reqs[i].user_tag;
     r.status = DD_OK;
-    // a packed count that left its field makes the total wrong (dd_carry.cu): the
-    // instance is then computed pair by pair
-    if (routes[i] >= ROUTE_CARRY) {
-      u128 total_pairs = 0;
-      for (int b = 0; b < kMaxBins; ++b) total_pairs += raw[b];
-      if (total_pairs != pairs) redo.push_back(i);
-    }
+    if (routes[i] >= ROUTE_CARRY && !holds_all_pairs(raw, pairs)) redo.push_back(i);
   }
-  for (uint32_t i : redo) {
-    dd_request q = reqs[i];
-    q.kernel = DD_KERNEL_MMA;
-    st = run_requests(ctx, &q, 1, &results[i], false);
-    if (st != DD_OK) return st;
-  }
-  return DD_OK;
+  return recount(reqs, results, redo,
+                 [ctx](const dd_request& q, dd_result& r) { return run_requests(ctx, &q, 1, &r, false); });
 }
 
 }  // namespace dd

@@ -3,6 +3,7 @@
 // the drop-in shims with the reference's signatures (dd_dropin.cpp).
 #pragma once
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -41,6 +42,14 @@ u128 planned_pairs(const Shape& s, const dd_request& req);
 
 // Post-processing of the raw histogram into res (counts, minb, error).
 void postprocess(const dd_request& req, const Shape& s, const uint64_t* raw, dd_result& res);
+
+// Whether the raw bins hold all of an instance's pairs.  The residue kernels count in
+// packed fields; one that overflows loses counts, and never adds any (dd_carry.cu).
+bool holds_all_pairs(const uint64_t* raw, u128 pairs);
+// Computes the instances `which` of a launch again, pair by pair, with `run`.  A result's
+// times are those of both passes.  Stops at the first status that is not DD_OK.
+int recount(const dd_request* reqs, dd_result* results, const std::vector<uint32_t>& which,
+            const std::function<int(const dd_request&, dd_result&)>& run);
 
 // Reference golden tables (src/solutions.h) and error estimates (src/globals.cpp:65-183).
 double rel_error_an(uint64_t A, uint32_t n, const u128* tgt, int offset, double* errors);

@@ -261,6 +261,26 @@ u128 planned_pairs(const Shape& s, const dd_request& req) {
   return s.samples;
 }
 
+bool holds_all_pairs(const uint64_t* raw, u128 pairs) {
+  u128 total = 0;
+  for (int b = 0; b < kMaxBins; ++b) total += raw[b];
+  return total == pairs;
+}
+
+int recount(const dd_request* reqs, dd_result* results, const std::vector<uint32_t>& which,
+            const std::function<int(const dd_request&, dd_result&)>& run) {
+  for (uint32_t i : which) {
+    const double kernel_ms = results[i].kernel_ms, total_ms = results[i].total_ms;
+    dd_request q = reqs[i];
+    q.kernel = DD_KERNEL_MMA;
+    const int st = run(q, results[i]);
+    if (st != DD_OK) return st;
+    results[i].kernel_ms += kernel_ms;
+    results[i].total_ms += total_ms;
+  }
+  return DD_OK;
+}
+
 // ---------------------------------------------------------------------------
 // post-processing
 // ---------------------------------------------------------------------------
