@@ -51,6 +51,7 @@ struct dd_context {
   // tuning
   int hist_mode = dd::HIST_RED;
   int tuned = 0;
+  bool tune_due = false;  // a call asked for the autotuner: it runs before the first launch that reads its verdict
   uint32_t mma_epilogue = DD_MMA_EPILOGUE_AUTO;         // requested (dd_set_mma_epilogue)
   uint32_t mma_tuned_epilogue = DD_MMA_EPILOGUE_PAIRED;  // the autotuner's verdict for AUTO
   unsigned long long mma_timeout_ns = 2000000000ull;  // bound of every device-side wait
@@ -215,15 +216,26 @@ static bool large_for_mma(const Job& j, double launch_pairs) {
   return pairs >= kMmaAlways || j.shape == SHAPE_TRIANGLE || j.col_kind != COL_PROGRESSION || progression_on_mma(j, shared);
 }
 
+// Whether the pair kernel of a job depends on the autotuner's verdict.
+static bool reads_verdict(const Job& j, uint32_t kernel, double launch_pairs = 0) {
+  return kernel != DD_KERNEL_MMA && kernel != DD_KERNEL_POPC && mma_eligible(j) && large_for_mma(j, launch_pairs);
+}
+
 // Which pair kernel runs a job: explicit MMA or POPC requests are honoured where
 // the job allows them; AUTO uses the context's measured preference for jobs
 // large enough to amortise the tcgen05 kernel's launch.
 static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel, double launch_pairs = 0) {
-  if (!mma_eligible(j)) return false;
-  if (kernel == DD_KERNEL_MMA) return true;
-  if (kernel == DD_KERNEL_POPC) return false;
-  return ctx->tuned == 2 && large_for_mma(j, launch_pairs);  // autotuner's verdict for AN exhaustive shapes
+  if (kernel == DD_KERNEL_MMA) return mma_eligible(j);
+  return ctx->tuned == 2 && reads_verdict(j, kernel, launch_pairs);  // autotuner's verdict for AN exhaustive shapes
 }
+
+// The first large AUTO exhaustive request, and the first batch of 16, ask for the
+// autotuner.  Residue routes do not read its verdict (a probe of 1.2 s before a call of 0.2 to
+// 85 ms), so it runs before the first launch of the context that does.
+static bool asks_for_tuning(const dd_request& q) {
+  return q.kernel == DD_KERNEL_AUTO && q.code == DD_CODE_AN && q.mode == DD_MODE_EXHAUSTIVE && q.n >= 20;
+}
+static int tune_if_due(dd_context* ctx) { return ctx->tune_due && !ctx->tuned ? dd_autotune(ctx, nullptr) : DD_OK; }
 
 // The jobs' routes: the carry path for each where it is asked for or wins and its
 // staging memory is to be had, a pair kernel for the others.
@@ -245,8 +257,8 @@ static bool takes_carry(dd_context* ctx, const Job& j, uint32_t kernel, Route* r
   }
   return false;
 }
-static std::vector<Route> routes_of(dd_context* ctx, const std::vector<Job>& jobs, const dd_request* reqs) {
-  std::vector<Route> routes(jobs.size(), ROUTE_POPC);
+static int routes_of(dd_context* ctx, const std::vector<Job>& jobs, const dd_request* reqs, std::vector<Route>& routes) {
+  routes.assign(jobs.size(), ROUTE_POPC);
   std::vector<bool> carry(jobs.size());
   double shared = 0;
   for (size_t i = 0; i < jobs.size(); ++i) {
@@ -254,9 +266,15 @@ static std::vector<Route> routes_of(dd_context* ctx, const std::vector<Job>& job
     if (!carry[i] && reqs[i].kernel != DD_KERNEL_POPC && mma_eligible(jobs[i]) && pairs_of(jobs[i]) >= kMmaMinShared)
       shared += pairs_of(jobs[i]);
   }
-  for (size_t i = 0; i < jobs.size(); ++i)
-    if (!carry[i]) routes[i] = want_mma(ctx, jobs[i], reqs[i].kernel, shared) ? ROUTE_MMA : ROUTE_POPC;
-  return routes;
+  for (size_t i = 0; i < jobs.size(); ++i) {
+    if (carry[i]) continue;
+    if (reads_verdict(jobs[i], reqs[i].kernel, shared)) {
+      const int st = tune_if_due(ctx);
+      if (st != DD_OK) return st;
+    }
+    routes[i] = want_mma(ctx, jobs[i], reqs[i].kernel, shared) ? ROUTE_MMA : ROUTE_POPC;
+  }
+  return DD_OK;
 }
 
 // Orders the job table (popc jobs, MMA jobs, then the two kinds of carry jobs), assigns
@@ -598,7 +616,7 @@ struct McContinuation {
 
 static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count, dd_result* results,
                         bool use_graph, const McContinuation* continued = nullptr) {
-  const double t0 = now_ms();
+  double t0 = now_ms();
   std::vector<Shape> shapes(count);
   std::vector<Job> jobs;
   jobs.reserve(count);
@@ -618,7 +636,12 @@ static int run_requests(dd_context* ctx, const dd_request* reqs, uint32_t count,
   }
   int st = ensure_capacity(ctx, count, count);
   if (st != DD_OK) return st;
-  const std::vector<Route> routes = routes_of(ctx, jobs, reqs);
+  const double t_routes = now_ms();
+  const bool tuned = ctx->tuned != 0;
+  std::vector<Route> routes;
+  st = routes_of(ctx, jobs, reqs, routes);
+  if (st != DD_OK) return st;
+  if (!tuned && ctx->tuned) t0 += now_ms() - t_routes;  // the autotuner's time is not the request's
   LaunchPlan lp;
   st = plan_launch(ctx, jobs, routes, lp);
   if (st != DD_OK) return st;
@@ -740,12 +763,7 @@ int dd_autotune(dd_context* ctx, dd_tuning* out) {
 
 int dd_histogram(dd_context* ctx, const dd_request* req, dd_result* res) {
   if (!ctx || !req || !res) { set_error("NULL argument"); return DD_ERR_INVALID_ARGUMENT; }
-  // First large AUTO exhaustive request: let the autotuner pick the kernel.
-  if (!ctx->tuned && req->kernel == DD_KERNEL_AUTO && req->code == DD_CODE_AN &&
-      req->mode == DD_MODE_EXHAUSTIVE && req->n >= 20) {
-    const int st = dd_autotune(ctx, nullptr);
-    if (st != DD_OK) return st;
-  }
+  if (asks_for_tuning(*req)) ctx->tune_due = true;
   return run_requests(ctx, req, 1, res, false);
 }
 
@@ -753,10 +771,7 @@ int dd_batch_run(dd_context* ctx, const dd_request* reqs, uint32_t count, dd_res
                  const dd_batch_options* opts) {
   if (!ctx || (!reqs && count) || (!results && count)) { set_error("NULL argument"); return DD_ERR_INVALID_ARGUMENT; }
   if (count == 0) return DD_OK;
-  if (!ctx->tuned && count >= 16 && (!opts || opts->kernel == DD_KERNEL_AUTO)) {
-    const int st = dd_autotune(ctx, nullptr);
-    if (st != DD_OK) return st;
-  }
+  if (count >= 16 && (!opts || opts->kernel == DD_KERNEL_AUTO)) ctx->tune_due = true;
   if (opts && opts->kernel != DD_KERNEL_AUTO) {
     std::vector<dd_request> r(reqs, reqs + count);
     for (auto& q : r) q.kernel = opts->kernel;
@@ -809,9 +824,9 @@ int dd_histogram_part(dd_context* ctx, const dd_request* req, uint64_t tile_begi
   }
   if (tile_count == 0) return DD_OK;
   // the kernel choice follows dd_histogram's (the autotuner's verdict for AUTO)
-  if (!ctx->tuned && req->kernel == DD_KERNEL_AUTO && req->code == DD_CODE_AN && req->mode == DD_MODE_EXHAUSTIVE &&
-      req->n >= 20) {
-    st = dd_autotune(ctx, nullptr);
+  if (asks_for_tuning(*req)) ctx->tune_due = true;
+  if (reads_verdict(j, req->kernel)) {
+    st = tune_if_due(ctx);
     if (st != DD_OK) return st;
   }
   st = ensure_capacity(ctx, 1, 1);
