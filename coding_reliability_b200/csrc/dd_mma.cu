@@ -75,7 +75,7 @@ namespace {
 constexpr int kEpiWarps = 16;                          // epilogue warps
 constexpr int kEpiThreads = kEpiWarps * 32;            // 512: bin columns per bin row
 constexpr int kIssuerWarp = kEpiWarps;                 // warp 16: its lane 0 issues every MMA
-constexpr int kGenWarps = 3;                           // warps 17..20: claim, decode, write operands
+constexpr int kGenWarps = 3;                           // warps 17..19: claim, decode, write operands
 constexpr int kGenThreads = kGenWarps * 32;
 constexpr int kThreads = kEpiThreads + 32 + kGenThreads;
 constexpr int kM = 128;                 // rows per strip (UMMA M)
@@ -427,7 +427,7 @@ __device__ __noinline__ void pk_fallback(uint32_t P, uint32_t S, float inv_s, in
 }
 
 // Warp roles: warps 0..15 bin (epilogue), warp 16 issues the MMAs (lane 0),
-// warps 17..20 claim strips and write their operands.  Hand-offs go through
+// warps 17..19 claim strips and write their operands.  Hand-offs go through
 // mbarriers only: slot_full/slot_free (a strip's operands written / its MMAs
 // done), full[b] (the MMA result in TMEM buffer b is ready, and for a strip's
 // first tile the strip's StripInfo),
