@@ -81,16 +81,13 @@ struct CarryBatch {
 static_assert(sizeof(CarryBatch) <= 4096, "kernel parameters");
 
 // One step in a running column: exchange with column c + s, combine, rotate the ring entry y.
-template <int kLevel>
-__device__ __forceinline__ Hist<kLevel> level(const Hist<kLevel - 1>& own, uint8_t* row, int c, int s,
-                                              Hist<kLevel>& y) {
+__device__ __forceinline__ H16 level(const H16& own, uint8_t* row, int c, int s, H16& y) {
   put(row, c, own);
   __syncthreads();
-  Hist<kLevel - 1> nb;
+  H16 nb;
   get(row, c + s, nb);
-  const Hist<kLevel> a = as_level<kLevel>(own), n = as_level<kLevel>(nb);
-  const Hist<kLevel> r = add(add_z(a, n), y);
-  y = add_z(n, a);
+  const H16 r = add(add_z(own, nb), y);
+  y = add_z(nb, own);
   return r;
 }
 
@@ -336,10 +333,10 @@ __global__ void __launch_bounds__(kFoldThreads, kLevels <= 2 ? 3 : 2) carry_fold
       copy_wait<kAhead - 1>();
       // remaining levels
       uint8_t* row = ex;
-      if constexpr (kLevels == 4) { g = level<6>(g, row, tid, 4, y4[u & 3]); row += 48 * kCols; }
-      if constexpr (kLevels >= 3) { g = level<6>(g, row, tid, 2, y2[u & 1]); row += 48 * kCols; }
+      if constexpr (kLevels == 4) { g = level(g, row, tid, 4, y4[u & 3]); row += 48 * kCols; }
+      if constexpr (kLevels >= 3) { g = level(g, row, tid, 2, y2[u & 1]); row += 48 * kCols; }
       if constexpr (kLevels == 2) row += ((it + u) & 1) * 48 * kCols;
-      if constexpr (kLevels >= 2) g = level<6>(g, row, tid, 1, y1);
+      if constexpr (kLevels >= 2) g = level(g, row, tid, 1, y1);
       else __syncthreads();  // the row loaded ahead is complete for the neighbours
       if constexpr (kPacked) to_u = to_u0 + ((it + u) & 2 ? kNext : 0u);
       // fold: every q of row residue v with every q' of column residue v'

@@ -1,8 +1,6 @@
 // dd_carry.cuh — packed distance histograms in registers and the tables they are
 // added to, shared by the residue-pair kernels (dd_carry.cu, dd_carry_rows.cu).
 #pragma once
-#include <type_traits>
-
 #include "dd_carry.h"
 
 namespace dd {
@@ -21,13 +19,7 @@ struct H8 {
 struct H16 {
   uint32_t p0[4], p1[3], p2[3], p3[3];
 };
-template <int kLevel>
-using Hist = std::conditional_t<(kLevel <= 4), H8, H16>;  // both codeword's window bits summed: 4^kLevel counts
 
-__device__ __forceinline__ void zero(H8& h) {
-#pragma unroll
-  for (int j = 0; j < 3; ++j) h.e[j] = h.o[j] = 0;
-}
 __device__ __forceinline__ void zero(H16& h) {
 #pragma unroll
   for (int j = 0; j < 3; ++j) h.p0[j] = h.p1[j] = h.p2[j] = h.p3[j] = 0;
@@ -89,17 +81,9 @@ __device__ __forceinline__ H16 widen(const H8& h) {
   r.p0[3] = 0;
   return r;
 }
-template <int kLevel>
-__device__ __forceinline__ Hist<kLevel> as_level(const Hist<kLevel - 1>& h) {
-  if constexpr (kLevel == 5) return widen(h);
-  else return h;
-}
-
 // One column's histogram in a shared exchange row: 24 bytes (8-bit counts) or 48
 // (16-bit counts below the last level, whose bins stop at 23), at strides that
 // make the vector accesses conflict-free.
-template <typename H>
-__host__ __device__ constexpr int slot_bytes() { return std::is_same_v<H, H8> ? 24 : 48; }
 __device__ __forceinline__ void put(uint8_t* row, int c, const H8& h) {
   uint2* p = reinterpret_cast<uint2*>(row + c * 24);
   p[0] = make_uint2(h.e[0], h.e[1]);
@@ -175,26 +159,11 @@ __device__ __forceinline__ void add_bin(uint32_t at, uint32_t f, uint32_t x) {
   }
 }
 template <int kProduct, int kBin>
-__device__ __forceinline__ void add_bytes(uint32_t at, uint32_t f, uint32_t w) {
-  if (w) {
-    add_bin<kProduct, kBin>(at, f, w & 0xFFu);
-    add_bin<kProduct, kBin + 2>(at, f, (w >> 8) & 0xFFu);
-    add_bin<kProduct, kBin + 4>(at, f, (w >> 16) & 0xFFu);
-    add_bin<kProduct, kBin + 6>(at, f, w >> 24);
-  }
-}
-template <int kProduct, int kBin>
 __device__ __forceinline__ void add_halves(uint32_t at, uint32_t f, uint32_t w) {
   if (w) {
     add_bin<kProduct, kBin>(at, f, w & 0xFFFFu);
     add_bin<kProduct, kBin + 4>(at, f, w >> 16);
   }
-}
-template <int kProduct>
-__device__ __forceinline__ void add_hist(uint32_t at, uint32_t f, const H8& h) {
-  add_bytes<kProduct, 0>(at, f, h.e[0]); add_bytes<kProduct, 1>(at, f, h.o[0]);
-  add_bytes<kProduct, 8>(at, f, h.e[1]); add_bytes<kProduct, 9>(at, f, h.o[1]);
-  add_bytes<kProduct, 16>(at, f, h.e[2]); add_bytes<kProduct, 17>(at, f, h.o[2]);
 }
 template <int kProduct>
 __device__ __forceinline__ void add_hist(uint32_t at, uint32_t f, const H16& h) {

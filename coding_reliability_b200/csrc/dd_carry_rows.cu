@@ -25,7 +25,7 @@
 // Thread = column residue; the neighbour u' + s comes through shared memory.  The
 // last 2^kB - 1 threads of a CTA only feed their neighbours.
 #include <algorithm>
-#include <cmath>
+#include <type_traits>
 
 #include "dd_carry.cuh"
 #include "dd_device.cuh"

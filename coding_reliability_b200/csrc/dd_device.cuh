@@ -79,9 +79,10 @@ struct PhiloxRun {
 
 // ---------------------------------------------------------------------------
 // Ext-Hamming codewords.  Two definitions exist in the reference:
-//  - hamming_cw_gpu: parity bits WITHOUT the overall parity bit, placed in the
-//    low bits (computeHamming<N>, src/hamming.cu:39-59; the grid/MC copies in
-//    hamming_grid.cu:32-48 and hamming_mc.cu lack the N<8 branch);
+//  - parity bits WITHOUT the overall parity bit, placed in the low bits
+//    (computeHamming<N>, src/hamming.cu:39-59; the grid/MC copies in hamming_grid.cu:32-48
+//    and hamming_mc.cu lack the N<8 branch), of which only the weight is needed
+//    (hamming_weight_gpu, dd_kernels.cu);
 //  - hamming_cw_ext: the extended codeword WITH the overall parity bit
 //    (computeHamming08/16/24/32, src/hamming.h:22-64), used by the brute force.
 // ---------------------------------------------------------------------------
@@ -91,20 +92,6 @@ __host__ __device__ __forceinline__ unsigned popc64(uint64_t v) {
 #else
   return (unsigned)__builtin_popcountll(v);
 #endif
-}
-
-__host__ __device__ __forceinline__ uint64_t hamming_cw_gpu(uint64_t v, unsigned N, bool n4_branch) {
-  uint64_t hm = 0;
-  hm |= (uint64_t)(popc64(v & 0x56AAAD5Bull) & 1);
-  hm |= (uint64_t)(popc64(v & 0x9B33366Dull) & 1) << 1;
-  hm |= (uint64_t)(popc64(v & 0xE3C3C78Eull) & 1) << 2;
-  if (n4_branch && N < 8) return (v << 3) | hm;
-  hm |= (uint64_t)(popc64(v & 0x03FC07F0ull) & 1) << 3;
-  if (N < 16) return (v << 4) | hm;
-  hm |= (uint64_t)(popc64(v & 0x03FFF800ull) & 1) << 4;
-  if (N < 32) return (v << 5) | hm;
-  hm |= (uint64_t)(popc64(v & 0xFC000000ull) & 1) << 5;
-  return (v << 6) | hm;
 }
 
 // Parity masks of the extended codes, bit 1.. of the parity field; bit 0 is

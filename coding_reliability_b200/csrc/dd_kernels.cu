@@ -433,8 +433,9 @@ __device__ void mc_tile(const Job& J, uint64_t lt, uint32_t part, uint32_t split
 // ---------------------------------------------------------------------------
 // Ext-Hamming weight tiles: 32 lanes x 256 generated messages.
 // ---------------------------------------------------------------------------
-// Weight of hamming_cw_gpu(v, N, n4): the message's bits and its parity bits.  The
-// masks cover the low 32 message bits, so a parity is one 32-bit popcount.
+// Weight of the codeword computeHamming<N> (src/hamming.cu:39-59) gives message v: the
+// message's bits and three to six parity bits.  The masks cover the low 32 message bits,
+// so a parity is one 32-bit popcount.
 __device__ __forceinline__ uint32_t hamming_weight_gpu(uint64_t v, unsigned N, bool n4_branch) {
   const uint32_t x = (uint32_t)v;
   uint32_t w = popc64(v) + (__popc(x & 0x56AAAD5Bu) & 1) + (__popc(x & 0x9B33366Du) & 1) + (__popc(x & 0xE3C3C78Eu) & 1);
