@@ -235,7 +235,6 @@ static bool want_mma(const dd_context* ctx, const Job& j, uint32_t kernel, doubl
 static bool asks_for_tuning(const dd_request& q) {
   return q.kernel == DD_KERNEL_AUTO && q.code == DD_CODE_AN && q.mode == DD_MODE_EXHAUSTIVE && q.n >= 20;
 }
-static int tune_if_due(dd_context* ctx) { return ctx->tune_due && !ctx->tuned ? dd_autotune(ctx, nullptr) : DD_OK; }
 
 // The jobs' routes: the carry path for each where it is asked for or wins and its
 // staging memory is to be had, a pair kernel for the others.
@@ -268,8 +267,8 @@ static int routes_of(dd_context* ctx, const std::vector<Job>& jobs, const dd_req
   }
   for (size_t i = 0; i < jobs.size(); ++i) {
     if (carry[i]) continue;
-    if (reads_verdict(jobs[i], reqs[i].kernel, shared)) {
-      const int st = tune_if_due(ctx);
+    if (ctx->tune_due && !ctx->tuned && reads_verdict(jobs[i], reqs[i].kernel, shared)) {
+      const int st = dd_autotune(ctx, nullptr);
       if (st != DD_OK) return st;
     }
     routes[i] = want_mma(ctx, jobs[i], reqs[i].kernel, shared) ? ROUTE_MMA : ROUTE_POPC;
@@ -825,8 +824,8 @@ int dd_histogram_part(dd_context* ctx, const dd_request* req, uint64_t tile_begi
   if (tile_count == 0) return DD_OK;
   // the kernel choice follows dd_histogram's (the autotuner's verdict for AUTO)
   if (asks_for_tuning(*req)) ctx->tune_due = true;
-  if (reads_verdict(j, req->kernel)) {
-    st = tune_if_due(ctx);
+  if (ctx->tune_due && !ctx->tuned && reads_verdict(j, req->kernel)) {
+    st = dd_autotune(ctx, nullptr);
     if (st != DD_OK) return st;
   }
   st = ensure_capacity(ctx, 1, 1);
