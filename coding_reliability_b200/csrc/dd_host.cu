@@ -366,7 +366,9 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
     }
     lp.msmem = mma_smem_bytes(lp.margs.hist_rows, lp.margs.b_bufs, lp.margs.packed != 0, lp.margs.pk_cells);
     lp.mgrid = (int)std::min<uint64_t>((uint64_t)ctx->num_sms, tm);  // one CTA (one TMEM owner) per SM
-    mma_claims(lp.margs, lp.mgrid);
+    const Job& j = table[lp.npopc];
+    const bool columns = lp.nmma == 1 && j.shape == SHAPE_RECT && j.cols % kTileCols == 0 && j.tiles == job_tiles(j);
+    mma_claims(lp.margs, lp.mgrid, columns ? j.tiles / j.col_tiles : 0);
   }
   std::memcpy(ctx->h_jobs, table.data(), table.size() * sizeof(Job));
   return DD_OK;

@@ -113,6 +113,7 @@ static_assert(kEpiWarps % 4 == 0 && kColsPerWarp % 32 == 0, "whole 32-column TME
 // claim and column).  Short launches take smaller claims, and so do the last strips of
 // any, so that the CTAs end together (mma_claims).
 constexpr uint64_t kMaxClaim = 32 * kStrips;
+constexpr double kColumnStrips = 2.4;  // strips binned in the time a column operand takes (k = 20, A of 16 bits)
 // pair-packed epilogue
 constexpr int kPkHalf = kSuper / 2;                 // packed columns of a strip: p holds columns 2p, 2p + 1
 constexpr int kPkTilesPerStrip = kPkHalf / kN;      // 2 MMA tiles of 256 packed columns per strip
@@ -1077,17 +1078,46 @@ uint32_t mma_b_bufs(uint32_t hist_rows) {
   return mma_smem_bytes(hist_rows, 2, false, 0) <= smem_optin() ? 2u : 1u;
 }
 
-// Big claims (a quarter of a CTA's share, at most kMaxClaim) up to the last one per CTA,
-// then claims of an eighth of that, at least one super tile; launches of few strips go
-// in two claims per CTA.  The column operand that a claim begins with is written while
-// the pipeline drains: claims of 32 strips throughout, 64, 128, 256 and 512 take 58.8,
-// 57.1, 56.2, 54.1 and 53.3 ms (256 instances of k = 16), 5.13, 4.94, 4.93, 4.91 and
-// 5.60 ms (1-D grid, A = 40001, k = 22, m = 10007; 256 with smaller claims at the end);
-// A = 58659, k = 13 0.205 ms with claims of 32, 0.041 ms.
-void mma_claims(MmaArgs& args, int grid) {
-  const uint64_t share = args.total_tiles / (uint64_t)grid;
+// column: strips of a column, where the launch is one grid whose column tiles are all whole
+// (else 0).  Its strips cost the same, but for the column operand, which a claim writes for
+// each column that it touches.  So claims of one size, a whole column or a power of two's
+// share of one, whichever ends first, or one claim per CTA where that ends 3 % earlier
+// (columns few for the CTAs).  k = 20, m = 4096 0.56 -> 0.53 ms, m = 8192 1.05 -> 1.00,
+// m = 10001 1.29 -> 1.26; k = 18, m = 2048 0.104 -> 0.093; k = 16, m = 4096 0.070 -> 0.060
+// against the claims below, which cut the columns anywhere (A = 62307); claims of 32 throughout
+// 0.53, 1.03, 1.35, 0.097 and 0.079 ms.  Columns above kMaxClaim gain nothing (m = 65536 7.45
+// and 7.50 ms).
+//
+// Other launches (triangles' columns differ in length, a ragged last column tile is the slowest,
+// jobs have columns of their own): big claims (a quarter of a CTA's share, at most kMaxClaim) up to
+// the last one per CTA, then claims of an eighth of that, at least one super tile; launches
+// of few strips go in two claims per CTA.  The column operand that a claim begins with is
+// written while the pipeline drains: claims of 32 strips throughout, 64, 128, 256 and 512
+// take 58.8, 57.1, 56.2, 54.1 and 53.3 ms (256 instances of k = 16); A = 58659, k = 13
+// 0.205 ms with claims of 32, 0.041 ms.
+void mma_claims(MmaArgs& args, int grid, uint64_t column) {
+  const uint64_t ctas = (uint64_t)grid, share = args.total_tiles / ctas;
+  if (column && column <= kMaxClaim) {
+    auto cost = [&](uint64_t size, double columns) {  // of the last CTA, in strips
+      const uint64_t claims = (args.total_tiles + size - 1) / size;
+      return (double)((claims + ctas - 1) / ctas) * ((double)size + kColumnStrips * columns);
+    };
+    uint64_t best = column;
+    double least = cost(column, 1.0);
+    for (uint64_t parts = 2; parts <= 8 && column % parts == 0; parts *= 2) {
+      const double c = cost(column / parts, 1.0);
+      if (c >= least) continue;
+      least = c;
+      best = column / parts;
+    }
+    const uint64_t one = (args.total_tiles + ctas - 1) / ctas;
+    if (cost(one, 1.0 + (double)one / (double)column) < 0.97 * least) best = one;
+    args.big_claims = 0;
+    args.big_claim = args.small_claim = (uint32_t)best;
+    return;
+  }
   args.big_claim = (uint32_t)std::min<uint64_t>(kMaxClaim, std::max<uint64_t>(1, share / 4 / kStrips) * kStrips);
-  const uint64_t tail = (uint64_t)grid * args.big_claim;
+  const uint64_t tail = ctas * args.big_claim;
   args.big_claims = args.total_tiles > tail ? (args.total_tiles - tail) / args.big_claim : 0;
   args.small_claim = (uint32_t)std::max<uint64_t>(
       1, std::min<uint64_t>(std::max<uint64_t>(kStrips, args.big_claim / 8 / kStrips * kStrips), share / 2));

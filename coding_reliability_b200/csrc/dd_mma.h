@@ -46,8 +46,9 @@ void mma_pack_setup(Job& j, uint32_t cells);
 // Column-operand buffers that fit in shared memory next to the bins (single epilogue).
 uint32_t mma_b_bufs(uint32_t hist_rows);
 size_t mma_smem_bytes(uint32_t hist_rows, uint32_t b_bufs, bool packed, uint32_t pk_cells);
-// Sets the sizes of the strips' claims for a grid of CTAs.
-void mma_claims(MmaArgs& args, int grid);
+// Sets the sizes of the strips' claims for a grid of CTAs.  column: strips of a column of
+// the launch's one job, a grid of whole column tiles (else 0).
+void mma_claims(MmaArgs& args, int grid, uint64_t column);
 cudaError_t launch_mma(const MmaArgs& args, int grid, size_t smem, cudaStream_t stream);
 
 }  // namespace dd
