@@ -295,6 +295,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
   uint64_t tp = 0, tm = 0;
   uint32_t maxb = 1, maxbm = 1;
   bool col_table = false;
+  TileSpan span;
   lp.npopc = of_route[ROUTE_POPC];
   lp.nmma = of_route[ROUTE_MMA];
   lp.carry.resize(of_route[ROUTE_CARRY]);
@@ -309,6 +310,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
     j.tile_begin = tp;
     tp += j.tiles;
     maxb = std::max(maxb, j.nbins);
+    span.add(j);
     lp.pkind = k == 0 || lp.pkind == (int)j.kind ? (int)j.kind : kMixedKinds;
     col_table |= (j.kind == JOB_PAIRS && j.col_kind == COL_HAMMING_EXT && !j.wide);
   }
@@ -332,7 +334,7 @@ static int plan_launch(dd_context* ctx, std::vector<Job>& jobs, const std::vecto
     int& occ = ctx->occupancy[ctx->hist_mode == HIST_RED][lp.pkind + 1][maxb][col_table];
     if (!occ) DD_CUDA(hist_occupancy(ctx->hist_mode, lp.pkind, lp.psmem, &occ));
     if (occ < 1) { set_error("kernel does not fit on an SM"); return DD_ERR_UNSUPPORTED; }
-    lp.pargs.split_log = hist_split_log(tp, (uint64_t)ctx->num_sms * occ * kWarpsPerCta);
+    lp.pargs.split_log = hist_split_log(tp, (uint64_t)ctx->num_sms * occ * kWarpsPerCta, span);
     const uint64_t want = ((tp << lp.pargs.split_log) + kWarpsPerCta - 1) / kWarpsPerCta;
     lp.pgrid = (int)std::min<uint64_t>((uint64_t)ctx->num_sms * occ, std::max<uint64_t>(want, 1));
   }

@@ -18,6 +18,8 @@
 //                                                  hamming_mc.cu:57-81
 //   super-A dancoding_shared / dancoding           distance_distribution_super_a/src/an_coding.cu:32-99
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <cstdint>
 
 #include "dd_device.cuh"
@@ -722,15 +724,36 @@ cudaError_t hist_occupancy(int mode, int kind, size_t smem, int* ctas_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, kernel_ptr(mode, kind), kWarpsPerCta * 32, smem);
 }
 
+void TileSpan::add(const Job& j) {
+  uint64_t c = kTileCols, p = 1u << kMaxSplitLog;
+  if (j.kind == JOB_PAIRS) {
+    c = j.cols;
+  } else if (j.kind == JOB_MC) {
+    const uint64_t rpl = mc_rows_per_lane(j.iters - j.sample_begin);
+    if (rpl > 1) p = rpl;  // the parts are whole codewords of a lane
+  }
+  columns = std::max(columns, (uint32_t)std::min<uint64_t>(c, kTileCols));
+  parts = std::max(parts, (uint32_t)std::min<uint64_t>(p, 1u << kMaxSplitLog));
+}
+
 // Few tiles leave SMs without work and a lane with hundreds of serial steps: the
 // warps then claim 2^split_log-th parts of a tile (32 columns, 8 samples at least),
 // enough of them for two per resident warp.  Whole tiles against parts, kernel time:
 // A = 641, k = 10 70 -> 13 us, k = 12 68 -> 17 us, A = 58659, k = 14 70 -> 49 us,
 // Ext-Hamming n = 16 weights 56 -> 9 us (diagonal tiles on the fast path included).
-uint32_t hist_split_log(uint64_t tiles, uint64_t warps) {
-  uint32_t s = 0;
-  while (s < kMaxSplitLog && (tiles << s) < 2 * warps) ++s;
-  return s;
+// A further split has to shorten the longest part by a quarter: the parts past a tile's
+// columns are empty, and each is claimed from the one counter all the same (2-D grids of
+// 100,000 rows, 782 row tiles: 17 columns in 16 parts, one with work, 22.6 us, whole tiles
+// 16.9; 33 columns 28.6 and 22.5).
+uint32_t hist_split_log(uint64_t tiles, uint64_t warps, const TileSpan& span) {
+  uint32_t best = 0, longest = span.columns;
+  for (uint32_t s = 1; s <= kMaxSplitLog && (tiles << (s - 1)) < 2 * warps && (1u << (s - 1)) < span.parts; ++s) {
+    const uint32_t part = std::min(span.columns, (uint32_t)kTileCols >> s);
+    if (4 * part > 3 * longest) continue;
+    longest = part;
+    best = s;
+  }
+  return best;
 }
 
 cudaError_t launch_hist(int mode, int kind, const LaunchArgs& args, int grid, size_t smem, cudaStream_t stream) {

@@ -12,8 +12,14 @@ namespace dd {
 // (red.shared.add) or a load/add/store on its private column.
 enum HistMode : int { HIST_RED = 0, HIST_LDST = 1 };
 
+// What the parts of a launch's tiles can hold, over its jobs: columns (of kTileCols) that a
+// tile has, and parts of a tile that have work.
+struct TileSpan {
+  uint32_t columns = 1, parts = 1;
+  void add(const Job& j);
+};
 // log2 of the parts a launch splits its tiles into, for `warps` resident warps.
-uint32_t hist_split_log(uint64_t tiles, uint64_t warps);
+uint32_t hist_split_log(uint64_t tiles, uint64_t warps, const TileSpan& span);
 size_t hist_smem_bytes(uint32_t smem_bins, bool col_table);
 // kind: the JobKind of all the launch's jobs, or kMixedKinds.
 constexpr int kMixedKinds = -1;

@@ -119,6 +119,7 @@ extern "C" int dd_histogram_noalloc(int device, void* stream, const dd_request* 
   uint64_t tiles = 0;
   uint32_t maxb = 1;
   bool col_table = false;
+  TileSpan span;
   for (uint32_t i = 0; i < count; ++i) {
     std::string err;
     st = derive_shape(reqs[i], shapes[i], err);
@@ -133,6 +134,7 @@ extern "C" int dd_histogram_noalloc(int device, void* stream, const dd_request* 
     table[i].tile_begin = tiles;
     tiles += table[i].tiles;
     if (table[i].nbins > maxb) maxb = table[i].nbins;
+    span.add(table[i]);
     col_table |= (table[i].kind == JOB_PAIRS && table[i].col_kind == COL_HAMMING_EXT && !table[i].wide);
   }
   LaunchArgs args;
@@ -152,7 +154,7 @@ extern "C" int dd_histogram_noalloc(int device, void* stream, const dd_request* 
     set_error(std::string("dd_histogram_noalloc: launch set-up: ") + cudaGetErrorString(e));
     return DD_ERR_CUDA;
   }
-  args.split_log = hist_split_log(tiles, (uint64_t)sms * occ * kWarpsPerCta);
+  args.split_log = hist_split_log(tiles, (uint64_t)sms * occ * kWarpsPerCta, span);
   const uint64_t want = ((tiles << args.split_log) + kWarpsPerCta - 1) / kWarpsPerCta;
   const int grid = (int)(want < (uint64_t)sms * occ ? (want ? want : 1) : (uint64_t)sms * occ);
 
