@@ -356,8 +356,17 @@ bool rows_plan(const Job& j, int num_sms, RowsPlan& p) {
 // 13.8 and 5.2 ms; A = 8191, 512 a residue, 2.3 and 4.7 ms), the ring's as many (A = 867,
 // m = 10001: k = 18, 302 a residue, 0.26 and 0.34 ms; k = 17, 0.23 and 0.19 ms); below 2^28 pairs the popc
 // kernel's single launch is as fast.
+// The shortest A leave most of a CTA without a residue, and a thread visits its columns one
+// by one.  A tree's CTA of 4096 columns a residue takes 0.12 ms however few its rows, as
+// long as the popc kernel takes for 2^29 pairs in whole row tiles (m = 128, k = 21: A = 13,
+// 2521 columns, 0.086 and 0.080 ms, A = 15 0.075; k = 18, m = 1024, A = 1 0.121 and 0.081).
+// A listed row past the ring's k takes A = 1 22 us and A = 3 7.7 us at k = 25, where the
+// tcgen05 kernel takes 5.1 ms for 1000 rows and 1.4 for each 128 whole ones.
 bool rows_win(const Job& j, const RowsPlan& p) {
-  return (double)j.rows * (double)j.cols >= 268435456.0 && j.cols >= (uint64_t)p.A * (p.tree ? 32 : p.ring ? 192 : 256);
+  const double pairs = (double)j.rows * (double)j.cols;
+  if (pairs < 268435456.0 || j.cols < (uint64_t)p.A * (p.tree ? 32 : p.ring ? 192 : 256)) return false;
+  if (p.tree) return p.per <= 2300 || j.rows < 128 || pairs >= 536870912.0;
+  return p.ring || p.A >= 5 || j.rows <= 100ull * p.A;
 }
 
 cudaError_t launch_rows(const Job& j, const RowsPlan& p, cudaStream_t stream) {
