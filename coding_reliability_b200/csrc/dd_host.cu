@@ -172,7 +172,8 @@ static uint32_t mma_epilogue_of(const dd_context* ctx) {
 constexpr double kMmaMinTriangle = 536870912.0;  // 2^29
 constexpr double kMmaMinRect = 134217728.0;      // 2^27
 constexpr double kMmaMinShared = 67108864.0;     // 2^26, in a launch of
-constexpr double kMmaMinLaunch = 1342177280.0;   // 1.25 x 2^30 or more in such jobs
+constexpr double kMmaMinTriangles = 1342177280.0;  // 1.25 x 2^30 or more in such jobs (triangles)
+constexpr double kMmaMinRects = 1073741824.0;      // 2^30 (grids: 16 of k = 14, m = 4096 0.26 and 0.24 ms)
 constexpr double kMmaAlways = 1073741824.0;      // 2^30
 
 static double pairs_of(const Job& j) {
@@ -184,24 +185,29 @@ static double pairs_of(const Job& j) {
 // is no multiple of 128 leaves one row tile on the checked loop, and the two loops
 // together run slower), while the tcgen05 kernel writes an operand for every column tile
 // whether 128 rows use it or 4096.  So the two costs, in microseconds of a launch, or of
-// one more job of a launch that is shared: fixed, for each column tile, for each full
-// tile, for each checked one.  The coefficients fit 450 measured shapes (k = 13 .. 24, m
-// of 2^25.5 .. 2^30 / 2^k in whole and ragged tiles, A of 7, 11 and 16 bits); where the
-// rule decides, its choice takes 1.005 times the faster kernel's time in the mean and 1.05 times
-// the popc kernel's at most (A = 62307, popc and tcgen05: k = 20, m = 128 0.045 and 0.084
-// ms, m = 512 0.136 and 0.131; k = 17, m = 1024 0.044 and 0.062, m = 4096 0.136 and 0.103;
-// k = 16, m = 2805 0.088 and 0.070; 16 jobs of k = 18, m = 256 0.26 and 0.36, of k = 14,
-// m = 4096 0.26 and 0.24).
+// one more job of a launch that is shared (whose claims do not follow the columns): fixed,
+// for each column tile, for each full tile, for each checked one.  The coefficients fit
+// 450 measured shapes (k = 13 .. 24, m of 2^25.5 .. 2^30 / 2^k in whole and ragged tiles, A
+// of 7, 11 and 16 bits); where the rule decides, its choice takes 1.006 times the faster
+// kernel's time in the mean, and no longer than the popc kernel (A = 62307, popc and
+// tcgen05: k = 20, m = 128 0.045 and 0.074 ms, m = 512 0.136 and 0.119; k = 17, m = 1024
+// 0.044 and 0.047, m = 4096 0.136 and 0.088; k = 16, m = 2805 0.088 and 0.060; 16 jobs of
+// k = 18, m = 256 0.26 and 0.36, of k = 14, m = 4096 0.26 and 0.24).
+struct GridCost {
+  double fixed, column, full, whole_warps, ragged;
+};
+constexpr GridCost kGridAlone{28.0, 0.035, 0.0145, 0.015, 0.030}, kGridShared{4.0, 0.045, 0.0135, 0.022, 0.042};
+
 static bool progression_on_mma(const Job& j, bool shared) {
+  const GridCost& c = shared ? kGridShared : kGridAlone;
   const double tiles = (double)j.col_tiles, full = (double)(j.rows / kWarpRows);
   const uint32_t rest = (uint32_t)(j.rows % kWarpRows);
-  double popc = shared ? 0.0 : 13.0, mma = shared ? 4.0 : 36.0;
+  double popc = shared ? 0.0 : 13.0, mma = c.fixed + tiles * (c.column + c.full * full);
   if (rest) {
     popc += tiles * (0.048 * full + 0.066 + 0.013 * ((rest + 31) / 32));
-    mma += tiles * (0.045 + 0.0135 * full + (rest % 32 ? 0.042 : 0.022));
+    mma += tiles * (rest % 32 ? c.ragged : c.whole_warps);
   } else {
     popc += tiles * 0.0295 * full;
-    mma += tiles * (0.045 + 0.0135 * full);
   }
   return mma < popc;
 }
@@ -210,10 +216,10 @@ static bool progression_on_mma(const Job& j, bool shared) {
 // autotuner prefers that.  launch_pairs: pairs of the launch's jobs that could share one
 // (0: unknown).
 static bool large_for_mma(const Job& j, double launch_pairs) {
-  const bool shared = launch_pairs >= kMmaMinLaunch;
+  const bool triangle = j.shape == SHAPE_TRIANGLE, shared = launch_pairs >= (triangle ? kMmaMinTriangles : kMmaMinRects);
   const double pairs = pairs_of(j);
-  if (pairs < (shared ? kMmaMinShared : j.shape == SHAPE_TRIANGLE ? kMmaMinTriangle : kMmaMinRect)) return false;
-  return pairs >= kMmaAlways || j.shape == SHAPE_TRIANGLE || j.col_kind != COL_PROGRESSION || progression_on_mma(j, shared);
+  if (pairs < (shared ? kMmaMinShared : triangle ? kMmaMinTriangle : kMmaMinRect)) return false;
+  return pairs >= kMmaAlways || triangle || j.col_kind != COL_PROGRESSION || progression_on_mma(j, shared);
 }
 
 // Whether the pair kernel of a job depends on the autotuner's verdict.
