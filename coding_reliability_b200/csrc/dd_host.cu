@@ -202,12 +202,15 @@ static bool progression_on_mma(const Job& j, bool shared) {
   const GridCost& c = shared ? kGridShared : kGridAlone;
   const double tiles = (double)j.col_tiles, full = (double)(j.rows / kWarpRows);
   const uint32_t rest = (uint32_t)(j.rows % kWarpRows);
+  // the popc kernel starts anew where the columns' high word changes, every 2^32 / A of them
+  // (k = 16, m = 2048: A of 28 bits 0.050 ms, 30 0.070, 32 0.144; tcgen05 0.047 to 0.052)
+  const double starts = 1.0 + 5.0 * (double)j.A / 4294967296.0;
   double popc = shared ? 0.0 : 13.0, mma = c.fixed + tiles * (c.column + c.full * full);
   if (rest) {
-    popc += tiles * (0.048 * full + 0.066 + 0.013 * ((rest + 31) / 32));
+    popc += tiles * (0.048 * starts * full + 0.066 + 0.013 * ((rest + 31) / 32));
     mma += tiles * (rest % 32 ? c.ragged : c.whole_warps);
   } else {
-    popc += tiles * 0.0295 * full;
+    popc += tiles * 0.0295 * starts * full;
   }
   return mma < popc;
 }

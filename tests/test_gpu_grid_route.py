@@ -20,7 +20,10 @@ def best(call, n=8):
 
 @pytest.mark.parametrize("A,k,m,mma", [(62307, 20, 128, False), (62307, 19, 256, False), (62307, 18, 512, False), (62307, 17, 1024, False),
                                        (62307, 20, 256, False), (62307, 15, 4096, False), (1733, 14, 8192, False), (62307, 17, 4096, True),
-                                       (62307, 16, 8192, True), (62307, 16, 2805, True), (62307, 20, 1024, True)])
+                                       (62307, 16, 8192, True), (62307, 16, 2805, True), (62307, 20, 1024, True),
+                                       # the popc kernel starts anew every 2^32 / A columns
+                                       (2147483659, 16, 2048, True), (2147483659, 20, 256, True), (1073741827, 17, 1024, True),
+                                       (16777259, 20, 256, False)])
 def test_route(ctx, A, k, m, mma):
     ctx.autotune()
     auto, popc = (best(lambda kern=kern: ctx.histogram(grid(A, k, m, kern))) for kern in (dd.KERNEL_AUTO, dd.KERNEL_POPC))
