@@ -188,10 +188,10 @@ static double pairs_of(const Job& j) {
 // one more job of a launch that is shared (whose claims do not follow the columns): fixed,
 // for each column tile, for each full tile, for each checked one.  The coefficients fit
 // 450 measured shapes (k = 13 .. 24, m of 2^25.5 .. 2^30 / 2^k in whole and ragged tiles, A
-// of 7, 11 and 16 bits); where the rule decides, its choice takes 1.006 times the faster
+// of 7, 11 and 16 bits); where the rule decides, its choice takes 1.005 times the faster
 // kernel's time in the mean, and no longer than the popc kernel (A = 62307, popc and
 // tcgen05: k = 20, m = 128 0.045 and 0.074 ms, m = 512 0.136 and 0.119; k = 17, m = 1024
-// 0.044 and 0.047, m = 4096 0.136 and 0.088; k = 16, m = 2805 0.088 and 0.060; 16 jobs of
+// 0.044 and 0.047, m = 4096 0.136 and 0.088; k = 16, m = 2805 0.088 and 0.057; 16 jobs of
 // k = 18, m = 256 0.26 and 0.36, of k = 14, m = 4096 0.26 and 0.24).
 struct GridCost {
   double fixed, column, full, whole_warps, ragged;

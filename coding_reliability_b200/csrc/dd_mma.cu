@@ -872,23 +872,23 @@ __global__ void __launch_bounds__(kThreads, 1) mma_hist_kernel(MmaArgs args) {
           // windowed branch for them made its loop 2-3 % slower, a non-inlined checked
           // loop 4 %.)
           if (__all_sync(0xffffffffu, lo_o + 1 >= hi_o)) return;
-          if (rect && dhi >= 64) {
-            // a grid's last rows: a lane's row counts wholly or not at all.  k = 22, A = 65537:
-            // m = 992 0.715 ms, 0.847 through the checked loop below (0.78 before the votes
-            // were put in front of that), m = 1000 0.85 and 0.92; k = 24, m = 300 2.16 and 2.46.
-            // (The comparison is written twice: kept in a variable it costs the full strips'
-            // loop 2.5 %, k = 18 3.21 and 3.29 ms, by another allocation of registers.)
-            const uint32_t limit = i < es.n ? pklimit : 0u;
-#pragma unroll
-            for (int u = 0; u < 32; ++u) {
-              if (x[u] < limit) red_shared(pk_lane + (x[u] << 7));
-              else if (i < es.n) pk_single(x[u], true, true);
-            }
-            return;
-          }
           if (pkall && __all_sync(0xffffffffu, lo_o < 0 && hi_o == 64)) {
 #pragma unroll
             for (int u = 0; u < 32; ++u) red_shared(pk_lane + (x[u] << 7));
+            return;
+          }
+          // A lane's row counts wholly or not at all in a grid's last rows, and in most halves
+          // of a triangle's edge: one test a value.  Grids, k = 22, A = 65537: m = 992 0.85 ->
+          // 0.70 ms, m = 1000 0.92 -> 0.74; k = 24, m = 300 2.46 -> 1.55 (through the loop
+          // below; 0.78, 0.90 and 2.40 before the votes above were put in front of that).
+          const bool whole = lo_o < 0 && hi_o == 64;
+          if (__all_sync(0xffffffffu, whole || lo_o + 1 >= hi_o)) {
+            const uint32_t limit = whole ? pklimit : 0u;
+#pragma unroll
+            for (int u = 0; u < 32; ++u) {
+              if (x[u] < limit) red_shared(pk_lane + (x[u] << 7));
+              else if (whole) pk_single(x[u], true, true);
+            }
             return;
           }
 #pragma unroll

@@ -330,7 +330,8 @@ typedef struct dd_tuning {
  * either epilogue) on a probe instance (A = 65521, k = 20: 36-bit codewords,
  * 5.5e11 pairs, about a second in all) on this context's GPU and keeps the
  * fastest for kernel = AUTO, and the faster tcgen05 epilogue for the
- * tcgen05 kernel.  Runs by itself before the first large AUTO request. */
+ * tcgen05 kernel.  Runs by itself before a context's first launch that depends on
+ * its verdict, once a large AUTO exhaustive request or a batch of 16 was made. */
 int dd_autotune(dd_context* ctx, dd_tuning* out);
 
 /* Epilogue of this context's tcgen05 launches (dd_mma_epilogue): AUTO follows

@@ -1,5 +1,5 @@
 """Grids whose last row tile is not full on the tcgen05 kernel (paired epilogue: a lane's row
-counts wholly or not at all): rows left over around the warps' 32, windows of every
+counts wholly or not at all in a half tile): rows left over around the warps' 32, windows of every
 distance and of a part (outliers included), ragged last columns beside them; against the
 popc kernel.  And the time of a grid with such a tile against one without."""
 import pytest
@@ -47,6 +47,6 @@ def test_time_of_a_part_tile(ctx):
         ctx.histogram(q)
         return min(ctx.histogram(q).kernel_ms for _ in range(n))
 
-    # three of a tile's four warps' rows, of eight tiles: 1.16 of the time of eight full ones
+    # three of a tile's four warps' rows, of eight tiles: 1.14 of the time of eight full ones
     # (1.38 through the checked loop, 1.22 before that loop had votes)
     assert best(992) <= 1.2 * best(1024)
