@@ -18,7 +18,7 @@
 // With b = k - bits(A) that is about b A^2 / 2 small steps instead of 4^k / 2 pairs
 // (A = 58659, k = 22: 1.0e10 against 8.8e12), all in integers.
 //
-// Measured on B200 against the tcgen05 kernel: A = 58659, k = 22: 40.6 ms against 941 ms
+// Measured on B200 against the tcgen05 kernel: A = 58659, k = 22: 40.4 ms against 941 ms
 // (965 ms before its generators were mended), k = 24: 85 ms against 15 s; A = 62307,
 // k = 20: 20.6 against 59.2 ms; A = 867, k = 21: 0.18 against 193 ms, k = 16: 0.046
 // against 0.28 ms.  Bound by instruction issue and its latencies at 12 to 18 warps an

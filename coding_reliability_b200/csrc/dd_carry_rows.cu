@@ -341,7 +341,7 @@ bool rows_plan(const Job& j, int num_sms, RowsPlan& p) {
   const uint64_t threads = p.tree ? Form<true>::kThreads : Form<false>::kThreads;
   const uint64_t useful = threads - ((1u << kb) - 1), strips = (p.A + useful - 1) / useful;
   const uint64_t row_sum = (threads / 32) * p.per * (p.tree ? 1ull << (2 * kb) : 1ull << kb);
-  const uint64_t bound = 0xFFFFFFFFull / row_sum;  // at least 16: per <= 4096
+  const uint64_t bound = 0xFFFFFFFFull / row_sum;  // at least 15: per <= 4096
   uint64_t seg = p.tree ? 8 : 256;
   while (seg > 1 && strips * ((p.rows + seg - 1) / seg) * p.slices < 8ull * num_sms) seg /= 2;
   while ((p.rows + seg - 1) / seg > 65535) seg *= 2;
@@ -360,13 +360,14 @@ bool rows_plan(const Job& j, int num_sms, RowsPlan& p) {
 // by one.  A tree's CTA of 4096 columns a residue takes 0.12 ms however few its rows, as
 // long as the popc kernel takes for 2^29 pairs in whole row tiles (m = 128, k = 21: A = 13,
 // 2521 columns, 0.086 and 0.080 ms, A = 15 0.075; k = 18, m = 1024, A = 1 0.121 and 0.081).
-// A listed row past the ring's k takes A = 1 22 us and A = 3 7.7 us at k = 25, where the
-// tcgen05 kernel takes 5.1 ms for 1000 rows and 1.4 for each 128 whole ones.
+// A listed row past the ring's k takes A = 1 22 us at k = 25, A = 3 7.7, A = 5 4.4 and A = 7
+// 3.3, the tcgen05 kernel 1.7 ms for up to 128 rows and 3.1 us for each more: as long with
+// 72 rows at A = 1, 300 at A = 3, 550 at A = 5.
 bool rows_win(const Job& j, const RowsPlan& p) {
   const double pairs = (double)j.rows * (double)j.cols;
   if (pairs < 268435456.0 || j.cols < (uint64_t)p.A * (p.tree ? 32 : p.ring ? 192 : 256)) return false;
   if (p.tree) return p.per <= 2300 || j.rows < 128 || pairs >= 536870912.0;
-  return p.ring || p.A >= 5 || j.rows <= 100ull * p.A;
+  return p.ring || p.A >= 7 || j.rows <= 120ull * p.A - 45;
 }
 
 cudaError_t launch_rows(const Job& j, const RowsPlan& p, cudaStream_t stream) {

@@ -11,8 +11,9 @@ def grid(A, k, m, kernel):
     return dd.Request(dd.CODE_AN, dd.MODE_GRID_1D, A, k, m=m, kernel=kernel)
 
 
-@pytest.mark.parametrize("A,k,m,carry", [(1, 25, 1000, False), (3, 25, 1000, False), (3, 26, 384, False), (1, 25, 129, False), (1, 25, 100, True),
-                                         (3, 25, 300, True), (5, 25, 1000, True), (1, 24, 1000, True), (1, 18, 1024, False), (3, 20, 256, False),
+@pytest.mark.parametrize("A,k,m,carry", [(1, 25, 1000, False), (3, 25, 1000, False), (3, 26, 384, False), (1, 25, 129, False), (1, 25, 100, False),
+                                         (3, 25, 300, True), (5, 25, 1000, False), (1, 25, 50, True), (5, 25, 500, True), (7, 25, 1000, True),
+                                         (1, 24, 1000, True), (1, 18, 1024, False), (3, 20, 256, False),
                                          (5, 20, 256, False), (13, 21, 128, False), (15, 21, 128, True), (1, 22, 64, True), (1, 20, 1024, True)])
 def test_route(ctx, A, k, m, carry):
     ctx.autotune()
